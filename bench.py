@@ -41,14 +41,14 @@ UNIT = "ms/projection"
 
 # Algorithmic bytes per pool cell (cells of 8^3 tiles holding >= 1 unknown)
 # for each kernel, FP32 data: reads + writes of the arrays it must touch once.
-# The MIC(0)-PCG iteration on 16^3 macro tiles runs as two passes:
+# The MIC(0)-PCG iteration on x-pencils of 16^3 macro tiles runs as two passes:
 ALGO_BYTES = {
-    # stencil with the direction update: read p_old, z, diag, 3 lower
-    # weights; write p_new, q
-    "spmv": 32,
-    # forward sweep with the x/r update: read r q p x d + 3 w, write r x t
-    # (44); backward sweep: read t d 3 w r, write z (28)
-    "mic_sweeps": 72,
+    # stencil with the x and direction updates: read p_old, z, x, diag, 3
+    # lower weights; write x, p_new, q
+    "spmv": 40,
+    # forward sweep with the r update: read r q d + 3 w, write r t (32);
+    # backward sweep: read t d 3 w r, write z (28)
+    "mic_sweeps": 60,
     # the unfused kernels (8^3-tile sweeps, learned preconditioner path)
     "spmv_plain": 24,        # x, diag, 3 lower weights, y
     "mic_sweeps_plain": 52,  # forward 24, backward 28
@@ -56,8 +56,8 @@ ALGO_BYTES = {
     "update_p": 12,          # read z, p; write p
 }
 
-# One fused MIC(0)-PCG iteration: stencil pass 32 + sweep pair 72.
-ITER_BYTES = 104
+# One fused MIC(0)-PCG iteration: stencil pass 40 + sweep pair 60.
+ITER_BYTES = 100
 
 # library kernels one splat call launches: bin, tile scan, three scan passes,
 # scatter, sort, three face compactions, three work counts, work scan, three
@@ -779,11 +779,11 @@ def main():
                               "achieved_gbs": ALGO_BYTES[name] * cells.value / (ms.value * 1e-3) / 1e9}
     peak, peak_kind = measured_peaks()
     traffic = ncu_traffic() or {}
-    names = {"spmv": "k_spmv (stencil q = A p, p = z + beta p formed on the fly, fused p.q)",
-             "mic_sweeps": "k_mic_forward16 + k_mic_backward16 (MIC(0) wavefront sweeps; x/r update and norms "
-                           "in the forward staging, fused z.r)",
+    names = {"spmv": "k_spmv (stencil q = A p, x += alpha p and p = z + beta p formed on the fly, fused p.q)",
+             "mic_sweeps": "k_pencil_forward + k_pencil_backward (MIC(0) wavefront sweeps; r update and norms in the "
+                           "forward staging, fused z.r)",
              "spmv_plain": "k_spmv (stencil q = A p with fused p.q)",
-             "mic_sweeps_plain": "k_mic_forward16 + k_mic_backward16 (plain MIC(0) apply)",
+             "mic_sweeps_plain": "k_mic_forward + k_mic_backward (plain MIC(0) apply)",
              "update_xr": "k_update_xr (x, r update with inf/2-norms)", "update_p": "k_update_p"}
     rooflines = {}
     for kname, entry in kern.items():
@@ -803,9 +803,9 @@ def main():
         dom = max(rooflines, key=lambda k: rooflines[k]["ms"])
         roofline = dict(rooflines[dom])
         if dom.startswith("mic_sweeps"):
-            roofline["note"] = ("wavefront-latency bound: each sweep is a chain of dependent macro-tile levels "
-                                "(38 in the 256^3 tank) of 46 diagonal steps each; the HBM fraction shows how far "
-                                "the dependency chain keeps it from streaming")
+            roofline["note"] = ("wavefront-latency bound: each sweep is a chain of pencil hand-offs (24 in the 256^3 "
+                                "tank) and of the steps along one pencil; the HBM fraction shows how far the "
+                                "dependency chain keeps it from streaming")
     ms_it = last["ms_solve"] / max(1, last["iterations"])
     fused = "spmv" in rooflines and "mic_sweeps" in rooflines
     it_cells = kern.get("spmv" if fused else "spmv_plain", {}).get("cells", 0)

@@ -320,9 +320,9 @@ int shkz_b200_apply_matrix(shkz_b200_ctx *ctx, const float *x_cells, float *y_ce
  * norms, 4 = p update, 5 = unknown labelling, 6 = weights/rhs assembly,
  * 7 = MIC(0) factor, 8 = one application of the learned preconditioner's
  * network (needs a loaded or initialised network), and the two passes of
- * the fused MIC(0)-PCG iteration on 16^3 macro tiles: 9 = stencil with the
- * direction update p = z + beta p, 10 = sweep pair with the x/r update in
- * the forward sweep (9 and 10 need a MIC(0) projection on macro tiles
+ * the fused MIC(0)-PCG iteration on pencils of 16^3 macro tiles: 9 = stencil
+ * with the updates x += alpha p, p = z + beta p, 10 = sweep pair with the r
+ * update in the forward sweep (9 and 10 need a MIC(0) projection on pencils
  * first, else SHKZ_B200_ERR_STATE). *cells_out (may be NULL)
  * receives the cells the kernel sweeps per launch (pool cells, or grid cells
  * for 5). No reference counterpart: it is the measurement hook for the

@@ -26,6 +26,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = {
     "assemble.cu": ["-fmad=false"],
     "solver.cu": [],
+    "mic_pencil.cu": [],
     "learned.cu": [],
     "api.cu": [],
     "noalloc.cu": [],
@@ -34,7 +35,7 @@ UNITS = {
     "splat.cu": ["-fmad=false"],
     "csr_mic0.cu": [],
 }
-HEADERS = ["common.cuh", "kernels.h", "solver.h", "learned.h", "tc_conv.cuh", "csr_mic0.h"]
+HEADERS = ["common.cuh", "wave.cuh", "kernels.h", "solver.h", "learned.h", "tc_conv.cuh", "csr_mic0.h"]
 
 
 def _stale(target: str, deps) -> bool:

@@ -52,7 +52,6 @@ struct shkz_b200_ctx {
       *sched = nullptr, *bsum = nullptr, *total = nullptr;
   // pool arrays
   float *diag = nullptr, *offx = nullptr, *offy = nullptr, *offz = nullptr, *d32 = nullptr;
-  float *upx = nullptr, *upy = nullptr, *upz = nullptr;  // upper weights of the backward sweep
   double *diag64 = nullptr, *offx64 = nullptr, *offy64 = nullptr, *offz64 = nullptr, *rhs64 = nullptr,
          *colsum = nullptr, *dmic64 = nullptr, *x64 = nullptr, *r64 = nullptr, *xref64 = nullptr,
          *p64 = nullptr, *q64 = nullptr, *z64 = nullptr;
@@ -64,10 +63,12 @@ struct shkz_b200_ctx {
   SolverState *st = nullptr;
   int *wflags = nullptr;  // factor wavefront flags [cap_pool]
   unsigned long long *faces_f = nullptr, *faces_b = nullptr;  // [cap_pool][3][64] epoch-tagged sweep faces
-  // 16^3 macro tiles of the MIC(0) sweeps
+  // 16^3 macro tiles and pencils of the MIC(0) sweeps
   int KM = 0, cap_macro = 0;
-  int *mcount = nullptr, *mstate = nullptr, *mtile = nullptr, *mnbr = nullptr, *msched = nullptr, *msub = nullptr;
-  unsigned long long *mfaces_f = nullptr, *mfaces_b = nullptr;  // [cap_macro][3][256]
+  int *mcount = nullptr, *mstate = nullptr, *mtile = nullptr, *mnbr = nullptr, *msub = nullptr, *nseg = nullptr;
+  int2 *seg = nullptr, *mseg = nullptr;
+  float *mfaces_f = nullptr, *mfaces_b = nullptr;  // [cap_macro][kFaceRows][32]
+  float *coef_f = nullptr, *coef_b = nullptr, *tp = nullptr;
   void *ws = nullptr;     // 3 WaveSync
   // last projection
   Geometry G{};
@@ -291,7 +292,6 @@ static int ensure_pool(shkz_b200_ctx *ctx, int K) {
   GROW(colsum, n); GROW(dmic64, n); GROW(x64, n); GROW(r64, n); GROW(xref64, n);
   GROW(p64, n); GROW(q64, n); GROW(z64, n);
   GROW(x, n); GROW(r, n); GROW(p, n); GROW(q, n); GROW(z, n); GROW(t, n); GROW(p32, n); GROW(pb, n);
-  GROW(upx, n); GROW(upy, n); GROW(upz, n);
   GROW(partials, (size_t)2 * cap + 4 * 8192);
   GROW(wflags, (size_t)cap);
   GROW(faces_f, (size_t)cap * 3 * 64);
@@ -300,14 +300,8 @@ static int ensure_pool(shkz_b200_ctx *ctx, int K) {
   SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->faces_f, 0, sizeof(unsigned long long) * (size_t)cap * 3 * 64, ctx->stream));
   SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->faces_b, 0, sizeof(unsigned long long) * (size_t)cap * 3 * 64, ctx->stream));
   if (ctx->ws) {
-    // flags were reset: restart the epochs (macro faces too, so no stale tag matches)
+    // flags were reset: restart the epochs
     SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->ws, 0, 3 * wave_sync_bytes(), ctx->stream));
-    if (ctx->mfaces_f) {
-      SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->mfaces_f, 0, sizeof(unsigned long long) * (size_t)ctx->cap_macro * 768,
-                                    ctx->stream));
-      SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->mfaces_b, 0, sizeof(unsigned long long) * (size_t)ctx->cap_macro * 768,
-                                    ctx->stream));
-    }
   }
   ctx->cap_pool = cap;
   return 0;
@@ -318,13 +312,15 @@ static int ensure_macro(shkz_b200_ctx *ctx, int KM) {
   const int cap = KM + KM / 4 + 16;
   GROW(mtile, cap);
   GROW(mnbr, (size_t)cap * 6);
-  GROW(msched, cap);
+  GROW(seg, cap);
+  GROW(mseg, cap);
+  if (!ctx->nseg) GROW(nseg, 1);
   GROW(msub, (size_t)cap * 8);
-  GROW(mfaces_f, (size_t)cap * 768);
-  GROW(mfaces_b, (size_t)cap * 768);
-  // new face words carry epoch 0, which no sweep uses
-  SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->mfaces_f, 0, sizeof(unsigned long long) * (size_t)cap * 768, ctx->stream));
-  SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->mfaces_b, 0, sizeof(unsigned long long) * (size_t)cap * 768, ctx->stream));
+  GROW(mfaces_f, (size_t)cap * kFaceRows * 32);
+  GROW(mfaces_b, (size_t)cap * kFaceRows * 32);
+  GROW(coef_f, (size_t)cap * 16 * 1024);
+  GROW(coef_b, (size_t)cap * 16 * 1024);
+  GROW(tp, (size_t)cap * 16 * kPencilRow);
   ctx->cap_macro = cap;
   return 0;
 }
@@ -349,7 +345,7 @@ static int build_macro_tiles(shkz_b200_ctx *ctx, const Geometry &G, int K, cudaS
   int rc = ensure_macro(ctx, KM > 0 ? KM : 1);
   if (rc) return rc;
   build_macro(G, M, ctx->tile_count, ctx->tile_state, ctx->mcount, ctx->mstate, ctx->mtile, ctx->mnbr,
-              ctx->level_count, ctx->msched, ctx->msub, KM, ctx->bsum, s);
+              ctx->level_count, ctx->seg, ctx->mseg, ctx->nseg, ctx->msub, KM, ctx->bsum, s);
   SHKZ_CUDA_TRY(cudaGetLastError());
   ctx->KM = KM;
   return 0;
@@ -407,11 +403,12 @@ extern "C" void shkz_b200_destroy(shkz_b200_ctx *ctx) {
                   ctx->h_vact[0], ctx->h_vact[1], ctx->h_vact[2], ctx->h_pact, ctx->flags, ctx->unk, ctx->tile_count,
                   ctx->tile_state, ctx->pool_tile, ctx->nbr, ctx->level_count, ctx->sched, ctx->bsum, ctx->total,
                   ctx->diag, ctx->offx, ctx->offy, ctx->offz, ctx->d32, ctx->diag64, ctx->offx64, ctx->offy64,
-                  ctx->offz64, ctx->rhs64, ctx->upx, ctx->upy, ctx->upz, ctx->colsum, ctx->dmic64, ctx->x64,
+                  ctx->offz64, ctx->rhs64, ctx->colsum, ctx->dmic64, ctx->x64,
                   ctx->r64, ctx->xref64, ctx->p64, ctx->q64, ctx->z64, ctx->x, ctx->r, ctx->p, ctx->q, ctx->z,
                   ctx->t, ctx->p32, ctx->partials, ctx->out4, ctx->counter, ctx->st,
                   ctx->wflags, ctx->faces_f, ctx->faces_b, ctx->ws, ctx->st_scratch, ctx->mcount, ctx->mstate,
-                  ctx->mtile, ctx->mnbr, ctx->msched, ctx->msub, ctx->mfaces_f, ctx->mfaces_b, ctx->curv,
+                  ctx->mtile, ctx->mnbr, ctx->seg, ctx->mseg, ctx->nseg, ctx->msub, ctx->mfaces_f, ctx->mfaces_b, ctx->coef_f,
+                  ctx->coef_b, ctx->tp, ctx->curv,
                   ctx->prev, ctx->rank_pool, ctx->rank_cnt, ctx->rank_total, ctx->xw, ctx->h_dens[0],
                   ctx->h_dens[1], ctx->h_dens[2], ctx->flush, ctx->pb, ctx->ext_v[0], ctx->ext_v[1], ctx->ext_v[2],
                   ctx->ext_a[0], ctx->ext_a[1], ctx->ext_a[2], ctx->ext_flag, ctx->sp_raw, ctx->sp_posm,
@@ -444,7 +441,9 @@ static PoolSystem pool_system(shkz_b200_ctx *ctx) {
   S.nbr = ctx->nbr;
   S.sched = ctx->sched;
   S.KM = ctx->cfg.mic_block == 8 ? 0 : ctx->KM;
-  S.msched = ctx->msched;
+  S.seg = ctx->seg;
+  S.mseg = ctx->mseg;
+  S.nseg = ctx->nseg;
   S.mnbr = ctx->mnbr;
   S.msub = ctx->msub;
   S.mfaces_f = ctx->mfaces_f;
@@ -457,9 +456,9 @@ static PoolSystem pool_system(shkz_b200_ctx *ctx) {
   S.offx64 = ctx->offx64;
   S.offy64 = ctx->offy64;
   S.offz64 = ctx->offz64;
-  S.upx = ctx->upx;
-  S.upy = ctx->upy;
-  S.upz = ctx->upz;
+  S.coef_f = ctx->coef_f;
+  S.coef_b = ctx->coef_b;
+  S.tp = ctx->tp;
   return S;
 }
 
@@ -476,6 +475,12 @@ static int arm_waves(shkz_b200_ctx *ctx) {
                           w == 1 && ctx->cfg.fault_skip_publish > 0 ? ctx->cfg.fault_skip_publish : 0};
     SHKZ_CUDA_TRY(cudaMemcpyAsync(wsync(ctx, w) + 3 * sizeof(int), words, sizeof(words), cudaMemcpyHostToDevice,
                                   ctx->stream));
+  }
+  // face words of the pencil sweeps: unset (a call that gave up may have left
+  // some written, and another grid's neighbours differ)
+  if (ctx->KM > 0) {
+    SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->mfaces_f, 0xff, sizeof(float) * (size_t)ctx->KM * kFaceRows * 32, ctx->stream));
+    SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->mfaces_b, 0xff, sizeof(float) * (size_t)ctx->KM * kFaceRows * 32, ctx->stream));
   }
   return 0;
 }
@@ -562,21 +567,25 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
   SolverState hst;
   int rc = 0, updates = 0;
   bool true_checked = false;
-  // MIC(0) on macro tiles: the direction update p = z + beta p rides in the
-  // next iteration's stencil (ping-pong between two p buffers) and the x/r
-  // update in the forward sweep's staging, so an iteration is three passes
-  // (stencil, forward sweep, backward sweep; the backward sweep's last CTA
-  // also finishes rho and beta)
+  // MIC(0) on pencils: the x update and the direction update p = z + beta p
+  // ride in the next iteration's stencil (ping-pong between two p buffers) and
+  // the r update in the forward sweep's staging, so an iteration is three
+  // passes (stencil, forward sweep, backward sweep; the backward sweep's last
+  // CTA also finishes rho and beta)
   // (the current direction is in ctx->p after an even number of completed
   // iterations and in ctx->pb after an odd one; the kernels pick it on the
   // device, where retired launches leave the count alone)
   const bool fused = precond == SHKZ_B200_PRECOND_MIC0 && S.KM > 0;
+  auto accumulate = [&]() {
+    if (fused) launch_accumulate_pending(n, ctx->x, ctx->p, ctx->pb, ctx->st, scale, ctx->x64, s);
+    else launch_accumulate(n, ctx->x, scale, ctx->x64, s);
+  };
   for (;;) {
     for (int b = 0; b < batch; ++b) {
       if (fused) {
-        launch_spmv_update(S, ctx->p, ctx->pb, ctx->z, ctx->q, ctx->partials, ctx->counter, ctx->st, s);
-        launch_mic_apply_update(S, ctx->d32, ctx->r, ctx->t, ctx->z, ctx->partials, ctx->p, ctx->pb, ctx->q, ctx->x,
-                                ctx->counter + 1, ctx->st, max_it, wsync(ctx, 1), wsync(ctx, 2), ctx->counter + 5, s);
+        launch_spmv_update(S, ctx->p, ctx->pb, ctx->z, ctx->q, ctx->x, ctx->partials, ctx->counter, ctx->st, s);
+        launch_mic_apply_update(S, ctx->r, ctx->z, ctx->partials, ctx->q, ctx->counter + 1, ctx->st, max_it,
+                                wsync(ctx, 1), wsync(ctx, 2), ctx->counter + 5, s);
         continue;
       }
       launch_spmv(S, ctx->p, ctx->q, ctx->partials, ctx->counter, ctx->st, 0, s);
@@ -592,7 +601,7 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
     if (hst.done == 2) break;
     if (hst.done == 1 && !reliable) break;
     // reliable update: fold the FP32 increment into x64 and replace r by b - A x64
-    launch_accumulate(n, ctx->x, scale, ctx->x64, s);
+    accumulate();
     launch_residual64(S, ctx->rhs64, ctx->x64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
     SHKZ_CUDA_TRY(cudaMemcpyAsync(h4, ctx->out4, sizeof(h4), cudaMemcpyDeviceToHost, s));
     SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
@@ -617,7 +626,7 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
   }
   if (!true_checked) {
     // plain FP32 finish (refine off) or max iterations: report the true residual
-    launch_accumulate(n, ctx->x, scale, ctx->x64, s);
+    accumulate();
     launch_residual64(S, ctx->rhs64, ctx->x64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
     SHKZ_CUDA_TRY(cudaMemcpyAsync(h4, ctx->out4, sizeof(h4), cudaMemcpyDeviceToHost, s));
     SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
@@ -836,7 +845,6 @@ static int project_device(shkz_b200_ctx *ctx, const shkz_b200_project_args *a, s
   CoeffOutputs co{ctx->diag, ctx->offx, ctx->offy, ctx->offz, ctx->diag64, ctx->offx64, ctx->offy64, ctx->offz64,
                   ctx->rhs64};
   launch_coeff(in, ctx->flags, ctx->pool_tile, K, ctx->unk, co, s);
-  if (K > 0) launch_upper_weights(pool_system(ctx), ctx->upx, ctx->upy, ctx->upz, s);
   cudaEventRecord(ctx->ev[10], s);
   const bool warm = K > 0 && ctx->cfg.warm_start;
   if (warm) {
@@ -1642,12 +1650,11 @@ extern "C" int shkz_b200_time_kernel(shkz_b200_ctx *ctx, int which, int reps, do
                                 ctx->d32, ctx->wflags, wsync(ctx, 0), s); break;
       case 8: learned_apply(ctx->model, learned_system(ctx), ctx->r, 1.0, ctx->t, s); break;
       case 9:
-        launch_spmv_update(S, ctx->p, ctx->pb, ctx->z, ctx->q, ctx->partials, ctx->counter, ctx->st_scratch, s);
+        launch_spmv_update(S, ctx->p, ctx->pb, ctx->z, ctx->q, ctx->x, ctx->partials, ctx->counter, ctx->st_scratch, s);
         break;
       case 10:
-        launch_mic_apply_update(S, ctx->d32, ctx->r, ctx->t, ctx->z, ctx->partials, ctx->p, ctx->pb, ctx->q, ctx->x,
-                                ctx->counter + 1, ctx->st_scratch, 1 << 30, wsync(ctx, 1), wsync(ctx, 2),
-                                ctx->counter + 5, s);
+        launch_mic_apply_update(S, ctx->r, ctx->z, ctx->partials, ctx->q, ctx->counter + 1, ctx->st_scratch, 1 << 30,
+                                wsync(ctx, 1), wsync(ctx, 2), ctx->counter + 5, s);
         break;
       default: break;
     }

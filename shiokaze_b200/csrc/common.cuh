@@ -42,7 +42,7 @@ struct SolverState {
   int iter;                // iterations completed
   int done;                // 1 = converged, 2 = max iterations, 3 = breakdown, 4 = replace residual
   int status;              // 0 ok, <0 error (wait timeout, NaN)
-  int pad;
+  int x_pending;           // the fused iteration's x += alpha p has not been applied yet
 };
 
 // Block-wide sum of one double; every thread gets the result.

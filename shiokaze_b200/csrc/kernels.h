@@ -25,22 +25,27 @@ struct CoeffOutputs {
   double *rhs64;
 };
 
+constexpr int kPencilRow = 256;  // floats of one x-plane of a pencil in tp
+constexpr int kFaceRows = 24;    // face rows a macro tile has room for (a pencil of n uses 16 n + 7)
+
 // Pool-resident system in 8^3 tiles.
 struct PoolSystem {
   int K;                 // tiles in the pool
   const int *nbr;        // [K][6] pool index of neighbour tiles or -1
   const int *sched;      // [K] pool indices ordered by wavefront level
   const float *diag, *offx, *offy, *offz;
-  // upper weights: the lower weight of the +x/+y/+z neighbour cell (across
-  // the tile face where needed), for the backward MIC(0) sweep
-  const float *upx, *upy, *upz;
   const double *diag64, *offx64, *offy64, *offz64;
-  // 16^3 macro tiles (2x2x2 pool tiles) for the MIC(0) sweeps
+  // 16^3 macro tiles (2x2x2 pool tiles), in x-pencils, for the MIC(0) sweeps
+  // (mic_pencil.cu)
   int KM;
-  const int *msched;     // [KM] macro tiles ordered by wavefront level
+  const int2 *seg;       // pencils (first macro tile, macro tiles) by wavefront level
+  const int *nseg;       // how many
   const int *mnbr;       // [KM][6] neighbour macro tiles or -1
   const int *msub;       // [KM][8] pool index of sub-tile (x + 2y + 4z) or -1
-  unsigned long long *mfaces_f, *mfaces_b;  // [KM][3][256] epoch-tagged sweep faces
+  const int2 *mseg;      // [KM] the pencil (first, macro tiles) a macro tile belongs to
+  float *mfaces_f, *mfaces_b;  // [KM][kFaceRows][32] +y (or -y) and +z (-z) faces of a sweep, all bits set where unwritten
+  float *coef_f, *coef_b;  // [KM][16 x][1024] sweep coefficients in the solver's order
+  float *tp;               // [KM][16 x][kPencilRow] forward result between the sweeps
 };
 
 // assemble.cu

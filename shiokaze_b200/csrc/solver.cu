@@ -33,6 +33,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "solver.h"
+#include "wave.cuh"
 #include <math_constants.h>
 #include <atomic>
 
@@ -42,25 +43,9 @@ static std::atomic<long long> g_launches{0};
 void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launches_so_far() { return g_launches.load(std::memory_order_relaxed); }
 
-#define SPIN_LIMIT (1 << 21)   // ~0.15 s with the back-off below
-
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 __device__ __forceinline__ float comp(const float4 &v, int e) { return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w)); }
-
-// Deterministic finish of a grid reduction: every block writes its partial;
-// the last block to arrive sums them in block order.
-__device__ __forceinline__ bool last_block(unsigned *counter) {
-  __shared__ bool s_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned ticket = atomicAdd(counter, 1u);
-    s_last = (ticket == gridDim.x - 1);
-  }
-  __syncthreads();
-  return s_last;
-}
 
 template <int NT>
 __device__ double sum_partials(const double *part, int n, double *red) {
@@ -150,7 +135,7 @@ __global__ void k_pool_neighbours(Geometry G, const int *tile_state, const int *
   nbr[pt * 6 + NB_YP] = look(ti, tj + 1, tk);
   nbr[pt * 6 + NB_ZM] = look(ti, tj, tk - 1);
   nbr[pt * 6 + NB_ZP] = look(ti, tj, tk + 1);
-  atomicAdd(&level_count[ti + tj + tk], 1);
+  if (level_count) atomicAdd(&level_count[ti + tj + tk], 1);
 }
 
 __global__ void k_level_scan(int *level_count, int nlev) {
@@ -182,19 +167,25 @@ struct SpmvSmem {
   float xs[10][10][16];  // (kk+1, jj+1, ii+4); halos at kk/jj 0,9 and ii 3,12
 };
 
-// zu != null: the pending direction update p <- z + beta p is applied on the
-// fly (k_update_p's arithmetic) to the tile and its halo, and the tile's new
-// p is written to pout (a different buffer: other CTAs still read the old p
-// for their halos).
+// zu != null: the pending updates of the previous iteration are applied on the
+// fly: x += alpha p with the old p (k_update_xr's arithmetic), then the
+// direction p <- z + beta p (k_update_p's) to the tile and its halo. The
+// tile's new p is written to pout (a different buffer: other CTAs still read
+// the old p for their halos). The x update costs 8 B per cell here, where the
+// old p is in registers, against 12 B in the forward sweep.
 __device__ __forceinline__ void stage_tile(const PoolSystem &S, const float *__restrict__ p, int pt, SpmvSmem &sm,
                                            float4 &xv, const float *__restrict__ zu = nullptr,
-                                           float *__restrict__ pout = nullptr, float beta = 0.0f) {
+                                           float *__restrict__ pout = nullptr, float beta = 0.0f,
+                                           float *__restrict__ x = nullptr, float alpha = 0.0f) {
   const int tid = threadIdx.x;
   const int q4 = tid & 1, jj = (tid >> 1) & 7, kk = tid >> 4;
   const size_t base = (size_t)pt * SHKZ_TC + kk * 64 + jj * 8 + q4 * 4;
   xv = ld4(p + base);
   if (zu) {
     const float4 zv = ld4(zu + base);
+    float4 sol = ld4(x + base);
+    sol.x += alpha * xv.x; sol.y += alpha * xv.y; sol.z += alpha * xv.z; sol.w += alpha * xv.w;
+    st4(x + base, sol);
     xv.x = zv.x + beta * xv.x; xv.y = zv.y + beta * xv.y; xv.z = zv.z + beta * xv.z; xv.w = zv.w + beta * xv.w;
     st4(pout + base, xv);
   }
@@ -316,7 +307,8 @@ __device__ __forceinline__ float4 stencil4(const SpmvSmem &sm, float4 xv, const 
 // (done != 0) do not flip it.
 __global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, const float *p, float *__restrict__ q,
                                               double *partials, unsigned *counter, SolverState *st, int mode,
-                                              const float *__restrict__ zu, float *pout) {
+                                              const float *__restrict__ zu, float *pout,
+                                              float *__restrict__ x) {
   __shared__ SpmvSmem sm;
   __shared__ double red[4];
   if (st && st->done) return;
@@ -324,6 +316,8 @@ __global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, co
   const int tid = threadIdx.x;
   const int q4 = tid & 1, jj = (tid >> 1) & 7, kk = tid >> 4;
   const float beta = zu ? (float)st->beta : 0.0f;
+  // alpha of the previous iteration, until the last block replaces it
+  const float alpha = zu && st->x_pending ? (float)st->alpha : 0.0f;
   if (zu && (st->iter & 1)) {
     float *t = const_cast<float *>(p);
     p = pout;
@@ -333,7 +327,7 @@ __global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, co
     float4 xv;
     const Coef4 cf = load_coef4(S, pt);
     __syncthreads();
-    stage_tile(S, p, pt, sm, xv, zu, pout, beta);
+    stage_tile(S, p, pt, sm, xv, zu, pout, beta, x, alpha);
     __syncthreads();
     const float4 y = stencil4(sm, xv, cf);
     st4(q + (size_t)pt * SHKZ_TC + kk * 64 + jj * 8 + q4 * 4, y);
@@ -473,21 +467,6 @@ __global__ void __launch_bounds__(512) k_mic_colsum(PoolSystem S, double *colsum
     if (nb >= 0) s += S.offz64[(size_t)nb * SHKZ_TC + cell];
   }
   colsum[o] = s;
-}
-
-struct WaveSync {
-  int slot;
-  unsigned finished;
-  int epoch;
-  int error;         // 0, or the slot that gave up waiting + 1
-  int spin_limit;    // polling rounds of a bounded wait (0: SPIN_LIMIT); set by the host
-  int skip_publish;  // fault injection (0: off): wavefront slot k - 1 of a forward macro sweep does not publish
-};
-
-// Rounds a bounded wait polls before it gives up.
-__device__ __forceinline__ int spin_rounds(const WaveSync *ws) {
-  const int v = *((volatile const int *)&ws->spin_limit);
-  return v > 0 ? v : SPIN_LIMIT;
 }
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
@@ -801,26 +780,8 @@ __global__ void __launch_bounds__(64) k_mic_backward(PoolSystem S, const int *sc
 }
 
 // ---------------------------------------------------------------------------
-// MIC(0) sweeps over 16^3 macro tiles (2x2x2 pool tiles per CTA).
-//
-// Same recurrences as the 8^3 kernels above, on four times as many cells per
-// CTA (256 threads, one per x-row of 16 cells, 46 in-tile diagonals): the
-// wavefront then crosses half as many tile levels, and the hand-off between
-// levels -- not the arithmetic -- is what bounds a sweep. Shared memory holds
-// the macro tile's six FP32 fields (96 KB); faces are 256 epoch-tagged words.
-
-#define MT 16
-#define MTC 4096
-// Solution array of a macro tile with one ghost layer: cell (x, y, z),
-// x, y, z in [-1, 16], at (x + 1) + 18 (y + 1) + 337 (z + 1). The ghosts hold
-// the upstream faces, so the sweep's neighbour reads are unconditional. Along
-// a diagonal (x = s - y - z) consecutive rows are 17 floats apart and the
-// warp's second plane 336 = 16 (mod 32) further, so its 32 rows fall in 32
-// distinct banks.
-#define MGY 18
-#define MGZ 337
-#define MGC 6080            // >= 18 * 337, padded to 16 bytes
-__device__ __forceinline__ int mghost(int x, int y, int z) { return (x + 1) + MGY * (y + 1) + MGZ * (z + 1); }
+// 16^3 macro tiles (2x2x2 pool tiles), the units of the pencil sweeps
+// (mic_pencil.cu).
 
 // macro tile counts = sum of the counts of its (up to) eight tiles
 __global__ void k_macro_count(Geometry G, const int *tile_count, Geometry M, int *macro_count) {
@@ -847,351 +808,6 @@ __global__ void k_macro_sub(Geometry G, Geometry M, const int *macro_tile, int K
   if (ti < G.bx && tj < G.by && tk < G.bz) pt = tile_state[(long long)ti + (long long)G.bx * ((long long)tj + (long long)G.by * tk)];
   msub[e] = pt;
 }
-
-// Stage five pool fields of the macro tile's sub-tiles into shared memory
-// (index x + 16y + 256z); absent sub-tiles read as zero.
-__device__ __forceinline__ void macro_load5(const int *sub, const float *s0, const float *s1, const float *s2,
-                                            const float *s3, const float *s4, float *d0, float *d1, float *d2,
-                                            float *d3, float *d4) {
-  for (int e = threadIdx.x; e < 8 * 128; e += blockDim.x) {
-    const int v = e & 127, st = e >> 7;
-    const int pt = sub[st];
-    const int c = v * 4;
-    const int x = (c & 7) + (st & 1) * 8, y = ((c >> 3) & 7) + ((st >> 1) & 1) * 8, z = (c >> 6) + (st >> 2) * 8;
-    const int o = x + 16 * y + 256 * z;
-    float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0, a2 = a0, a3 = a0, a4 = a0;
-    if (pt >= 0) {
-      const size_t b = (size_t)pt * (SHKZ_TC / 4) + v;
-      a0 = reinterpret_cast<const float4 *>(s0)[b];
-      a1 = reinterpret_cast<const float4 *>(s1)[b];
-      a2 = reinterpret_cast<const float4 *>(s2)[b];
-      a3 = reinterpret_cast<const float4 *>(s3)[b];
-      a4 = reinterpret_cast<const float4 *>(s4)[b];
-    }
-    *reinterpret_cast<float4 *>(d0 + o) = a0;
-    *reinterpret_cast<float4 *>(d1 + o) = a1;
-    *reinterpret_cast<float4 *>(d2 + o) = a2;
-    *reinterpret_cast<float4 *>(d3 + o) = a3;
-    *reinterpret_cast<float4 *>(d4 + o) = a4;
-  }
-}
-// Fused PCG update while staging (forward sweep of an iteration): r -= alpha q
-// and x += alpha p on the macro tile's cells, the new r staged for the sweep,
-// written back, and its inf-norm / squared 2-norm returned for this thread.
-__device__ __forceinline__ void macro_load_update(const int *sub, float *r, const float *q, const float *p, float *x,
-                                                  float alpha, const float *s1, const float *s2, const float *s3,
-                                                  const float *s4, float *d0, float *d1, float *d2, float *d3,
-                                                  float *d4, double &m, double &s2sum) {
-  for (int e = threadIdx.x; e < 8 * 128; e += blockDim.x) {
-    const int v = e & 127, st = e >> 7;
-    const int pt = sub[st];
-    const int c = v * 4;
-    const int xx = (c & 7) + (st & 1) * 8, y = ((c >> 3) & 7) + ((st >> 1) & 1) * 8, z = (c >> 6) + (st >> 2) * 8;
-    const int o = xx + 16 * y + 256 * z;
-    float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0, a2 = a0, a3 = a0, a4 = a0;
-    if (pt >= 0) {
-      const size_t b = (size_t)pt * (SHKZ_TC / 4) + v;
-      float4 rv = reinterpret_cast<const float4 *>(r)[b];
-      const float4 qv = reinterpret_cast<const float4 *>(q)[b];
-      const float4 pv = reinterpret_cast<const float4 *>(p)[b];
-      float4 xv = reinterpret_cast<const float4 *>(x)[b];
-      a1 = reinterpret_cast<const float4 *>(s1)[b];
-      a2 = reinterpret_cast<const float4 *>(s2)[b];
-      a3 = reinterpret_cast<const float4 *>(s3)[b];
-      a4 = reinterpret_cast<const float4 *>(s4)[b];
-      // the expressions of k_update_xr
-      xv.x += alpha * pv.x; xv.y += alpha * pv.y; xv.z += alpha * pv.z; xv.w += alpha * pv.w;
-      rv.x -= alpha * qv.x; rv.y -= alpha * qv.y; rv.z -= alpha * qv.z; rv.w -= alpha * qv.w;
-      reinterpret_cast<float4 *>(x)[b] = xv;
-      reinterpret_cast<float4 *>(r)[b] = rv;
-      m = fmax(m, fmax(fmax(fabs((double)rv.x), fabs((double)rv.y)), fmax(fabs((double)rv.z), fabs((double)rv.w))));
-      s2sum += (double)rv.x * rv.x + (double)rv.y * rv.y + (double)rv.z * rv.z + (double)rv.w * rv.w;
-      a0 = rv;
-    }
-    *reinterpret_cast<float4 *>(d0 + o) = a0;
-    *reinterpret_cast<float4 *>(d1 + o) = a1;
-    *reinterpret_cast<float4 *>(d2 + o) = a2;
-    *reinterpret_cast<float4 *>(d3 + o) = a3;
-    *reinterpret_cast<float4 *>(d4 + o) = a4;
-  }
-}
-
-// Write the interior of a ghosted solution array back to the pool sub-tiles.
-__device__ __forceinline__ void macro_store_ghosted(const int *sub, const float *srcg, float *dst) {
-  for (int e = threadIdx.x; e < 8 * 128; e += blockDim.x) {
-    const int v = e & 127, st = e >> 7;
-    const int pt = sub[st];
-    if (pt < 0) continue;
-    const int c = v * 4;
-    const int x = (c & 7) + (st & 1) * 8, y = ((c >> 3) & 7) + ((st >> 1) & 1) * 8, z = (c >> 6) + (st >> 2) * 8;
-    const int o = mghost(x, y, z);
-    reinterpret_cast<float4 *>(dst + (size_t)pt * SHKZ_TC)[v] = make_float4(srcg[o], srcg[o + 1], srcg[o + 2], srcg[o + 3]);
-  }
-}
-
-__device__ __forceinline__ void macro_store(const int *sub, const float *srcs, float *dst) {
-  for (int e = threadIdx.x; e < 8 * 128; e += blockDim.x) {
-    const int v = e & 127, st = e >> 7;
-    const int pt = sub[st];
-    if (pt < 0) continue;
-    const int c = v * 4;
-    const int x = (c & 7) + (st & 1) * 8, y = ((c >> 3) & 7) + ((st >> 1) & 1) * 8, z = (c >> 6) + (st >> 2) * 8;
-    reinterpret_cast<float4 *>(dst + (size_t)pt * SHKZ_TC)[v] = *reinterpret_cast<const float4 *>(srcs + x + 16 * y + 256 * z);
-  }
-}
-
-// With fu != null the kernel also performs the preceding x/r update of the
-// PCG iteration (k_update_xr's arithmetic and convergence bookkeeping, the
-// last CTA reducing the norms); the update's extra loads sit in the staging
-// phase, which overlaps the wait for the upstream faces.
-struct SweepUpdate {
-  const float *p, *q;
-  const float *p_alt;  // non-null: p / p_alt are the two direction buffers, the current one
-                       // chosen by the parity of st->iter + 1 (the stencil of this iteration wrote it)
-  float *x, *r;
-  SolverState *st;
-  unsigned *counter;
-  double *part;        // [2 * KM]: per-tile inf-norm, squared 2-norm
-  int max_iterations;
-};
-
-__global__ void __launch_bounds__(256, 2) k_mic_forward16(PoolSystem S, const float *__restrict__ d32,
-                                                       const float *__restrict__ r, float *__restrict__ t,
-                                                       unsigned long long *faces, WaveSync *ws, const SolverState *st,
-                                                       SweepUpdate fu) {
-  extern __shared__ __align__(16) float smf[];
-  float *Tg = smf, *R = Tg + MGC, *Dd = R + MTC, *WX = Dd + MTC, *WY = WX + MTC, *WZ = WY + MTC;
-  __shared__ int sub[8];
-  if (st && st->done) return;
-  int slot, epoch, limit;
-  sweep_begin(ws, slot, epoch, limit);
-  const int mt = S.msched[slot];
-  const int tid = threadIdx.x, jj = tid & 15, kk = tid >> 4;
-  if (tid < 8) sub[tid] = S.msub[mt * 8 + tid];
-  __syncthreads();
-  if (fu.st) {
-    __shared__ double red[8];
-    double m = 0.0, s2 = 0.0;
-    const float *pcur = (fu.p_alt && ((fu.st->iter + 1) & 1)) ? fu.p_alt : fu.p;
-    macro_load_update(sub, fu.r, fu.q, pcur, fu.x, (float)fu.st->alpha, d32, S.offx, S.offy, S.offz, R, Dd, WX, WY,
-                      WZ, m, s2);
-    m = block_max<256>(m, red);
-    s2 = block_sum<256>(s2, red);
-    if (tid == 0) {
-      fu.part[mt] = m;
-      fu.part[S.KM + mt] = s2;
-    }
-  } else {
-    macro_load5(sub, r, d32, S.offx, S.offy, S.offz, R, Dd, WX, WY, WZ);
-  }
-  __syncthreads();
-  // The thread's x-row in registers, rotated by its wavefront offset
-  // o = jj + kk: slot k holds cell (k - o) mod 16, so the cell of step s
-  // (x = s - o) sits in slot s mod 16, a constant of the unrolled step loop.
-  const int o = jj + kk;
-  float cd[MT], cr[MT], cx[MT], cy[MT], cz[MT];
-  {
-    const int rb = MT * jj + MT * MT * kk;
-    #pragma unroll
-    for (int k = 0; k < MT; ++k) {
-      const int c = rb + ((k - o) & (MT - 1));
-      cd[k] = Dd[c]; cr[k] = R[c]; cx[k] = WX[c]; cy[k] = WY[c]; cz[k] = WZ[c];
-    }
-  }
-  float tx;
-  {
-    const int nxm = S.mnbr[mt * 6 + NB_XM], nym = S.mnbr[mt * 6 + NB_YM], nzm = S.mnbr[mt * 6 + NB_ZM];
-    const int u = tid & 15, v = tid >> 4;
-    bool ok = true;
-    float gx, gy, gz;
-    face_get3(nxm >= 0 ? faces + ((size_t)nxm * 3 + 0) * 256 + tid : nullptr,
-              nym >= 0 ? faces + ((size_t)nym * 3 + 1) * 256 + tid : nullptr,
-              nzm >= 0 ? faces + ((size_t)nzm * 3 + 2) * 256 + tid : nullptr, epoch, limit, gx, gy, gz, ok);
-    Tg[mghost(-1, u, v)] = gx;
-    Tg[mghost(u, -1, v)] = gy;
-    Tg[mghost(u, v, -1)] = gz;
-    tx = gx;
-    if (!ok) atomicCAS(&ws->error, 0, slot + 1);
-  }
-  __syncthreads();
-  {
-    const int gb = mghost(0, jj, kk) - o;
-    #pragma unroll
-    for (int s = 0; s < 3 * MT - 2; ++s) {
-      if ((unsigned)(s - o) < (unsigned)MT) {
-        const int g = s + gb, k = s & (MT - 1);
-        const float ty = Tg[g - MGY], tz = Tg[g - MGZ];
-        tx = cd[k] * (cr[k] + cx[k] * tx + cy[k] * ty + cz[k] * tz);
-        Tg[g] = tx;
-      }
-      __syncthreads();
-    }
-  }
-  if (*((volatile const int *)&ws->skip_publish) != slot + 1) {
-    unsigned long long *f = faces + (size_t)mt * 3 * 256;
-    const int u = tid & 15, v = tid >> 4;
-    face_put(f + 0 * 256 + tid, epoch, Tg[mghost(15, u, v)]);
-    face_put(f + 1 * 256 + tid, epoch, Tg[mghost(u, 15, v)]);
-    face_put(f + 2 * 256 + tid, epoch, Tg[mghost(u, v, 15)]);
-  }
-  macro_store_ghosted(sub, Tg, t);
-  if (fu.st && last_block(fu.counter)) {
-    // the convergence bookkeeping of k_update_xr, on the new residual
-    __shared__ double red2[8];
-    double mm = 0.0, ss = 0.0;
-    for (int i = tid; i < S.KM; i += 256) {
-      mm = fmax(mm, fu.part[i]);
-      ss += fu.part[S.KM + i];
-    }
-    mm = block_max<256>(mm, red2);
-    ss = block_sum<256>(ss, red2);
-    const bool nan = !(ss == ss);
-    if (tid == 0) {
-      SolverState *sw = fu.st;
-      sw->rmax = nan ? CUDART_NAN : mm;
-      sw->r2 = ss;
-      sw->iter += 1;
-      if (nan) { sw->done = 3; sw->status = -5; }
-      else if (mm <= sw->tol_abs) sw->done = 1;
-      else if (sw->iter >= fu.max_iterations) sw->done = 2;
-      else if (mm < sw->ru_threshold) sw->done = 4;
-      *fu.counter = 0;
-    }
-  }
-  sweep_end(ws, epoch);
-}
-
-__global__ void __launch_bounds__(256, 2) k_mic_backward16(PoolSystem S, const float *__restrict__ d32,
-                                                        const float *__restrict__ t, const float *__restrict__ r,
-                                                        float *__restrict__ z, double *partials,
-                                                        unsigned long long *faces, WaveSync *ws,
-                                                        SolverState *st, unsigned *finish) {
-  extern __shared__ __align__(16) float smb[];
-  float *Zg = smb, *Tt = Zg + MGC, *Dd = Tt + MTC, *WX = Dd + MTC, *WY = WX + MTC, *WZ = WY + MTC;
-  __shared__ int sub[8];
-  __shared__ double red[8];
-  if (st && st->done) return;
-  int slot, epoch, limit;
-  sweep_begin(ws, slot, epoch, limit);
-  const int mt = S.msched[S.KM - 1 - slot];
-  const int tid = threadIdx.x, jj = tid & 15, kk = tid >> 4;
-  if (tid < 8) sub[tid] = S.msub[mt * 8 + tid];
-  __syncthreads();
-  // the upper weights come precomputed (launch_upper_weights): W?[c] is the
-  // lower weight of the +x/+y/+z neighbour cell, across the macro face where
-  // needed, so the sweep reads them at the cell's own index
-  macro_load5(sub, t, d32, S.upx, S.upy, S.upz, Tt, Dd, WX, WY, WZ);
-  const int nxp = S.mnbr[mt * 6 + NB_XP], nyp = S.mnbr[mt * 6 + NB_YP], nzp = S.mnbr[mt * 6 + NB_ZP];
-  __syncthreads();
-  // the thread's x-row in registers, rotated as in the forward sweep: slot k
-  // holds cell (k - o) mod 16
-  const int o = jj + kk;
-  float ct[MT], cd[MT], cx[MT], cy[MT], cz[MT];
-  {
-    const int rb = MT * jj + MT * MT * kk;
-    #pragma unroll
-    for (int k = 0; k < MT; ++k) {
-      const int c = rb + ((k - o) & (MT - 1));
-      ct[k] = Tt[c]; cd[k] = Dd[c]; cx[k] = WX[c]; cy[k] = WY[c]; cz[k] = WZ[c];
-    }
-  }
-  float zx;
-  {
-    const int u = tid & 15, v = tid >> 4;
-    bool ok = true;
-    float gx, gy, gz;
-    face_get3(nxp >= 0 ? faces + ((size_t)nxp * 3 + 0) * 256 + tid : nullptr,
-              nyp >= 0 ? faces + ((size_t)nyp * 3 + 1) * 256 + tid : nullptr,
-              nzp >= 0 ? faces + ((size_t)nzp * 3 + 2) * 256 + tid : nullptr, epoch, limit, gx, gy, gz, ok);
-    Zg[mghost(MT, u, v)] = gx;
-    Zg[mghost(u, MT, v)] = gy;
-    Zg[mghost(u, v, MT)] = gz;
-    zx = gx;
-    if (!ok) atomicCAS(&ws->error, 0, slot + 1);
-  }
-  __syncthreads();
-  {
-    const int gb = mghost(0, jj, kk) - o;
-    #pragma unroll
-    for (int s = 3 * MT - 3; s >= 0; --s) {
-      if ((unsigned)(s - o) < (unsigned)MT) {
-        const int g = s + gb, k = s & (MT - 1);
-        const float zy = Zg[g + MGY], zz = Zg[g + MGZ];
-        zx = ct[k] + cd[k] * (cx[k] * zx + cy[k] * zy + cz[k] * zz);
-        Zg[g] = zx;
-      }
-      __syncthreads();
-    }
-  }
-  {
-    unsigned long long *f = faces + (size_t)mt * 3 * 256;
-    const int u = tid & 15, v = tid >> 4;
-    face_put(f + 0 * 256 + tid, epoch, Zg[mghost(0, u, v)]);
-    face_put(f + 1 * 256 + tid, epoch, Zg[mghost(u, 0, v)]);
-    face_put(f + 2 * 256 + tid, epoch, Zg[mghost(u, v, 0)]);
-  }
-  macro_store_ghosted(sub, Zg, z);
-  // fused z.r over the macro tile's cells (absent sub-tiles contribute zero)
-  double dot = 0.0;
-  for (int e = tid; e < 8 * 128; e += 256) {
-    const int v = e & 127, stt = e >> 7;
-    const int pt = sub[stt];
-    if (pt < 0) continue;
-    const int c = v * 4;
-    const int x = (c & 7) + (stt & 1) * 8, y = ((c >> 3) & 7) + ((stt >> 1) & 1) * 8, zc = (c >> 6) + (stt >> 2) * 8;
-    const int o = mghost(x, y, zc);
-    const float4 rv = reinterpret_cast<const float4 *>(r + (size_t)pt * SHKZ_TC)[v];
-    dot += (double)Zg[o] * rv.x + (double)Zg[o + 1] * rv.y + (double)Zg[o + 2] * rv.z + (double)Zg[o + 3] * rv.w;
-  }
-  const double tot = block_sum<256>(dot, red);
-  if (tid == 0 && partials) partials[mt] = tot;
-  if (finish && last_block(finish)) {
-    // k_finish_rho of the PCG iteration: rho_new = z.r from the macro-tile
-    // partials in tile order, beta = rho_new / rho
-    const double rho_new = sum_partials<256>(partials, S.KM, red);
-    if (tid == 0) {
-      st->beta = rho_new / st->rho;
-      st->rho = rho_new;
-      *finish = 0;
-    }
-  }
-  sweep_end(ws, epoch);
-}
-
-// Upper weights of every pool cell: the lower weight of the +x/+y/+z
-// neighbour cell (A(i, i+e) = -off?(i+e)), from the neighbour tile across a
-// tile face, zero where that tile is not in the pool. They depend on the
-// matrix only, so the backward MIC(0) sweep stages them instead of shifting
-// the lower weights every iteration.
-__global__ void __launch_bounds__(256) k_upper_weights(PoolSystem S, float *__restrict__ upx,
-                                                       float *__restrict__ upy, float *__restrict__ upz) {
-  const long long n = (long long)S.K * SHKZ_TC;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int pt = (int)(i >> 9), c = (int)(i & 511);
-    const int ii = c & 7, jj = (c >> 3) & 7, kk = c >> 6;
-    const size_t base = (size_t)pt * SHKZ_TC;
-    float ux = 0.f, uy = 0.f, uz = 0.f;
-    if (ii < 7) ux = S.offx[base + c + 1];
-    else if (S.nbr[pt * 6 + NB_XP] >= 0) ux = S.offx[(size_t)S.nbr[pt * 6 + NB_XP] * SHKZ_TC + c - 7];
-    if (jj < 7) uy = S.offy[base + c + 8];
-    else if (S.nbr[pt * 6 + NB_YP] >= 0) uy = S.offy[(size_t)S.nbr[pt * 6 + NB_YP] * SHKZ_TC + c - 56];
-    if (kk < 7) uz = S.offz[base + c + 64];
-    else if (S.nbr[pt * 6 + NB_ZP] >= 0) uz = S.offz[(size_t)S.nbr[pt * 6 + NB_ZP] * SHKZ_TC + c - 448];
-    upx[i] = ux;
-    upy[i] = uy;
-    upz[i] = uz;
-  }
-}
-
-static int grid_for(long long n, int per, int cap);
-void launch_upper_weights(const PoolSystem &S, float *upx, float *upy, float *upz, cudaStream_t s) {
-  if (S.K <= 0) return;
-  count_launches(1);
-  k_upper_weights<<<grid_for((long long)S.K * SHKZ_TC, 256 * 4, 148 * 8), 256, 0, s>>>(S, upx, upy, upz);
-}
-
-size_t mic16_smem_forward() { return sizeof(float) * (MGC + 5 * MTC); }
-size_t mic16_smem_backward() { return sizeof(float) * (MGC + 5 * MTC); }
 
 // ---------------------------------------------------------------------------
 // FP64 residual r64 = b64 - A64 x64 (x64 in FP64), its norms, and the FP32
@@ -1288,6 +904,21 @@ __global__ void __launch_bounds__(256) k_accumulate(int n, const float *__restri
     x64[i] += scale * (double)x32[i];
 }
 
+// The same with the last iteration's x update, which the fused iteration
+// leaves to its next stencil: x64 += scale * (x32 + alpha p). p0 holds the
+// direction after an even number of completed iterations, p1 after an odd one.
+__global__ void __launch_bounds__(256) k_accumulate_pending(int n, const float *__restrict__ x32,
+                                                            const float *p0, const float *p1, const SolverState *st,
+                                                            double scale, double *__restrict__ x64) {
+  const float alpha = st->x_pending ? (float)st->alpha : 0.0f;
+  const float *__restrict__ p = (st->iter & 1) ? p1 : p0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float x = x32[i];
+    x += alpha * p[i];
+    x64[i] += scale * (double)x;
+  }
+}
+
 __global__ void __launch_bounds__(256) k_to_float(int n, const double *__restrict__ a, float *__restrict__ b) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = (float)a[i];
 }
@@ -1326,6 +957,7 @@ __global__ void __launch_bounds__(256) k_inner_setup(int n, const float *__restr
       if (!(ss == ss)) st->done = 3;
       st->rho = 0.0;
       st->beta = 0.0;
+      st->x_pending = 0;
       st->ru_threshold = 0.0;
       *counter = 0;
     }
@@ -1335,6 +967,7 @@ __global__ void __launch_bounds__(256) k_inner_setup(int n, const float *__restr
 // Host-directed state edits between batches (one thread).
 __global__ void k_state_resume(SolverState *st, double ru_threshold, int iter_offset) {
   st->done = 0;
+  st->x_pending = 0;  // folded in by launch_accumulate_pending
   st->ru_threshold = ru_threshold;
   (void)iter_offset;
 }
@@ -1598,13 +1231,14 @@ void pool_assign(const Geometry &G, const int *tile_count, int K, const int *scr
   count_launches(1);
   k_pool_assign<<<nb, 1024, 0, s>>>(tile_count, nt, scratch_bsum, tile_state, pool_tile);
   const int nlev = G.bx + G.by + G.bz;
-  cudaMemsetAsync(level_count, 0, sizeof(int) * (nlev + 1), s);
+  if (sched) cudaMemsetAsync(level_count, 0, sizeof(int) * (nlev + 1), s);
   if (K > 0) {
     count_launches(1);
-    k_pool_neighbours<<<(K + 255) / 256, 256, 0, s>>>(G, tile_state, pool_tile, K, nbr, level_count);
-    count_launches(1);
+    k_pool_neighbours<<<(K + 255) / 256, 256, 0, s>>>(G, tile_state, pool_tile, K, nbr, sched ? level_count : nullptr);
+  }
+  if (K > 0 && sched) {
+    count_launches(2);
     k_level_scan<<<1, 32, 0, s>>>(level_count, nlev);
-    count_launches(1);
     k_level_scatter<<<(K + 255) / 256, 256, 0, s>>>(G, pool_tile, K, level_count, sched);
   }
 }
@@ -1615,14 +1249,14 @@ void launch_spmv(const PoolSystem &S, const float *p, float *q, double *partials
                  int mode, cudaStream_t s) {
   if (S.K <= 0) return;
   count_launches(1);
-  k_spmv<<<spmv_grid(S.K), 128, 0, s>>>(S, p, q, partials, counter, st, mode, nullptr, nullptr);
+  k_spmv<<<spmv_grid(S.K), 128, 0, s>>>(S, p, q, partials, counter, st, mode, nullptr, nullptr, nullptr);
 }
 
-void launch_spmv_update(const PoolSystem &S, float *p0, float *p1, const float *z, float *q, double *partials,
-                        unsigned *counter, SolverState *st, cudaStream_t s) {
+void launch_spmv_update(const PoolSystem &S, float *p0, float *p1, const float *z, float *q, float *x,
+                        double *partials, unsigned *counter, SolverState *st, cudaStream_t s) {
   if (S.K <= 0) return;
   count_launches(1);
-  k_spmv<<<spmv_grid(S.K), 128, 0, s>>>(S, p0, q, partials, counter, st, 0, z, p1);
+  k_spmv<<<spmv_grid(S.K), 128, 0, s>>>(S, p0, q, partials, counter, st, 0, z, p1, x);
 }
 
 // one wave of resident CTAs looping over the tiles
@@ -1658,6 +1292,7 @@ void launch_mic_factor(const PoolSystem &S, double *colsum, double omega, double
   k_mic_colsum<<<S.K, 512, 0, s>>>(S, colsum);
   count_launches(1);
   k_mic_factor<<<S.K, 64, 0, s>>>(S, S.sched, colsum, omega, min_ratio, d64, d32, flags, (WaveSync *)ws);
+  if (S.KM > 0) launch_pencil_coefs(S, d32, s);
 }
 
 void launch_mic_apply(const PoolSystem &S, const float *d32, const float *r, float *t, float *z, double *partials,
@@ -1665,20 +1300,7 @@ void launch_mic_apply(const PoolSystem &S, const float *d32, const float *r, flo
                       const SolverState *st, cudaStream_t s) {
   if (S.K <= 0) return;
   if (S.KM > 0) {
-    static bool attr[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !attr[dev]) {
-      cudaFuncSetAttribute(k_mic_forward16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mic16_smem_forward());
-      cudaFuncSetAttribute(k_mic_backward16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mic16_smem_backward());
-      if (dev >= 0 && dev < 64) attr[dev] = true;
-    }
-    count_launches(2);
-    k_mic_forward16<<<S.KM, 256, mic16_smem_forward(), s>>>(S, d32, r, t, S.mfaces_f, (WaveSync *)ws_f, st,
-                                                             SweepUpdate{});
-    k_mic_backward16<<<S.KM, 256, mic16_smem_backward(), s>>>(S, d32, t, r, z, partials, S.mfaces_b,
-                                                               (WaveSync *)ws_b, const_cast<SolverState *>(st),
-                                                               nullptr);
+    launch_pencil_sweeps(S, r, z, partials, ws_f, ws_b, st, SweepUpdate{}, nullptr, s);
     return;
   }
   count_launches(1);
@@ -1687,43 +1309,29 @@ void launch_mic_apply(const PoolSystem &S, const float *d32, const float *r, flo
   k_mic_backward<<<S.K, 64, 0, s>>>(S, S.sched, d32, t, r, z, partials, faces_b, (WaveSync *)ws_b, st);
 }
 
-bool launch_mic_apply_update(const PoolSystem &S, const float *d32, float *r, float *t, float *z, double *partials,
-                             const float *p, const float *p_alt, const float *q, float *x, unsigned *counter,
-                             SolverState *st, int max_iterations, void *ws_f, void *ws_b, unsigned *finish,
-                             cudaStream_t s) {
+bool launch_mic_apply_update(const PoolSystem &S, float *r, float *z, double *partials, const float *q,
+                             unsigned *counter, SolverState *st, int max_iterations, void *ws_f, void *ws_b,
+                             unsigned *finish, cudaStream_t s) {
   if (S.K <= 0 || S.KM <= 0) return false;
-  static bool attr[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !attr[dev]) {
-    cudaFuncSetAttribute(k_mic_forward16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mic16_smem_forward());
-    cudaFuncSetAttribute(k_mic_backward16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mic16_smem_backward());
-    if (dev >= 0 && dev < 64) attr[dev] = true;
-  }
   SweepUpdate fu;
-  fu.p = p;
-  fu.p_alt = p_alt;
   fu.q = q;
-  fu.x = x;
   fu.r = r;
   fu.st = st;
   fu.counter = counter;
   fu.part = partials;  // [2 KM]; the backward sweep then writes its z.r partials over [0, KM)
   fu.max_iterations = max_iterations;
-  count_launches(2);
-  k_mic_forward16<<<S.KM, 256, mic16_smem_forward(), s>>>(S, d32, r, t, S.mfaces_f, (WaveSync *)ws_f, st, fu);
-  k_mic_backward16<<<S.KM, 256, mic16_smem_backward(), s>>>(S, d32, t, r, z, partials, S.mfaces_b, (WaveSync *)ws_b,
-                                                             st, finish);
+  launch_pencil_sweeps(S, r, z, partials, ws_f, ws_b, st, fu, finish, s);
   return true;
 }
 
 void build_macro(const Geometry &G, const Geometry &M, const int *tile_count, const int *tile_state, int *macro_count,
-                 int *macro_state, int *macro_tile, int *mnbr, int *level_count, int *msched, int *msub, int KM,
+                 int *macro_state, int *macro_tile, int *mnbr, int *level_count, int2 *seg, int2 *mseg, int *nseg, int *msub, int KM,
                  const int *bsum, cudaStream_t s) {
-  pool_assign(M, macro_count, KM, bsum, macro_state, macro_tile, mnbr, level_count, msched, s);
+  pool_assign(M, macro_count, KM, bsum, macro_state, macro_tile, mnbr, nullptr, nullptr, s);
   if (KM > 0) {
     count_launches(1);
     k_macro_sub<<<(KM * 8 + 255) / 256, 256, 0, s>>>(G, M, macro_tile, KM, tile_state, msub);
+    build_pencils(M, macro_tile, mnbr, KM, level_count, seg, mseg, nseg, s);
   }
 }
 
@@ -1746,6 +1354,11 @@ void launch_inner_init(int n, const double *r64, double inv_scale, float *r32, f
 void launch_accumulate(int n, const float *x32, double scale, double *x64, cudaStream_t s) {
   count_launches(1);
   k_accumulate<<<grid_for(n, 256 * 4, 148 * 8), 256, 0, s>>>(n, x32, scale, x64);
+}
+void launch_accumulate_pending(int n, const float *x32, const float *p0, const float *p1, const SolverState *st,
+                               double scale, double *x64, cudaStream_t s) {
+  count_launches(1);
+  k_accumulate_pending<<<grid_for(n, 256 * 4, 148 * 8), 256, 0, s>>>(n, x32, p0, p1, st, scale, x64);
 }
 void launch_to_float(int n, const double *a, float *b, cudaStream_t s) {
   count_launches(1);
