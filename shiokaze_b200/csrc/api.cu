@@ -20,6 +20,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <unordered_map>
 #include <vector>
 
@@ -92,10 +93,13 @@ struct shkz_b200_ctx {
   int cap_warm_pool = 0;
   size_t cap_rank_cnt = 0;
   float *h_dens[3] = {};           // staging of the solid density faces (host path)
-  float *ext_v[3] = {};            // velocity extension: side buffer of new values per component
-  uint8_t *ext_a[3] = {};          // and its flags
+  float *ext_v[3] = {};            // velocity extension: the constraint's new values per component
+  unsigned *ext_bits[3][2] = {};   // and the masks before and after a pass, as bits
   size_t cap_ext[3] = {0, 0, 0};
-  int *ext_flag = nullptr;         // levelset_exist(solid) of the extension's constraint
+  unsigned *ext_solid = nullptr;   // solid nodes as bits
+  size_t cap_ext_solid = 0;
+  unsigned *ext_list[3] = {};      // faces the constraint looks at
+  unsigned *ext_flag = nullptr;    // [4]: their numbers, levelset_exist(solid)
   // FLIP splat (splat.cu)
   unsigned char *sp_raw = nullptr;  // particle records (host path)
   size_t cap_sp_raw = 0;
@@ -411,7 +415,9 @@ extern "C" void shkz_b200_destroy(shkz_b200_ctx *ctx) {
                   ctx->coef_b, ctx->tp, ctx->curv,
                   ctx->prev, ctx->rank_pool, ctx->rank_cnt, ctx->rank_total, ctx->xw, ctx->h_dens[0],
                   ctx->h_dens[1], ctx->h_dens[2], ctx->flush, ctx->pb, ctx->ext_v[0], ctx->ext_v[1], ctx->ext_v[2],
-                  ctx->ext_a[0], ctx->ext_a[1], ctx->ext_a[2], ctx->ext_flag, ctx->sp_raw, ctx->sp_posm,
+                  ctx->ext_bits[0][0], ctx->ext_bits[0][1], ctx->ext_bits[1][0],
+                  ctx->ext_bits[1][1], ctx->ext_bits[2][0], ctx->ext_bits[2][1], ctx->ext_solid, ctx->ext_flag,
+                  ctx->ext_list[0], ctx->ext_list[1], ctx->ext_list[2], ctx->sp_raw, ctx->sp_posm,
                   ctx->sp_vc[0], ctx->sp_vc[1], ctx->sp_vc[2], ctx->sp_key, ctx->sp_rank, ctx->sp_list, ctx->sp_sposm,
                   ctx->sp_svc, ctx->sp_faces, ctx->sp_sorted, ctx->sp_face_bin, ctx->sp_nfaces, ctx->sp_work,
                   ctx->sp_count, ctx->sp_tile_start, ctx->sp_tile_act, ctx->sp_tiles, ctx->sp_act[0],
@@ -1032,38 +1038,53 @@ static int validate_extend(const shkz_b200_extend_args *a) {
 
 static int extend_device(shkz_b200_ctx *ctx, const shkz_b200_extend_args *a) {
   cudaStream_t s = ctx->stream;
-  size_t nf[3];
+  ExtendFields f{};
+  f.nx = a->nx;
+  f.ny = a->ny;
+  f.nz = a->nz;
+  f.dx = a->dx;
   for (int d = 0; d < 3; ++d) {
-    nf[d] = (size_t)(a->nx + (d == 0)) * (a->ny + (d == 1)) * (a->nz + (d == 2));
-    if (nf[d] > ctx->cap_ext[d]) {
-      GROW(ext_v[d], nf[d]);
-      GROW(ext_a[d], nf[d]);
-      ctx->cap_ext[d] = nf[d];
+    f.W[d] = a->nx + (d == 0);
+    f.H[d] = a->ny + (d == 1);
+    f.D[d] = a->nz + (d == 2);
+    const size_t nf = (size_t)f.W[d] * f.H[d] * f.D[d];
+    if (nf > ctx->cap_ext[d]) {
+      GROW(ext_v[d], nf);
+      GROW(ext_list[d], nf);
+      GROW(ext_bits[d][0], (nf + 31) / 32);
+      GROW(ext_bits[d][1], (nf + 31) / 32);
+      ctx->cap_ext[d] = nf;
     }
+    f.n[d] = (unsigned)nf;
+    f.vel[d] = a->velocity[d];
+    f.act[d] = a->velocity_active[d];
+    f.bits[d] = ctx->ext_bits[d][0];
+    f.next[d] = ctx->ext_bits[d][1];
+    f.list[d] = ctx->ext_list[d];
+    f.side[d] = ctx->ext_v[d];
   }
-  if (!ctx->ext_flag) GROW(ext_flag, 1);
-  // ext_v / ext_a are a side buffer and its flags; the flags start (and end) zero
-  for (int d = 0; d < 3; ++d) SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->ext_a[d], 0, nf[d], s));
-  for (int d = 0; d < 3; ++d) {
-    const int W = a->nx + (d == 0), H = a->ny + (d == 1), D = a->nz + (d == 2);
-    for (int w = 0; w < a->width; ++w)
-      launch_extrapolate(W, H, D, a->velocity[d], a->velocity_active[d], ctx->ext_v[d], ctx->ext_a[d], s);
+  if (!ctx->ext_flag) GROW(ext_flag, 4);
+  launch_ext_pack(f, s);
+  for (int w = 0; w < a->width; ++w) {
+    launch_extrapolate(f, s);
+    for (int d = 0; d < 3; ++d) std::swap(f.bits[d], f.next[d]);
   }
   if (a->constrain) {
-    ConstrainFields f;
-    for (int d = 0; d < 3; ++d) {
-      f.save[d] = a->velocity[d];
-      f.act[d] = a->velocity_active[d];
-    }
-    SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->ext_flag, 0, sizeof(int), s));
     if (a->solid) {
       const size_t nodes = (size_t)(a->nx + 1) * (a->ny + 1) * (a->nz + 1);
-      launch_solid_exists(a->solid, a->solid_active, nodes, ctx->ext_flag, s);
+      if (nodes > ctx->cap_ext_solid) {
+        GROW(ext_solid, (nodes + 31) / 32);
+        ctx->cap_ext_solid = nodes;
+      }
     }
+    f.solid = a->solid;
+    f.solid_bits = ctx->ext_solid;
+    f.listed = ctx->ext_flag;
+    int *solid_flag = reinterpret_cast<int *>(ctx->ext_flag + 3);
+    f.solid_flag = solid_flag;
+    SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->ext_flag, 0, 4 * sizeof(unsigned), s));
     // all three components are found on the unchanged field, then committed
-    for (int d = 0; d < 3; ++d)
-      launch_constrain_find(d, a->nx, a->ny, a->nz, a->dx, a->solid, ctx->ext_flag, f, ctx->ext_v[d], ctx->ext_a[d], s);
-    for (int d = 0; d < 3; ++d) launch_apply_side(nf[d], a->velocity[d], ctx->ext_v[d], ctx->ext_a[d], s);
+    launch_constrain(f, a->solid_active, solid_flag, s);
   }
   SHKZ_CUDA_TRY(cudaGetLastError());
   SHKZ_CUDA_TRY(cudaStreamSynchronize(s));

@@ -55,18 +55,27 @@ void launch_coeff(const AssemblyInputs &in, const int *flags, const int *pool_ti
 void launch_velocity_update(const AssemblyInputs &in, const int *flags, const int *tile_state,
                             const float *pressure_pool, float *const vel[3], uint8_t *const vact[3], cudaStream_t s);
 // velocity extension after a projection (extend.cu)
-struct ConstrainFields {
-  const float *save[3];    // the velocity components (read-only while the constraint is found)
-  const uint8_t *act[3];   // their active masks
+struct ExtendFields {
+  int nx, ny, nz;
+  double dx;
+  int W[3], H[3], D[3];    // extents of the face grids, n = W H D faces each
+  unsigned n[3];
+  float *vel[3];           // the velocity components and their active masks, updated in place
+  uint8_t *act[3];
+  unsigned *bits[3];       // active masks as bits, (n + 31) / 32 words
+  unsigned *next[3];       // the masks after a pass
+  unsigned *list[3];       // faces the constraint may change (room for all), and their new values
+  float *side[3];
+  unsigned *listed;        // [3] how many
+  const float *solid;      // nodes, or null
+  unsigned *solid_bits;    // nodes that are not outside the solid
+  const int *solid_flag;   // whether the solid level set exists
 };
-// one extrapolation pass in place: frontier values into side/flag, then committed
-// (flag must be all zero on entry and is all zero again on return)
-void launch_extrapolate(int W, int H, int D, float *v, uint8_t *a, float *side, uint8_t *flag, cudaStream_t s);
-void launch_solid_exists(const float *solid, const uint8_t *act, size_t n, int *flag, cudaStream_t s);
-// constrained values of component d that differ from the field, into side/flag
-void launch_constrain_find(int d, int nx, int ny, int nz, double dx, const float *solid, const int *solid_flag,
-                           const ConstrainFields &f, float *side, uint8_t *flag, cudaStream_t s);
-void launch_apply_side(size_t n, float *v, const float *side, uint8_t *flag, cudaStream_t s);
+// byte masks into bits; one extrapolation pass (bits -> next); the constraint
+// (on bits; listed and *solid_flag zeroed by the caller)
+void launch_ext_pack(const ExtendFields &f, cudaStream_t s);
+void launch_extrapolate(const ExtendFields &f, cudaStream_t s);
+void launch_constrain(const ExtendFields &f, const uint8_t *solid_active, int *solid_flag, cudaStream_t s);
 
 // FLIP splat (splat.cu). Particle records read in place: float fields at byte
 // offsets (multiples of 4) of `stride`-byte records.

@@ -104,3 +104,30 @@ def test_extension_without_constraint_or_passes_and_argument_errors():
     assert L.shkz_b200_extend_velocity_host(ctx.handle, ctypes.byref(e)) == -1
     e.nx, e.width = 4, -1
     assert L.shkz_b200_extend_velocity_host(ctx.handle, ctypes.byref(e)) == -1
+
+
+@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 2, 5), (31, 3, 4), (32, 5, 3), (33, 17, 6), (64, 9, 11), (95, 12, 7)])
+@pytest.mark.parametrize("with_solid", [False, True])
+def test_extension_on_odd_grids_bitexact(shape, with_solid):
+    """Rows shorter than, equal to and longer than the 32 faces of a mask
+    word, random masks (any nonzero byte is active), a solid that cuts the
+    grid: the packed-mask passes against the oracle."""
+    from shiokaze_b200 import native
+    nx, ny, nz = shape
+    rng = np.random.default_rng(nx + 7 * ny + 31 * nz)
+    dx = 1.0 / max(shape)
+    vel = [rng.standard_normal((nz + (d == 2), ny + (d == 1), nx + (d == 0))).astype(np.float32) for d in range(3)]
+    act = [((rng.random(v.shape) < 0.15) * rng.integers(1, 256, v.shape)).astype(np.uint8) for v in vel]
+    for d in range(3):
+        vel[d] = np.where(act[d] != 0, vel[d], np.float32(0))
+    solid = sact = None
+    if with_solid:
+        k, j, i = np.meshgrid(*[np.arange(n + 1) for n in (nz, ny, nx)], indexing="ij")
+        solid = (dx * (np.abs(i - 0.4 * nx) + 0.7 * np.abs(j - 0.5 * ny) + 0.6 * np.abs(k - 0.5 * nz) - 0.45 * min(shape)
+                       + 0.3 * rng.standard_normal(i.shape))).astype(np.float32)
+        sact = np.ones(solid.shape, np.uint8)
+    ctx = native.Context(native.default_config())
+    for width in (0, 1, 4):
+        got_v, got_a = native.extend_velocity(ctx, vel, act, solid, sact, dx, width, True)
+        want_v, want_a = ext.extend(vel, act, solid, sact, dx, width, True)
+        _assert_same(got_v, got_a, want_v, want_a)
