@@ -380,7 +380,7 @@ int shkz_b200_conv3d(int nx, int ny, int nz, int c0, int c1, int cout, int plane
  * waits for the stream to drain and reads the kernel's error word back before
  * it returns. in0, in1 and out must start on 16-byte boundaries and w, bias on
  * 4-byte boundaries (SHKZ_B200_ERR_ARG otherwise). Its scratch (packed
- * weights, block flags, an error word) is a fixed 1.1 MiB array in the library
+ * weights, an error word) is a fixed 0.85 MiB array in the library
  * that each GPU holds until exit. Limits: cout in {16, 32, 64, 128}, c0 + c1 <=
  * 128 (both multiples of 16), planes x max(cout, 32) <= 512 tensor-memory
  * columns (planes = 8 only with cout <= 64), at most 2^18 output blocks of

@@ -55,12 +55,14 @@ __global__ void __launch_bounds__(128, 1) k_conv_tc(ConvArgs a, const __grid_con
   bid /= a.gbx;
   const int byi = bid % a.gby;
   const int bzi = bid / a.gby;
-  if (!a.block_act[((size_t)bzi * a.gby + byi) * a.gbx + bxi]) return;  // whole CTA
+  if (a.block_act && !a.block_act[((size_t)bzi * a.gby + byi) * a.gbx + bxi]) return;  // whole CTA
   const int X0 = bxi * 8, Y0 = byi * 16, Z0 = bzi * 8 + zpart * P;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  // each plane's accumulator starts on a 32-column boundary of TMEM
-  const int pstride = (a.cout + 31) & ~31;
+  // merged taps: the planes' accumulators lie side by side in TMEM; else each
+  // starts on a 32-column boundary
+  const bool merged = conv_merged(a.cout);
+  const int pstride = merged ? a.cout : (a.cout + 31) & ~31;
   uint32_t ncols = 32;
   while (ncols < (uint32_t)(P * pstride)) ncols <<= 1;
   if (warp == 0) {
@@ -78,6 +80,17 @@ __global__ void __launch_bounds__(128, 1) k_conv_tc(ConvArgs a, const __grid_con
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  if (merged) {
+    // a merged MMA adds to planes that are at different taps, so all start from zero
+    for (int c = 0; c < P * pstride; c += 16)
+      asm volatile(
+          "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(
+              tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c),
+          "r"(0)
+          : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // the staging barrier below follows
+  }
 
   const int nchunk = (a.c0 + a.c1) / 16;
   const uint32_t idesc = umma_idesc_bf16(a.cout);
@@ -154,8 +167,26 @@ __global__ void __launch_bounds__(128, 1) k_conv_tc(ConvArgs a, const __grid_con
       // 14 bits and shared addresses stay below 2^18, so a tap's descriptor is
       // the base descriptor plus the tap's offset in 16-byte units.
       const uint64_t da0 = umma_desc(halo_s, LBO_A, 160);
-      const uint64_t db0 = umma_desc(w_s, (uint32_t)a.cout * 16, 128);
-      for (int zo = 0; zo < P; ++zo) {
+      const uint64_t db0 = umma_desc(w_s, (uint32_t)(merged ? 3 * a.cout : a.cout) * 16, 128);
+      // Merged: halo plane zi is tap dz of output plane zi - dz, so one MMA with
+      // the weights of up to three dz side by side (dz descending) adds to that
+      // many neighbouring accumulators. Every output still takes its taps in
+      // the order dz, dy, dx.
+      for (int zi = 0; merged && zi < P + 2; ++zi) {
+        const int lo = zi < 2 ? 0 : zi - 2, hi = zi < P ? zi : P - 1, n = (hi - lo + 1) * a.cout;
+        const uint32_t d_tmem = tmem + (uint32_t)(lo * pstride), id = umma_idesc_bf16(n);
+        const uint64_t db1 = db0 + (uint64_t)((2 - (zi - lo)) * a.cout);
+        for (int t = 0; t < 9; ++t) {
+          const uint64_t da = da0 + (uint64_t)((zi * 18 + t / 3) * 10 + t % 3);
+          const uint64_t db = db1 + (uint64_t)(t * 3 * a.cout * 2);
+          asm volatile(
+              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d_tmem),
+              "l"(da), "l"(db), "r"(id), "r"(1), "r"(0), "r"(0), "r"(0), "r"(0)
+              : "memory");
+        }
+      }
+      for (int zo = 0; !merged && zo < P; ++zo) {
         const uint32_t d_tmem = tmem + (uint32_t)(zo * pstride);
         int t = 0;
         for (int dz = 0; dz < 3; ++dz)
@@ -285,21 +316,28 @@ static void launch_conv_tc(ConvArgs a, int nblocks, size_t smem, cudaStream_t s)
 // ---------------------------------------------------------------------------
 // elementwise kernels
 
-// Packs FP32 weights w[27][cout][cin] into the per-chunk canonical layout;
+// Packs FP32 weights w[27][cout][cin] into the per-chunk canonical layout (with
+// merged taps the three dz of a (dy, dx) in one operand, dz descending);
 // transposed = 1 packs the input-gradient weights W'[t][ci][co] = W[26-t][co][ci]
 // (padded so that both channel counts are multiples of 16).
 __global__ void k_pack_weights(const float *w, int cout_real, int cin_real, int n_pad, int k_pad, int transposed,
-                               __nv_bfloat16 *out) {
-  // out element (chunk, t, kh, n/8, n%8, k8) for n < n_pad, k = chunk*16 + kh*8 + k8 < k_pad
+                               __nv_bfloat16 *out, int *clear = nullptr) {
+  if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;  // a word the next kernel needs zero
+  // out element (chunk, t, kh, n/8, n%8, k8) for n < n_pad, k = chunk*16 + kh*8 + k8 < k_pad;
+  // merged: (chunk, 3 dy + dx, kh, 2 - dz, n/8, n%8, k8)
+  const bool merged = conv_merged(n_pad);
   const int total = 27 * n_pad * k_pad;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
     int r = e;
     const int k8 = r & 7; r >>= 3;
     const int n8 = r & 7; r >>= 3;
     const int ng = r % (n_pad / 8); r /= (n_pad / 8);
+    int t = 0;
+    if (merged) { t = 9 * (2 - r % 3); r /= 3; }
     const int kh = r & 1; r >>= 1;
-    const int t = r % 27;
-    const int chunk = r / 27;
+    const int taps = merged ? 9 : 27;
+    t += r % taps;
+    const int chunk = r / taps;
     const int n = ng * 8 + n8, k = chunk * 16 + kh * 8 + k8;
     float v = 0.0f;
     if (!transposed) {
@@ -1185,23 +1223,16 @@ int conv3d_run(int nx, int ny, int nz, int c0, int c1, int cout, int planes, con
   return rc;
 }
 
-__global__ void k_fill_u8(uint8_t *a, int n, uint8_t v) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = v;
-}
-
 // The same convolution on device arrays with caller-provided scratch (packed
-// weights, block activity, error word); launches on `s` and returns without
-// synchronising. cout must be 16, 32, 64 or 128 (output stride = cout).
+// weights, error word); launches on `s` and returns without synchronising. cout must be 16, 32, 64 or 128 (output stride = cout).
 int conv3d_launch_scratch(int nx, int ny, int nz, int c0, int c1, int cout, int planes, const __nv_bfloat16 *in0,
                           const __nv_bfloat16 *in1, const float *w, const float *bias, int relu, __nv_bfloat16 *out,
-                          __nv_bfloat16 *wpk, uint8_t *act, int *err, cudaStream_t s) {
+                          __nv_bfloat16 *wpk, int *err, cudaStream_t s) {
   const int cin = c0 + c1;
   const int gbx = (nx + 7) / 8, gby = (ny + 15) / 16, gbz = (nz + 7) / 8;
   const int nb = gbx * gby * gbz;
-  count_launches(2);
-  k_pack_weights<<<256, 256, 0, s>>>(w, cout, cin, cout, cin, 0, wpk);
-  k_fill_u8<<<grid_blocks((size_t)nb, 256, 1024), 256, 0, s>>>(act, nb, 1);
-  if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return SHKZ_B200_ERR_CUDA;
+  count_launches(1);
+  k_pack_weights<<<256, 256, 0, s>>>(w, cout, cin, cout, cin, 0, wpk, err);
   ConvArgs a;
   a.in0 = in0;
   a.in1 = c1 ? in1 : nullptr;
@@ -1216,7 +1247,7 @@ int conv3d_launch_scratch(int nx, int ny, int nz, int c0, int c1, int cout, int 
   a.relu = relu;
   a.out = out;
   a.out32 = nullptr;
-  a.block_act = act;
+  a.block_act = nullptr;
   a.gbx = gbx; a.gby = gby; a.gbz = gbz;
   a.planes = planes;
   a.err = err;

@@ -6,9 +6,9 @@
 // loop that must not pay the device-wide synchronisation cudaMalloc/cudaFree
 // may imply. This entry point allocates nothing. The caller passes the inputs
 // and the output; the only scratch the kernel needs -- the weights packed in
-// the tensor-core layout, the block-activity array and an error word -- lives
-// in the file-scope array below, which every GPU that loads this library holds
-// until the process exits (1.1 MiB).
+// the tensor-core layout and an error word -- lives in the file-scope array
+// below, which every GPU that loads this library holds until the process exits
+// (0.85 MiB).
 //
 // Host code must not hand the array's name to a kernel: on the host it is a
 // stand-in symbol, not a device address. The first call on each device
@@ -16,8 +16,7 @@
 // cudaGetSymbolAddress; make that first call before any stream capture. Each
 // call waits for its stream to drain and reads the error word back before it
 // returns. All calls share the array and it keeps the last call's contents: each call
-// rewrites the packed weights and the activity bytes it uses and clears the
-// error word. Calls that overlap on the GPU (other streams, other host
+// rewrites the packed weights and clears the error word. Calls that overlap on the GPU (other streams, other host
 // threads) race on the array; serialise them.
 #include "common.cuh"
 #include "learned.h"
@@ -30,8 +29,8 @@ namespace {
 constexpr int kMaxCin = 128;                            // c0 + c1
 constexpr int kMaxCout = 128;
 constexpr size_t kWpkBytes = (size_t)27 * kMaxCout * kMaxCin * 2;  // packed BF16 weights
-constexpr size_t kMaxBlocks = (size_t)1 << 18;          // 8x16x8 output blocks (a 512^3 grid)
-constexpr size_t kScratchBytes = kWpkBytes + kMaxBlocks + 256;
+constexpr size_t kMaxBlocks = (size_t)1 << 18;          // documented limit: 8x16x8 output blocks (a 512^3 grid)
+constexpr size_t kScratchBytes = kWpkBytes + 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -83,15 +82,15 @@ extern "C" int shkz_b200_conv3d_noalloc(int nx, int ny, int nz, int c0, int c1, 
   int rc = scratch_base(dev, &base);
   if (rc) return rc;
   __nv_bfloat16 *wpk = reinterpret_cast<__nv_bfloat16 *>(base);
-  uint8_t *act = base + kWpkBytes;
-  int *err = reinterpret_cast<int *>(base + kWpkBytes + kMaxBlocks);
+  int *err = reinterpret_cast<int *>(base + kWpkBytes);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   rc = shkz::conv3d_launch_scratch(nx, ny, nz, c0, c1, cout, planes, reinterpret_cast<const __nv_bfloat16 *>(in0),
                                    reinterpret_cast<const __nv_bfloat16 *>(in1), w, bias, relu,
-                                   reinterpret_cast<__nv_bfloat16 *>(out), wpk, act, err, s);
+                                   reinterpret_cast<__nv_bfloat16 *>(out), wpk, err, s);
   if (rc) return rc;
-  if (cudaStreamSynchronize(s) != cudaSuccess) return SHKZ_B200_ERR_CUDA;
   int herr = 0;
-  if (cudaMemcpy(&herr, err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return SHKZ_B200_ERR_CUDA;
+  if (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess)
+    return SHKZ_B200_ERR_CUDA;
   return herr ? SHKZ_B200_ERR_TIMEOUT : 0;
 }

@@ -18,6 +18,16 @@
 // between the two 8-channel halves). One thread issues all MMAs; FP32
 // accumulators live in TMEM (P x Cout columns); tcgen05.commit signals an
 // mbarrier that all threads wait on (bounded) before the next chunk is staged.
+// For Cout <= 64 the taps are merged along z: what bounds such MMAs is reading A
+// (4 KB of shared memory, 32 cycles, for 8 - 32 cycles of multiply-adds at
+// N = 16 - 64), so the weights of the three dz of a (dy, dx) form one operand of
+// N = 3 Cout rows and one read of A serves three output planes, whose
+// accumulators are neighbours in TMEM: 9 (P + 2) MMAs per chunk for 27 P, and at
+// Cout = 16 room for three CTAs' accumulators on an SM. N <= 256 draws the line:
+// Cout = 128 keeps an MMA per tap. Measured on 128^3 voxels, B200, the whole
+// call, a tap an MMA -> merged: 16+32 -> 16 channels 359 -> 189 us, 32 -> 32
+// 261 -> 188, 32 -> 64 375 -> 310 (12 us of each from two launches and a
+// synchronisation less).
 // The epilogue reads each warp's 32 TMEM lanes (rows) with tcgen05.ld, adds
 // the bias, applies ReLU and stores BF16 channels-last (or channel 0 in FP32).
 #pragma once
@@ -40,7 +50,7 @@ struct ConvArgs {
   int relu;
   __nv_bfloat16 *out;         // channels-last, cout channels (or null)
   float *out32;               // FP32 channel 0 (or null)
-  const uint8_t *block_act;   // per 8x16x8 block, 1 = compute
+  const uint8_t *block_act;   // per 8x16x8 block, 1 = compute (null: all)
   int gbx, gby, gbz;          // blocks per axis
   int planes;                 // 8 or 4 z planes per CTA
   int *err;                   // set on a bounded-wait timeout
@@ -55,6 +65,9 @@ struct ConvArgs {
 struct ConvMaps {
   CUtensorMap m[2 * CONV_MAX_TMA_CHUNKS];
 };
+
+// Whether a convolution of this N runs with merged taps (it fixes the weights' packing).
+__host__ __device__ constexpr bool conv_merged(int cout) { return cout <= 64; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

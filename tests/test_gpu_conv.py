@@ -43,3 +43,21 @@ def test_conv_matches_numpy(shape, c0, c1, cout, planes):
     out, ref = run_conv(nx, ny, nz, c0, c1, cout, planes)
     err = np.linalg.norm(out - ref) / np.linalg.norm(ref)
     assert err < 1e-2, err
+
+
+@pytest.mark.parametrize("shape,c0,c1,cout,planes", [
+    ((2, 2, 2), 16, 0, 16, 8),        # less than one block, one plane of two
+    ((8, 16, 8), 16, 0, 32, 4),       # two z parts of one block
+    ((10, 18, 14), 16, 16, 32, 8),    # ragged blocks, upsampled second input
+    ((24, 34, 10), 32, 0, 64, 4),     # the widest merged operand (N = 192)
+    ((24, 34, 10), 48, 0, 48, 4),     # padded to it
+    ((10, 18, 6), 16, 0, 128, 4),     # a tap an MMA
+])
+def test_conv_merged_taps_at_edges(shape, c0, c1, cout, planes):
+    """Block remainders and every operand width of the tap merging, with and
+    without ReLU. FP32 sums of exact BF16 products, rounded once to BF16: half
+    a unit in the last place, 2^-9 of a value, and as much in the norm."""
+    nx, ny, nz = shape
+    for relu in (0, 1):
+        out, ref = run_conv(nx, ny, nz, c0, c1, cout, planes, relu=relu, seed=nx + cout)
+        assert np.linalg.norm(out - ref) <= 2.0 ** -9 * np.linalg.norm(ref) + 1e-6
