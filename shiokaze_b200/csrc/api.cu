@@ -15,6 +15,7 @@
 #include "csr_mic0.h"
 #include "../../include/shkz_b200.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -93,12 +94,12 @@ struct shkz_b200_ctx {
   int cap_warm_pool = 0;
   size_t cap_rank_cnt = 0;
   float *h_dens[3] = {};           // staging of the solid density faces (host path)
-  float *ext_v[3] = {};            // velocity extension: the constraint's new values per component
-  unsigned *ext_bits[3][2] = {};   // and the masks before and after a pass, as bits
-  size_t cap_ext[3] = {0, 0, 0};
+  unsigned *ext_bits = nullptr;    // velocity extension: the components' masks before and after a pass, as bits
+  size_t cap_ext = 0;
   unsigned *ext_solid = nullptr;   // solid nodes as bits
   size_t cap_ext_solid = 0;
-  unsigned *ext_list[3] = {};      // faces the constraint looks at
+  unsigned *ext_list = nullptr;    // faces the constraint looks at and their new values
+  size_t cap_ext_list = 0;
   unsigned *ext_flag = nullptr;    // [4]: their numbers, levelset_exist(solid)
   // FLIP splat (splat.cu)
   unsigned char *sp_raw = nullptr;  // particle records (host path)
@@ -414,10 +415,8 @@ extern "C" void shkz_b200_destroy(shkz_b200_ctx *ctx) {
                   ctx->mtile, ctx->mnbr, ctx->seg, ctx->mseg, ctx->nseg, ctx->msub, ctx->mfaces_f, ctx->mfaces_b, ctx->coef_f,
                   ctx->coef_b, ctx->tp, ctx->curv,
                   ctx->prev, ctx->rank_pool, ctx->rank_cnt, ctx->rank_total, ctx->xw, ctx->h_dens[0],
-                  ctx->h_dens[1], ctx->h_dens[2], ctx->flush, ctx->pb, ctx->ext_v[0], ctx->ext_v[1], ctx->ext_v[2],
-                  ctx->ext_bits[0][0], ctx->ext_bits[0][1], ctx->ext_bits[1][0],
-                  ctx->ext_bits[1][1], ctx->ext_bits[2][0], ctx->ext_bits[2][1], ctx->ext_solid, ctx->ext_flag,
-                  ctx->ext_list[0], ctx->ext_list[1], ctx->ext_list[2], ctx->sp_raw, ctx->sp_posm,
+                  ctx->h_dens[1], ctx->h_dens[2], ctx->flush, ctx->pb, ctx->ext_bits, ctx->ext_solid,
+                  ctx->ext_flag, ctx->ext_list, ctx->sp_raw, ctx->sp_posm,
                   ctx->sp_vc[0], ctx->sp_vc[1], ctx->sp_vc[2], ctx->sp_key, ctx->sp_rank, ctx->sp_list, ctx->sp_sposm,
                   ctx->sp_svc, ctx->sp_faces, ctx->sp_sorted, ctx->sp_face_bin, ctx->sp_nfaces, ctx->sp_work,
                   ctx->sp_count, ctx->sp_tile_start, ctx->sp_tile_act, ctx->sp_tiles, ctx->sp_act[0],
@@ -1043,25 +1042,27 @@ static int extend_device(shkz_b200_ctx *ctx, const shkz_b200_extend_args *a) {
   f.ny = a->ny;
   f.nz = a->nz;
   f.dx = a->dx;
+  size_t words = 0;
   for (int d = 0; d < 3; ++d) {
     f.W[d] = a->nx + (d == 0);
     f.H[d] = a->ny + (d == 1);
     f.D[d] = a->nz + (d == 2);
     const size_t nf = (size_t)f.W[d] * f.H[d] * f.D[d];
-    if (nf > ctx->cap_ext[d]) {
-      GROW(ext_v[d], nf);
-      GROW(ext_list[d], nf);
-      GROW(ext_bits[d][0], (nf + 31) / 32);
-      GROW(ext_bits[d][1], (nf + 31) / 32);
-      ctx->cap_ext[d] = nf;
-    }
     f.n[d] = (unsigned)nf;
     f.vel[d] = a->velocity[d];
     f.act[d] = a->velocity_active[d];
-    f.bits[d] = ctx->ext_bits[d][0];
-    f.next[d] = ctx->ext_bits[d][1];
-    f.list[d] = ctx->ext_list[d];
-    f.side[d] = ctx->ext_v[d];
+    words += 2 * ((nf + 31) / 32);
+  }
+  if (words > ctx->cap_ext) {
+    ctx->cap_ext = 0;
+    GROW(ext_bits, words);
+    ctx->cap_ext = words;
+  }
+  unsigned *at = ctx->ext_bits;
+  for (int d = 0; d < 3; ++d) {
+    f.bits[d] = at;
+    f.next[d] = at + (f.n[d] + 31) / 32;
+    at = f.next[d] + (f.n[d] + 31) / 32;
   }
   if (!ctx->ext_flag) GROW(ext_flag, 4);
   launch_ext_pack(f, s);
@@ -1082,9 +1083,33 @@ static int extend_device(shkz_b200_ctx *ctx, const shkz_b200_extend_args *a) {
     f.listed = ctx->ext_flag;
     int *solid_flag = reinterpret_cast<int *>(ctx->ext_flag + 3);
     f.solid_flag = solid_flag;
-    SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->ext_flag, 0, 4 * sizeof(unsigned), s));
-    // all three components are found on the unchanged field, then committed
-    launch_constrain(f, a->solid_active, solid_flag, s);
+    SHKZ_CUDA_TRY(cudaMemsetAsync(solid_flag, 0, sizeof(int), s));
+    launch_solid_bits(f, a->solid_active, solid_flag, s);
+    // the faces next to a solid, the floor and the ceiling are listed: under 1 %
+    // of a simulation's faces, so the lists start at 1/16 of them; a call that
+    // needs more grows them and lists again
+    unsigned listed[3] = {f.n[0] / 16 + 4096, f.n[1] / 16 + 4096, f.n[2] / 16 + 4096};
+    for (bool fits = false; !fits;) {
+      const size_t most = std::max(listed[0], std::max(listed[1], listed[2]));
+      if (most > ctx->cap_ext_list) {
+        ctx->cap_ext_list = 0;
+        GROW(ext_list, 6 * most);
+        ctx->cap_ext_list = most;
+      }
+      for (int d = 0; d < 3; ++d) {
+        f.list[d] = ctx->ext_list + (size_t)(2 * d) * ctx->cap_ext_list;
+        f.side[d] = reinterpret_cast<float *>(ctx->ext_list + (size_t)(2 * d + 1) * ctx->cap_ext_list);
+        f.room[d] = (unsigned)ctx->cap_ext_list;
+      }
+      SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->ext_flag, 0, 3 * sizeof(unsigned), s));
+      // all three components are found on the unchanged field, then committed
+      launch_constrain(f, s);
+      SHKZ_CUDA_TRY(cudaGetLastError());
+      SHKZ_CUDA_TRY(cudaMemcpyAsync(listed, ctx->ext_flag, sizeof(listed), cudaMemcpyDeviceToHost, s));
+      SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+      fits = listed[0] <= f.room[0] && listed[1] <= f.room[1] && listed[2] <= f.room[2];
+    }
+    return 0;
   }
   SHKZ_CUDA_TRY(cudaGetLastError());
   SHKZ_CUDA_TRY(cudaStreamSynchronize(s));

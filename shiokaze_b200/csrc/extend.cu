@@ -345,9 +345,16 @@ __global__ void __launch_bounds__(kListThreads) k_constrain_list(ExtendFields f)
     }
     if (threadIdx.x == 0 && total) base = atomicAdd(&f.listed[d], (unsigned)total);
     __syncthreads();
-    unsigned *at = f.list[d] + base + before + incl - __popc(m);
-    for (; m; m &= m - 1) *at++ = o + (__ffs(m) - 1);
+    unsigned at = base + before + incl - __popc(m);
+    for (; m; m &= m - 1, ++at)
+      if (at < f.room[d]) f.list[d][at] = o + (__ffs(m) - 1);
   }
+}
+
+// A list that did not fit: nothing is constrained, the host makes room and
+// calls again.
+__device__ __forceinline__ bool overfull(const ExtendFields &f) {
+  return f.listed[0] > f.room[0] || f.listed[1] > f.room[1] || f.listed[2] > f.room[2];
 }
 
 // The listed faces' constrained values. The field is not modified here: a new
@@ -357,7 +364,7 @@ __global__ void __launch_bounds__(kListThreads) k_constrain_list(ExtendFields f)
 constexpr unsigned kStruck = 0xffffffffu;
 __global__ void __launch_bounds__(128) k_constrain_find(ExtendFields f) {
   const int d = blockIdx.y, W = f.W[d], H = f.H[d];
-  const unsigned listed = f.listed[d];
+  const unsigned listed = overfull(f) ? 0u : f.listed[d];
   const bool has_solid = f.solid && *f.solid_flag;
   for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < listed; e += gridDim.x * blockDim.x) {
     const unsigned o = f.list[d][e];
@@ -372,7 +379,7 @@ __global__ void __launch_bounds__(128) k_constrain_find(ExtendFields f) {
 // The new values, into the field.
 __global__ void __launch_bounds__(256) k_constrain_apply(ExtendFields f) {
   const int d = blockIdx.y;
-  const unsigned listed = f.listed[d];
+  const unsigned listed = overfull(f) ? 0u : f.listed[d];
   for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < listed; e += gridDim.x * blockDim.x)
     if (f.list[d][e] != kStruck) f.vel[d][f.list[d][e]] = f.side[d][e];
 }
@@ -398,12 +405,15 @@ void launch_extrapolate(const ExtendFields &f, cudaStream_t s) {
   k_extrapolate<<<ext_grid(most_words(f), kExtrapolateThreads), kExtrapolateThreads, 0, s>>>(f);
 }
 
-void launch_constrain(const ExtendFields &f, const uint8_t *solid_active, int *solid_flag, cudaStream_t s) {
+void launch_solid_bits(const ExtendFields &f, const uint8_t *solid_active, int *solid_flag, cudaStream_t s) {
   if (f.solid) {
     const unsigned nodes = (unsigned)(f.nx + 1) * (f.ny + 1) * (f.nz + 1);
     count_launches(1);
     k_solid_bits<<<ext_grid((nodes + 31) / 32, 256).x, 256, 0, s>>>(f.solid, solid_active, nodes, f.solid_bits, solid_flag);
   }
+}
+
+void launch_constrain(const ExtendFields &f, cudaStream_t s) {
   count_launches(3);
   // rows are cut into words of their own: a few more than the flat masks have
   const unsigned words = (unsigned)((f.nx + 32) / 32) * (f.ny + 1) * (f.nz + 1);

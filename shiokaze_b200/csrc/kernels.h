@@ -64,18 +64,21 @@ struct ExtendFields {
   uint8_t *act[3];
   unsigned *bits[3];       // active masks as bits, (n + 31) / 32 words
   unsigned *next[3];       // the masks after a pass
-  unsigned *list[3];       // faces the constraint may change (room for all), and their new values
+  unsigned *list[3];       // faces the constraint may change, and their new values
   float *side[3];
-  unsigned *listed;        // [3] how many
+  unsigned room[3];        // entries the lists hold
+  unsigned *listed;        // [3] entries there are; over room, the constraint changes nothing
   const float *solid;      // nodes, or null
   unsigned *solid_bits;    // nodes that are not outside the solid
   const int *solid_flag;   // whether the solid level set exists
 };
-// byte masks into bits; one extrapolation pass (bits -> next); the constraint
-// (on bits; listed and *solid_flag zeroed by the caller)
+// byte masks into bits; one extrapolation pass (bits -> next); solid_bits and
+// solid_flag (zeroed by the caller); the constraint (on bits; listed zeroed by
+// the caller)
 void launch_ext_pack(const ExtendFields &f, cudaStream_t s);
 void launch_extrapolate(const ExtendFields &f, cudaStream_t s);
-void launch_constrain(const ExtendFields &f, const uint8_t *solid_active, int *solid_flag, cudaStream_t s);
+void launch_solid_bits(const ExtendFields &f, const uint8_t *solid_active, int *solid_flag, cudaStream_t s);
+void launch_constrain(const ExtendFields &f, cudaStream_t s);
 
 // FLIP splat (splat.cu). Particle records read in place: float fields at byte
 // offsets (multiples of 4) of `stride`-byte records.

@@ -131,3 +131,20 @@ def test_extension_on_odd_grids_bitexact(shape, with_solid):
         got_v, got_a = native.extend_velocity(ctx, vel, act, solid, sact, dx, width, True)
         want_v, want_a = ext.extend(vel, act, solid, sact, dx, width, True)
         _assert_same(got_v, got_a, want_v, want_a)
+
+
+def test_extension_with_more_constrained_faces_than_listed_room_bitexact():
+    """A solid over most of the grid: the constraint looks at more faces than
+    its lists first hold, grows them and lists again."""
+    from shiokaze_b200 import native
+    nx, ny, nz = 40, 48, 36
+    rng = np.random.default_rng(5)
+    vel = [rng.standard_normal((nz + (d == 2), ny + (d == 1), nx + (d == 0))).astype(np.float32) for d in range(3)]
+    act = [np.ones(v.shape, np.uint8) for v in vel]
+    solid = (0.02 * rng.standard_normal((nz + 1, ny + 1, nx + 1)) - 0.02).astype(np.float32)
+    sact = np.ones(solid.shape, np.uint8)
+    ctx = native.Context(native.default_config())
+    want_v, want_a = ext.extend(vel, act, solid, sact, 1.0 / 48, 1, True)
+    for _ in range(2):
+        got_v, got_a = native.extend_velocity(ctx, vel, act, solid, sact, 1.0 / 48, 1, True)
+        _assert_same(got_v, got_a, want_v, want_a)
