@@ -75,7 +75,7 @@ typedef struct shkz_b200_config {
   int refine;                 /* FP64 outer refinement of the FP32 solve (default 1) */
   int fp64_reference;         /* also run an FP64 tight solve and report the error (default 0) */
   double fp64_tol;            /* tolerance of that solve (default 1e-12) */
-  int check_interval;         /* iterations per device-side batch between host checks (default 16) */
+  int check_interval;         /* at most so many iterations queued beyond the last the device reported (default 16; the solve queues 3) */
   int stall_window;           /* learned FPCG: iterations without progress before MIC(0) fallback */
   int device;                 /* CUDA device ordinal (default 0) */
   int mic_block;              /* MIC(0) sweep block edge: 16 (default, 2x2x2 tiles per CTA) or 8 */

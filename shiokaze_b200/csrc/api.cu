@@ -5,9 +5,10 @@
 //   label unknowns -> build the 8^3 tile pool -> weights/rhs -> MIC(0) factor
 //   -> FP32 PCG with FP64 reductions inside an FP64 refinement loop
 //   -> pressure scatter and velocity update.
-// The PCG runs in batches of `check_interval` iterations; each kernel reads
-// the device-side solver state and returns at once after convergence, so the
-// host only synchronises once per batch.
+// The PCG's iterations are queued a few ahead of the device, which reports
+// each one it completes to a word of pinned host memory; each kernel reads the
+// device-side solver state and returns at once after convergence, so neither
+// side waits for the other inside the loop.
 #include "common.cuh"
 #include "kernels.h"
 #include "solver.h"
@@ -51,7 +52,8 @@ struct shkz_b200_ctx {
   int *flags = nullptr;
   uint8_t *unk = nullptr;
   int *tile_count = nullptr, *tile_state = nullptr, *pool_tile = nullptr, *nbr = nullptr, *level_count = nullptr,
-      *sched = nullptr, *bsum = nullptr, *total = nullptr;
+      *sched = nullptr, *bsum = nullptr;
+  long long *usum = nullptr;
   // pool arrays
   float *diag = nullptr, *offx = nullptr, *offy = nullptr, *offz = nullptr, *d32 = nullptr;
   double *diag64 = nullptr, *offx64 = nullptr, *offy64 = nullptr, *offz64 = nullptr, *rhs64 = nullptr,
@@ -61,6 +63,8 @@ struct shkz_b200_ctx {
   float *pb = nullptr;  // second direction buffer: the fused stencil writes the new p beside the old one
   // reductions and wavefront sync
   double *partials = nullptr, *out4 = nullptr;
+  Mailbox *mail = nullptr;         // pinned host memory the device reports to
+  unsigned mail_seq = 0;           // number of the last report asked for
   unsigned *counter = nullptr;
   SolverState *st = nullptr;
   int *wflags = nullptr;  // factor wavefront flags [cap_pool]
@@ -245,7 +249,9 @@ static int ensure_grid(shkz_b200_ctx *ctx, const Geometry &G) {
   if (G.ntiles > ctx->cap_tiles) {
     GROW(tile_count, G.ntiles);
     GROW(tile_state, G.ntiles);
-    GROW(bsum, (G.ntiles + 1023) / 1024 + 1);
+    // block sums of the tiles and, after them, of the macro tiles
+    GROW(bsum, 2 * ((G.ntiles + 1023) / 1024 + 1));
+    GROW(usum, (G.ntiles + 1023) / 1024 + 1);
     GROW(mcount, G.ntiles);
     GROW(mstate, G.ntiles);
     ctx->cap_tiles = G.ntiles;
@@ -333,24 +339,64 @@ static int ensure_macro(shkz_b200_ctx *ctx, int KM) {
 // 16^3 macro tiles over the pool (2x2x2 tiles each) for the MIC(0) sweeps:
 // the pool kernels run again on a grid twice as coarse, with the summed
 // unknown counts of each macro tile's eight tiles.
-static int build_macro_tiles(shkz_b200_ctx *ctx, const Geometry &G, int K, cudaStream_t s) {
-  ctx->KM = 0;
-  if (K <= 0 || ctx->cfg.mic_block == 8) return 0;
+static Geometry macro_geometry(const Geometry &G) {
   Geometry M = G;
   M.bx = (G.bx + 1) / 2;
   M.by = (G.by + 1) / 2;
   M.bz = (G.bz + 1) / 2;
   M.ntiles = (long long)M.bx * M.by * M.bz;
-  launch_macro_count(G, ctx->tile_count, M, ctx->mcount, s);
-  const int KM = pool_count(M, ctx->mcount, ctx->bsum, ctx->total, s);
-  if (KM < 0) {
-    shkz_set_cuda_error(cudaGetLastError(), "pool_count (macro)", __FILE__, __LINE__);
-    return SHKZ_B200_ERR_CUDA;
+  return M;
+}
+static int *macro_bsum(shkz_b200_ctx *ctx, const Geometry &G) { return ctx->bsum + (G.ntiles + 1023) / 1024 + 1; }
+
+// Polls `arrived` until it holds. When the stream has run dry (or failed)
+// without it, whatever was going to be reported has been: false.
+template <class F>
+static bool poll_mail(cudaStream_t s, F arrived) {
+  for (unsigned spins = 1;; ++spins) {
+    if (arrived()) return true;
+    if ((spins & 0x3fff) == 0 && cudaStreamQuery(s) != cudaErrorNotReady) return arrived();
   }
-  int rc = ensure_macro(ctx, KM > 0 ? KM : 1);
+}
+static int wait_mail(shkz_b200_ctx *ctx, unsigned seq) {
+  if (poll_mail(ctx->stream, [&] { return __atomic_load_n(&ctx->mail->seq, __ATOMIC_ACQUIRE) == seq; })) return 0;
+  shkz_set_cuda_error(cudaGetLastError(), "report of a kernel", __FILE__, __LINE__);
+  return SHKZ_B200_ERR_CUDA;
+}
+// the number of the next report; 0 stands for none
+static unsigned next_mail(shkz_b200_ctx *ctx) {
+  if (++ctx->mail_seq == 0) ++ctx->mail_seq;
+  return ctx->mail_seq;
+}
+
+// Tiles and macro tiles that hold unknowns, and the unknowns: counted by four
+// small kernels and read by the host in one go.
+static int count_pool(shkz_b200_ctx *ctx, const Geometry &G, int *K, int *KM, long long *unknowns) {
+  cudaStream_t s = ctx->stream;
+  const bool macro = ctx->cfg.mic_block != 8;
+  const unsigned seq = next_mail(ctx);
+  launch_pool_count(G, ctx->tile_count, ctx->bsum, ctx->usum, false, ctx->mail, macro ? 0 : seq, s);
+  if (macro) {
+    const Geometry M = macro_geometry(G);
+    launch_macro_count(G, ctx->tile_count, M, ctx->mcount, s);
+    launch_pool_count(M, ctx->mcount, macro_bsum(ctx, G), ctx->usum, true, ctx->mail, seq, s);
+  }
+  SHKZ_CUDA_TRY(cudaGetLastError());
+  const int rc = wait_mail(ctx, seq);
   if (rc) return rc;
-  build_macro(G, M, ctx->tile_count, ctx->tile_state, ctx->mcount, ctx->mstate, ctx->mtile, ctx->mnbr,
-              ctx->level_count, ctx->seg, ctx->mseg, ctx->nseg, ctx->msub, KM, ctx->bsum, s);
+  *K = ctx->mail->tiles;
+  *KM = macro ? ctx->mail->macro_tiles : 0;
+  *unknowns = ctx->mail->unknowns;
+  return 0;
+}
+
+static int build_macro_tiles(shkz_b200_ctx *ctx, const Geometry &G, int KM, cudaStream_t s) {
+  ctx->KM = 0;
+  if (KM <= 0) return 0;
+  const int rc = ensure_macro(ctx, KM);
+  if (rc) return rc;
+  build_macro(G, macro_geometry(G), ctx->tile_count, ctx->tile_state, ctx->mcount, ctx->mstate, ctx->mtile, ctx->mnbr,
+              ctx->level_count, ctx->seg, ctx->mseg, ctx->nseg, ctx->msub, KM, macro_bsum(ctx, G), s);
   SHKZ_CUDA_TRY(cudaGetLastError());
   ctx->KM = KM;
   return 0;
@@ -380,7 +426,8 @@ extern "C" int shkz_b200_create(shkz_b200_ctx **out, const shkz_b200_config *cfg
     return SHKZ_B200_ERR_CUDA;
   }
   for (auto &e : ctx->ev) cudaEventCreate(&e);
-  if (cudaMalloc(&ctx->flags, sizeof(int)) != cudaSuccess || cudaMalloc(&ctx->total, sizeof(int)) != cudaSuccess ||
+  if (cudaMalloc(&ctx->flags, sizeof(int)) != cudaSuccess ||
+      cudaHostAlloc((void **)&ctx->mail, sizeof(Mailbox), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess ||
       cudaMalloc(&ctx->counter, sizeof(unsigned) * 8) != cudaSuccess ||
       cudaMalloc(&ctx->st, sizeof(SolverState)) != cudaSuccess || cudaMalloc(&ctx->out4, sizeof(double) * 8) != cudaSuccess ||
       cudaMalloc(&ctx->ws, 3 * wave_sync_bytes()) != cudaSuccess ||
@@ -390,7 +437,15 @@ extern "C" int shkz_b200_create(shkz_b200_ctx **out, const shkz_b200_config *cfg
   }
   cudaMemsetAsync(ctx->counter, 0, sizeof(unsigned) * 8, ctx->stream);
   cudaMemsetAsync(ctx->ws, 0, 3 * wave_sync_bytes(), ctx->stream);
-  cudaMemsetAsync(ctx->st, 0, sizeof(SolverState), ctx->stream);
+  std::memset((void *)ctx->mail, 0, sizeof(Mailbox));
+  SolverState st0{};
+  st0.waves = ctx->ws;
+  if (cudaHostGetDevicePointer((void **)&st0.mail, ctx->mail, 0) != cudaSuccess || st0.mail != ctx->mail) {
+    shkz_b200_destroy(ctx);  // the kernels are given the host's address
+    return SHKZ_B200_ERR_CUDA;
+  }
+  cudaMemsetAsync(ctx->st_scratch, 0, sizeof(SolverState), ctx->stream);  // reports nowhere
+  cudaMemcpyAsync(ctx->st, &st0, sizeof(SolverState), cudaMemcpyHostToDevice, ctx->stream);
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
     shkz_b200_destroy(ctx);
     return SHKZ_B200_ERR_CUDA;
@@ -406,7 +461,7 @@ extern "C" void shkz_b200_destroy(shkz_b200_ctx *ctx) {
   void *ptrs[] = {ctx->h_fluid, ctx->h_solid, ctx->h_vel[0], ctx->h_vel[1], ctx->h_vel[2], ctx->h_svel[0],
                   ctx->h_svel[1], ctx->h_svel[2], ctx->h_pressure, ctx->h_fluid_active, ctx->h_solid_active,
                   ctx->h_vact[0], ctx->h_vact[1], ctx->h_vact[2], ctx->h_pact, ctx->flags, ctx->unk, ctx->tile_count,
-                  ctx->tile_state, ctx->pool_tile, ctx->nbr, ctx->level_count, ctx->sched, ctx->bsum, ctx->total,
+                  ctx->tile_state, ctx->pool_tile, ctx->nbr, ctx->level_count, ctx->sched, ctx->bsum, ctx->usum,
                   ctx->diag, ctx->offx, ctx->offy, ctx->offz, ctx->d32, ctx->diag64, ctx->offx64, ctx->offy64,
                   ctx->offz64, ctx->rhs64, ctx->colsum, ctx->dmic64, ctx->x64,
                   ctx->r64, ctx->xref64, ctx->p64, ctx->q64, ctx->z64, ctx->x, ctx->r, ctx->p, ctx->q, ctx->z,
@@ -425,6 +480,7 @@ extern "C" void shkz_b200_destroy(shkz_b200_ctx *ctx) {
                   ctx->sp_sact[0], ctx->sp_sact[1], ctx->sp_sact[2]};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  if (ctx->mail) cudaFreeHost(ctx->mail);
   if (ctx->model) learned_free(ctx->model);
   for (auto &e : ctx->ev)
     if (e) cudaEventDestroy(e);
@@ -471,22 +527,16 @@ static char *wsync(shkz_b200_ctx *ctx, int which) { return (char *)ctx->ws + whi
 
 // Before a call's wavefront kernels: clear the three wave-sync error words
 // (a timed-out call leaves one set) and write the configured spin limit and
-// the fault-injection slot (forward sweep only). The words are
-// error, spin_limit, skip_publish at byte offset 12 of each WaveSync; the
-// slot, epoch and finished words are left alone, so face tags stay valid.
+// the fault-injection slot (forward sweep only). The slot, epoch and finished
+// words are left alone, so face tags stay valid.
 static int arm_waves(shkz_b200_ctx *ctx) {
-  for (int w = 0; w < 3; ++w) {
-    const int words[3] = {0, ctx->cfg.spin_limit > 0 ? ctx->cfg.spin_limit : 0,
-                          w == 1 && ctx->cfg.fault_skip_publish > 0 ? ctx->cfg.fault_skip_publish : 0};
-    SHKZ_CUDA_TRY(cudaMemcpyAsync(wsync(ctx, w) + 3 * sizeof(int), words, sizeof(words), cudaMemcpyHostToDevice,
-                                  ctx->stream));
-  }
   // face words of the pencil sweeps: unset (a call that gave up may have left
   // some written, and another grid's neighbours differ)
-  if (ctx->KM > 0) {
-    SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->mfaces_f, 0xff, sizeof(float) * (size_t)ctx->KM * kFaceRows * 32, ctx->stream));
-    SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->mfaces_b, 0xff, sizeof(float) * (size_t)ctx->KM * kFaceRows * 32, ctx->stream));
-  }
+  const size_t faces = ctx->KM > 0 ? (size_t)ctx->KM * kFaceRows * 32 : 0;
+  launch_arm_waves(ctx->ws, ctx->cfg.spin_limit > 0 ? ctx->cfg.spin_limit : 0,
+                   ctx->cfg.fault_skip_publish > 0 ? ctx->cfg.fault_skip_publish : 0, ctx->mfaces_f, ctx->mfaces_b,
+                   faces, ctx->stream);
+  SHKZ_CUDA_TRY(cudaGetLastError());
   return 0;
 }
 
@@ -517,6 +567,62 @@ static int wave_errors(shkz_b200_ctx *ctx) {
 
 static const double kReliableDrop = 0.1;
 
+// r64 = b - A x64 over the pool; norms = ||r||inf, ||r||^2, ||b||inf, ||b||^2
+static int residual_norms(shkz_b200_ctx *ctx, const PoolSystem &S, const double *x64, double norms[4]) {
+  MailSlot slot;
+  slot.mail = ctx->mail;
+  slot.seq = next_mail(ctx);
+  slot.waves = ctx->ws;
+  launch_residual64(S, ctx->rhs64, x64, ctx->r64, ctx->partials, ctx->counter + 2, slot, ctx->stream);
+  SHKZ_CUDA_TRY(cudaGetLastError());
+  const int rc = wait_mail(ctx, slot.seq);
+  if (rc) return rc;
+  for (int i = 0; i < 4; ++i) norms[i] = ctx->mail->norms[i];
+  return 0;
+}
+
+struct Progress {
+  int iter = 0, done = 0;
+  bool nan = false, wave_error = false;
+  double rmax = 0.0;
+};
+// The solve loop's state once at least `iter` iterations are complete or the
+// solve has stopped. A stop that no kernel reported (or a failure) leaves the
+// stream idle; the state is then read by a copy.
+static int wait_progress(shkz_b200_ctx *ctx, int iter, Progress *p) {
+  unsigned long long v = 0;
+  auto arrived = [&] {
+    v = __atomic_load_n(&ctx->mail->progress, __ATOMIC_ACQUIRE);
+    return (int)(unsigned)v >= iter || (v >> kProgressDone) != 0;
+  };
+  if (poll_mail(ctx->stream, arrived)) {
+    p->iter = (int)(unsigned)v;
+    p->done = (int)(v >> kProgressDone) & 0xff;
+    p->nan = (v & kProgressNan) != 0;
+    p->wave_error = (v & kProgressWaveError) != 0;
+    p->rmax = ctx->mail->rmax;
+    return 0;
+  }
+  SolverState st;
+  SHKZ_CUDA_TRY(cudaMemcpyAsync(&st, ctx->st, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
+  SHKZ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  p->iter = st.iter;
+  p->done = st.done;
+  p->nan = st.status < 0;
+  p->rmax = st.rmax;
+  p->wave_error = wave_errors(ctx) != 0;
+  return 0;
+}
+// before the loop is resumed after `iter` iterations (nothing queued reports any more)
+static void reset_progress(shkz_b200_ctx *ctx, int iter) {
+  __atomic_store_n(&ctx->mail->progress, (unsigned long long)(unsigned)iter, __ATOMIC_RELEASE);
+}
+
+// Iterations queued beyond the last one reported. A retired launch costs 4 us
+// (12 an iteration) whenever the loop stops, which it does once per reliable
+// update; too few queued and the device waits for the host.
+static const int kQueueAhead = 3;
+
 // z = M^-1 r, rho_new, beta, p = z + beta p (or the identity-preconditioned variant)
 static void launch_iteration_tail(shkz_b200_ctx *ctx, const PoolSystem &S, int n, int precond, cudaStream_t s) {
   if (precond == SHKZ_B200_PRECOND_MIC0) {
@@ -536,9 +642,8 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
   const int n = ctx->K * SHKZ_TC;
   SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->x64, 0, sizeof(double) * n, s));
   double h4[4];
-  launch_residual64(S, ctx->rhs64, ctx->x64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
-  SHKZ_CUDA_TRY(cudaMemcpyAsync(h4, ctx->out4, sizeof(h4), cudaMemcpyDeviceToHost, s));
-  SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+  int rc = residual_norms(ctx, S, ctx->x64, h4);
+  if (rc) return rc;
   const double bmax = h4[2], b2 = h4[3];
   double rmax = h4[0], r2 = h4[1];
   res->outer_steps = 0;
@@ -557,6 +662,7 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
   launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, s);
   launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st, tol, s);
   launch_state_resume(ctx->st, reliable ? kReliableDrop : 0.0, s);
+  reset_progress(ctx, 0);
   // z0 = M^-1 r0, rho0, p0 = z0
   if (precond == SHKZ_B200_PRECOND_MIC0) {
     launch_mic_apply(S, ctx->d32, ctx->r, ctx->t, ctx->z, ctx->partials, ctx->faces_f,
@@ -568,9 +674,9 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
     SHKZ_CUDA_TRY(cudaMemcpyAsync(ctx->p, ctx->r, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
   }
   const int max_it = ctx->cfg.max_iterations;
-  const int batch = ctx->cfg.check_interval > 0 ? ctx->cfg.check_interval : 16;
-  SolverState hst;
-  int rc = 0, updates = 0;
+  const int ahead = ctx->cfg.check_interval > 0 ? std::min(ctx->cfg.check_interval, kQueueAhead) : kQueueAhead;
+  Progress hst;
+  int queued = 0, updates = 0;
   bool true_checked = false;
   // MIC(0) on pencils: the x update and the direction update p = z + beta p
   // ride in the next iteration's stencil (ping-pong between two p buffers) and
@@ -586,36 +692,35 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
     else launch_accumulate(n, ctx->x, scale, ctx->x64, s);
   };
   for (;;) {
-    for (int b = 0; b < batch; ++b) {
-      if (fused) {
-        launch_spmv_update(S, ctx->p, ctx->pb, ctx->z, ctx->q, ctx->x, ctx->partials, ctx->counter, ctx->st, s);
-        launch_mic_apply_update(S, ctx->r, ctx->z, ctx->partials, ctx->q, ctx->counter + 1, ctx->st, max_it,
-                                wsync(ctx, 1), wsync(ctx, 2), ctx->counter + 5, s);
-        continue;
-      }
+    if (fused) {
+      launch_spmv_update(S, ctx->p, ctx->pb, ctx->z, ctx->q, ctx->x, ctx->partials, ctx->counter, ctx->st, s);
+      launch_mic_apply_update(S, ctx->r, ctx->z, ctx->partials, ctx->q, ctx->counter + 1, ctx->st, max_it,
+                              wsync(ctx, 1), wsync(ctx, 2), ctx->counter + 5, s);
+    } else {
       launch_spmv(S, ctx->p, ctx->q, ctx->partials, ctx->counter, ctx->st, 0, s);
       launch_update_xr(n, ctx->p, ctx->q, ctx->x, ctx->r, ctx->partials, ctx->counter + 1, ctx->st, max_it, s);
       launch_iteration_tail(ctx, S, n, precond, s);
     }
-    SHKZ_CUDA_TRY(cudaMemcpyAsync(&hst, ctx->st, sizeof(hst), cudaMemcpyDeviceToHost, s));
-    SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+    SHKZ_CUDA_TRY(cudaGetLastError());
+    ++queued;
+    if ((rc = wait_progress(ctx, queued - ahead + 1, &hst))) return rc;
     // a bounded wait that gave up leaves its iterate undefined: stop here
-    if (wave_errors(ctx)) { rc = SHKZ_B200_ERR_TIMEOUT; break; }
-    if (hst.done == 0) continue;
-    if (hst.done == 3 || hst.status == -5) { rc = SHKZ_B200_ERR_NAN; break; }
+    if (hst.wave_error) { rc = SHKZ_B200_ERR_TIMEOUT; break; }
+    if (hst.done == 0 && !hst.nan) continue;
+    if (hst.done == 3 || hst.nan) { rc = SHKZ_B200_ERR_NAN; break; }
     if (hst.done == 2) break;
     if (hst.done == 1 && !reliable) break;
     // reliable update: fold the FP32 increment into x64 and replace r by b - A x64
     accumulate();
-    launch_residual64(S, ctx->rhs64, ctx->x64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
-    SHKZ_CUDA_TRY(cudaMemcpyAsync(h4, ctx->out4, sizeof(h4), cudaMemcpyDeviceToHost, s));
-    SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int e = residual_norms(ctx, S, ctx->x64, h4)) return e;
     rmax = h4[0];
     r2 = h4[1];
     ++updates;
     true_checked = true;
     if (!(rmax == rmax)) { rc = SHKZ_B200_ERR_NAN; break; }
     if (rmax <= tol * bmax) break;
+    reset_progress(ctx, hst.iter);
+    queued = hst.iter;
     launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, s);
     launch_state_resume(ctx->st, kReliableDrop * rmax / scale, s);
     true_checked = false;
@@ -632,13 +737,11 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
   if (!true_checked) {
     // plain FP32 finish (refine off) or max iterations: report the true residual
     accumulate();
-    launch_residual64(S, ctx->rhs64, ctx->x64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
-    SHKZ_CUDA_TRY(cudaMemcpyAsync(h4, ctx->out4, sizeof(h4), cudaMemcpyDeviceToHost, s));
-    SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int e = residual_norms(ctx, S, ctx->x64, h4)) return e;
     rmax = h4[0];
     r2 = h4[1];
   }
-  if (wave_errors(ctx)) rc = SHKZ_B200_ERR_TIMEOUT;
+  if (hst.wave_error || ctx->mail->wave_error) rc = SHKZ_B200_ERR_TIMEOUT;
   res->iterations = hst.iter;
   res->outer_steps = updates;
   res->reresid = rmax / bmax;
@@ -703,9 +806,7 @@ static int fp64_reference_solve(shkz_b200_ctx *ctx, shkz_b200_result *res, const
     rho = rho_new;
   }
   // true residual of the reference solution and the error of x64
-  launch_residual64(S, ctx->rhs64, ctx->xref64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
-  SHKZ_CUDA_TRY(cudaMemcpyAsync(h, ctx->out4, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
-  SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+  if (const int e = residual_norms(ctx, S, ctx->xref64, h)) return e;
   res->fp64_reresid = h[0] / h[2];
   if (x0) launch_axpy2_64(n, 1.0, x0, ctx->xref64, x0, ctx->p64, s);  // xref64 += x0 (p64 scratch)
   // error: ||x64 - xref64||inf over ||xref64||inf  (q64 = x64 - xref64)
@@ -816,17 +917,16 @@ static int project_device(shkz_b200_ctx *ctx, const shkz_b200_project_args *a, s
     launch_surface_tension(in, ctx->flags, ctx->curv, a->surface_tension, vel, vact, s);
   }
   // pool size (one small host read), then the pool itself
-  const int K = pool_count(G, ctx->tile_count, ctx->bsum, ctx->total, s);
-  if (K < 0) {
-    shkz_set_cuda_error(cudaGetLastError(), "pool_count", __FILE__, __LINE__);
-    return SHKZ_B200_ERR_CUDA;
-  }
+  int K = 0, KM = 0;
+  long long unknowns = 0;
+  rc = count_pool(ctx, G, &K, &KM, &unknowns);
+  if (rc) return rc;
   rc = ensure_pool(ctx, K > 0 ? K : 1);
   if (rc) return rc;
   pool_assign(G, ctx->tile_count, K, ctx->bsum, ctx->tile_state, ctx->pool_tile, ctx->nbr, ctx->level_count,
               ctx->sched, s);
   SHKZ_CUDA_TRY(cudaGetLastError());
-  rc = build_macro_tiles(ctx, G, K, s);
+  rc = build_macro_tiles(ctx, G, KM, s);
   if (rc) return rc;
   rc = arm_waves(ctx);
   if (rc) return rc;
@@ -860,7 +960,7 @@ static int project_device(shkz_b200_ctx *ctx, const shkz_b200_project_args *a, s
     const PoolSystem S0 = pool_system(ctx);
     launch_unknown_rank(G, K, ctx->unk, T, ctx->tile_state, ctx->rank_pool, ctx->rank_cnt, ctx->rank_total, s);
     launch_warm_gather((long long)K * SHKZ_TC, ctx->rank_pool, ctx->prev, ctx->prev_n, ctx->xw, s);
-    launch_residual64(S0, ctx->rhs64, ctx->xw, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
+    launch_residual64(S0, ctx->rhs64, ctx->xw, ctx->r64, ctx->partials, ctx->counter + 2, MailSlot{}, s);
     SHKZ_CUDA_TRY(cudaMemcpyAsync(ctx->rhs64, ctx->r64, sizeof(double) * (size_t)K * SHKZ_TC,
                                   cudaMemcpyDeviceToDevice, s));
   }
@@ -875,16 +975,8 @@ static int project_device(shkz_b200_ctx *ctx, const shkz_b200_project_args *a, s
   SHKZ_CUDA_TRY(cudaGetLastError());
   cudaEventRecord(ctx->ev[1], s);
   ctx->has_system = 1;
-  // unknown count (for the result)
-  {
-    std::vector<int> tc((size_t)G.ntiles);
-    SHKZ_CUDA_TRY(cudaMemcpyAsync(tc.data(), ctx->tile_count, sizeof(int) * G.ntiles, cudaMemcpyDeviceToHost, s));
-    SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
-    long long u = 0;
-    for (int v : tc) u += v;
-    ctx->unknowns = u;
-    res->unknowns = u;
-  }
+  ctx->unknowns = unknowns;
+  res->unknowns = unknowns;
   int solve_rc = 0;
   if (K > 0) {
     if (precond == SHKZ_B200_PRECOND_LEARNED && ctx->model)
@@ -1781,9 +1873,7 @@ static int learned_solve(shkz_b200_ctx *ctx, double tol, shkz_b200_result *res) 
   const int n = ctx->K * SHKZ_TC;
   SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->x64, 0, sizeof(double) * n, s));
   double h4[4];
-  launch_residual64(S, ctx->rhs64, ctx->x64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
-  SHKZ_CUDA_TRY(cudaMemcpyAsync(h4, ctx->out4, sizeof(h4), cudaMemcpyDeviceToHost, s));
-  SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+  if ((rc = residual_norms(ctx, S, ctx->x64, h4))) return rc;
   const double bmax = h4[2], b2 = h4[3];
   double rmax_true = h4[0], r2 = h4[1];
   res->outer_steps = 0;
@@ -1798,6 +1888,7 @@ static int learned_solve(shkz_b200_ctx *ctx, double tol, shkz_b200_result *res) 
   launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, s);
   launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st, tol, s);
   launch_state_resume(ctx->st, kReliableDrop, s);
+  reset_progress(ctx, 0);
   bool use_mic = false;
   auto precondition = [&](double rmax_scaled) -> int {
     if (use_mic) {
@@ -1813,43 +1904,45 @@ static int learned_solve(shkz_b200_ctx *ctx, double tol, shkz_b200_result *res) 
   const int max_it = ctx->cfg.max_iterations;
   const int W = ctx->cfg.stall_window > 0 ? ctx->cfg.stall_window : 8;
   std::vector<double> hist;
-  SolverState hst;
+  Progress hst;
   int updates = 0;
+  double ru_threshold = kReliableDrop;
   bool true_checked = false;
   for (;;) {
     launch_spmv(S, ctx->p, ctx->q, ctx->partials, ctx->counter, ctx->st, 0, s);
     launch_update_xr(n, ctx->p, ctx->q, ctx->x, ctx->r, ctx->partials, ctx->counter + 1, ctx->st, max_it, s);
-    SHKZ_CUDA_TRY(cudaMemcpyAsync(&hst, ctx->st, sizeof(hst), cudaMemcpyDeviceToHost, s));
-    SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
-    if (use_mic && wave_errors(ctx)) { rc = SHKZ_B200_ERR_TIMEOUT; break; }
+    SHKZ_CUDA_TRY(cudaGetLastError());
+    if ((rc = wait_progress(ctx, hst.iter + 1, &hst))) return rc;
+    if (use_mic && hst.wave_error) { rc = SHKZ_B200_ERR_TIMEOUT; break; }
     if (hst.done == 5) {
       // the learned z broke down (z.r <= 0 or not finite): x and r are those of
       // the last completed iteration; continue with MIC(0) from r
       use_mic = true;
       res->fallbacks += 1;
-      launch_state_resume(ctx->st, hst.ru_threshold, s);
+      reset_progress(ctx, hst.iter);
+      launch_state_resume(ctx->st, ru_threshold, s);
       if ((rc = precondition(hst.rmax))) break;
       launch_fpcg_dots(n, ctx->z, ctx->r, ctx->q, ctx->partials, ctx->counter + 5, ctx->st, 1, s);
       SHKZ_CUDA_TRY(cudaMemcpyAsync(ctx->p, ctx->z, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
       continue;
     }
-    if (hst.done == 3 || hst.status == -5) { rc = SHKZ_B200_ERR_NAN; break; }
+    if (hst.done == 3 || hst.nan) { rc = SHKZ_B200_ERR_NAN; break; }
     if (hst.done == 2) break;
     true_checked = false;
     double rmax = hst.rmax;
     if (hst.done == 1 || hst.done == 4) {
       launch_accumulate(n, ctx->x, scale, ctx->x64, s);
-      launch_residual64(S, ctx->rhs64, ctx->x64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
-      SHKZ_CUDA_TRY(cudaMemcpyAsync(h4, ctx->out4, sizeof(h4), cudaMemcpyDeviceToHost, s));
-      SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+      if ((rc = residual_norms(ctx, S, ctx->x64, h4))) return rc;
       rmax_true = h4[0];
       r2 = h4[1];
       ++updates;
       true_checked = true;
       if (!(rmax_true == rmax_true)) { rc = SHKZ_B200_ERR_NAN; break; }
       if (rmax_true <= tol * bmax) break;
+      reset_progress(ctx, hst.iter);
       launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, s);
-      launch_state_resume(ctx->st, kReliableDrop * rmax_true / scale, s);
+      ru_threshold = kReliableDrop * rmax_true / scale;
+      launch_state_resume(ctx->st, ru_threshold, s);
       rmax = rmax_true / scale;
     }
     hist.push_back(rmax);
@@ -1868,9 +1961,7 @@ static int learned_solve(shkz_b200_ctx *ctx, double tol, shkz_b200_result *res) 
   }
   if (!true_checked && rc == 0) {
     launch_accumulate(n, ctx->x, scale, ctx->x64, s);
-    launch_residual64(S, ctx->rhs64, ctx->x64, ctx->r64, ctx->partials, ctx->counter + 2, ctx->out4, s);
-    SHKZ_CUDA_TRY(cudaMemcpyAsync(h4, ctx->out4, sizeof(h4), cudaMemcpyDeviceToHost, s));
-    SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
+    if ((rc = residual_norms(ctx, S, ctx->x64, h4))) return rc;
     rmax_true = h4[0];
     r2 = h4[1];
   }

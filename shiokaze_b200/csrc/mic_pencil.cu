@@ -762,6 +762,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_pencil_forward(PoolSystem S, co
       else if (mm <= sw->tol_abs) sw->done = 1;
       else if (sw->iter >= fu.max_iterations) sw->done = 2;
       else if (mm < sw->ru_threshold) sw->done = 4;
+      if (sw->done) report_progress(sw);  // otherwise the backward sweep does
       *fu.counter = 0;
     }
   }
@@ -875,6 +876,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_pencil_backward(PoolSystem S, c
     if (threadIdx.x == 0) {
       st->beta = rho_new / st->rho;
       st->rho = rho_new;
+      report_progress(st);
       *finish = 0;
     }
   }
@@ -928,15 +930,8 @@ __global__ void k_pencil_count(Geometry M, const int *mtile, const int *mnbr, in
   atomicAdd(&level_count[(int)((t / M.bx) % M.by) + (int)(t / ((long long)M.bx * M.by))], 1);
 }
 __global__ void k_pencil_scan(int *level_count, int nlev, int *nseg) {
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int i = 0; i < nlev; ++i) {
-      const int v = level_count[i];
-      level_count[i] = acc;
-      acc += v;
-    }
-    *nseg = acc;
-  }
+  const int n = warp_scan_counts(level_count, nlev);
+  if (threadIdx.x == 0) *nseg = n;
 }
 __global__ void k_pencil_scatter(Geometry M, const int *mtile, const int *mnbr, int KM, int *cursor, int2 *seg,
                                  int2 *mseg) {

@@ -63,28 +63,52 @@ __device__ double max_partials(const double *part, int n, double *red) {
 // ---------------------------------------------------------------------------
 // Tile pool construction
 
-__global__ void k_pool_blocksum(const int *tile_count, long long nt, int *bsum) {
+__global__ void k_pool_blocksum(const int *tile_count, long long nt, int *bsum, long long *usum) {
   __shared__ double red[8];
   const long long base = (long long)blockIdx.x * 1024;
-  int c = 0;
+  int c = 0, u = 0;  // a tile holds at most 4096 unknowns (a macro tile): 2^22 in a block
   for (int i = threadIdx.x; i < 1024; i += 256) {
     const long long t = base + i;
-    if (t < nt && tile_count[t] > 0) ++c;
+    const int v = t < nt ? tile_count[t] : 0;
+    if (v > 0) ++c;
+    u += v;
   }
-  const double s = block_sum<256>((double)c, red);
-  if (threadIdx.x == 0) bsum[blockIdx.x] = (int)s;
+  const double s = block_sum<256>((double)c, red), su = block_sum<256>((double)u, red);
+  if (threadIdx.x == 0) {
+    bsum[blockIdx.x] = (int)s;
+    usum[blockIdx.x] = (long long)su;
+  }
 }
 
-__global__ void k_pool_scan_blocks(int *bsum, int nb, int *total) {
-  // one block: exclusive scan of up to a few thousand block sums
+// one warp: offsets of the blocks and the totals, reported to the host
+__global__ void k_pool_scan(int *bsum, const long long *usum, int nb, int macro, Mailbox *mail, unsigned seq) {
+  const int total = warp_scan_counts(bsum, nb);
+  long long u = 0;
+  for (int i = threadIdx.x; i < nb; i += 32) u += usum[i];
+  #pragma unroll
+  for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
   if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int i = 0; i < nb; ++i) {
-      const int v = bsum[i];
-      bsum[i] = acc;
-      acc += v;
+    if (macro) {
+      *(volatile int *)&mail->macro_tiles = total;
+    } else {
+      *(volatile int *)&mail->tiles = total;
+      *(volatile long long *)&mail->unknowns = u;
     }
-    *total = acc;
+    if (seq) store_release_system(&mail->seq, seq);
+  }
+}
+
+__global__ void k_arm_waves(WaveSync *ws, int spin_limit, int skip_publish, uint4 *faces_f, uint4 *faces_b, size_t n4) {
+  if (blockIdx.x == 0 && threadIdx.x < 3) {
+    WaveSync *w = ws + threadIdx.x;
+    w->error = 0;
+    w->spin_limit = spin_limit;
+    w->skip_publish = threadIdx.x == 1 ? skip_publish : 0;
+  }
+  const uint4 unset = make_uint4(~0u, ~0u, ~0u, ~0u);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
+    faces_f[i] = unset;
+    faces_b[i] = unset;
   }
 }
 
@@ -138,16 +162,7 @@ __global__ void k_pool_neighbours(Geometry G, const int *tile_state, const int *
   if (level_count) atomicAdd(&level_count[ti + tj + tk], 1);
 }
 
-__global__ void k_level_scan(int *level_count, int nlev) {
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int i = 0; i < nlev; ++i) {
-      const int v = level_count[i];
-      level_count[i] = acc;
-      acc += v;
-    }
-  }
-}
+__global__ void k_level_scan(int *level_count, int nlev) { warp_scan_counts(level_count, nlev); }
 
 __global__ void k_level_scatter(Geometry G, const int *pool_tile, int K, int *level_cursor, int *sched) {
   const int pt = blockIdx.x * blockDim.x + threadIdx.x;
@@ -344,6 +359,7 @@ __global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, co
       if (!(pq == pq) || pq == 0.0) {
         st->done = 3;
         if (!(pq == pq)) st->status = -5;
+        report_progress(st);
       }
       *counter = 0;
     }
@@ -392,6 +408,7 @@ __global__ void __launch_bounds__(256) k_update_xr(int n4, const float4 *__restr
       else if (mm <= st->tol_abs) st->done = 1;
       else if (st->iter >= max_iterations) st->done = 2;
       else if (mm < st->ru_threshold) st->done = 4;
+      report_progress_rmax(st);
       *counter = 0;
     }
   }
@@ -409,6 +426,7 @@ __global__ void __launch_bounds__(1024) k_finish_rho(const double *partials, int
       if (s == 0.0 || !(s == s)) {
         st->done = 3;
         if (!(s == s)) st->status = -5;
+        report_progress(st);
       }
     } else {
       st->beta = s / st->rho;
@@ -814,7 +832,7 @@ __global__ void k_macro_sub(Geometry G, Geometry M, const int *macro_tile, int K
 // scaled copy r32 = r64 / ||r64||inf for the next inner solve.
 __global__ void __launch_bounds__(256) k_residual64(PoolSystem S, const double *__restrict__ b, const double *__restrict__ x,
                                                     double *__restrict__ r, double *partials, unsigned *counter,
-                                                    double *out3) {
+                                                    MailSlot slot) {
   __shared__ double red[8];
   double m = 0.0, s2 = 0.0, bm = 0.0, b2 = 0.0;
   const size_t n = (size_t)S.K * SHKZ_TC;
@@ -879,11 +897,16 @@ __global__ void __launch_bounds__(256) k_residual64(PoolSystem S, const double *
     a2 = block_max<256>(a2, red);
     a3 = block_sum<256>(a3, red);
     if (threadIdx.x == 0) {
-      out3[0] = a0;
-      out3[1] = a1;
-      out3[2] = a2;
-      out3[3] = a3;
       *counter = 0;
+      if (slot.mail) {
+        volatile double *o = slot.mail->norms;
+        o[0] = a0;
+        o[1] = a1;
+        o[2] = a2;
+        o[3] = a3;
+        *(volatile int *)&slot.mail->wave_error = any_wave_error(slot.waves);
+        store_release_system(&slot.mail->seq, slot.seq);
+      }
     }
   }
 }
@@ -959,6 +982,7 @@ __global__ void __launch_bounds__(256) k_inner_setup(int n, const float *__restr
       st->beta = 0.0;
       st->x_pending = 0;
       st->ru_threshold = 0.0;
+      if (st->mail) *(volatile double *)&st->mail->rmax = mm;
       *counter = 0;
     }
   }
@@ -1173,6 +1197,7 @@ __global__ void __launch_bounds__(256) k_fpcg_dots(int n4, const float4 *__restr
         st->done = 3;
         if (!(ta == ta)) st->status = -5;
       }
+      if (st->done) report_progress(st);
       *counter = 0;
     }
   }
@@ -1211,17 +1236,20 @@ static int grid_for(long long n, int per, int cap) {
   return (int)g;
 }
 
-int pool_count(const Geometry &G, const int *tile_count, int *scratch_bsum, int *d_total, cudaStream_t s) {
+void launch_pool_count(const Geometry &G, const int *tile_count, int *bsum, long long *usum, bool macro, Mailbox *mail,
+                       unsigned seq, cudaStream_t s) {
   const long long nt = G.ntiles;
   const int nb = (int)((nt + 1023) / 1024);
+  count_launches(2);
+  k_pool_blocksum<<<nb, 256, 0, s>>>(tile_count, nt, bsum, usum);
+  k_pool_scan<<<1, 32, 0, s>>>(bsum, usum, nb, macro, mail, seq);
+}
+
+void launch_arm_waves(void *ws, int spin_limit, int skip_publish, float *faces_f, float *faces_b, size_t n,
+                      cudaStream_t s) {
   count_launches(1);
-  k_pool_blocksum<<<nb, 256, 0, s>>>(tile_count, nt, scratch_bsum);
-  count_launches(1);
-  k_pool_scan_blocks<<<1, 32, 0, s>>>(scratch_bsum, nb, d_total);
-  int K = -1;
-  if (cudaMemcpyAsync(&K, d_total, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) return -1;
-  if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-  return K;
+  k_arm_waves<<<grid_for((long long)(n / 4) + 1, 256, 148 * 8), 256, 0, s>>>(
+      (WaveSync *)ws, spin_limit, skip_publish, (uint4 *)faces_f, (uint4 *)faces_b, n / 4);
 }
 
 void pool_assign(const Geometry &G, const int *tile_count, int K, const int *scratch_bsum, int *tile_state,
@@ -1341,10 +1369,10 @@ void launch_macro_count(const Geometry &G, const int *tile_count, const Geometry
 }
 
 void launch_residual64(const PoolSystem &S, const double *b, const double *x, double *r, double *partials,
-                       unsigned *counter, double *out4, cudaStream_t s) {
+                       unsigned *counter, const MailSlot &mail, cudaStream_t s) {
   const long long n = (long long)S.K * SHKZ_TC;
   count_launches(1);
-  k_residual64<<<grid_for(n, 256 * 4, 148 * 8), 256, 0, s>>>(S, b, x, r, partials, counter, out4);
+  k_residual64<<<grid_for(n, 256 * 4, 148 * 8), 256, 0, s>>>(S, b, x, r, partials, counter, mail);
 }
 
 void launch_inner_init(int n, const double *r64, double inv_scale, float *r32, float *x32, cudaStream_t s) {

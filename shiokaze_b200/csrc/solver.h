@@ -5,8 +5,23 @@
 
 namespace shkz {
 
-// Number of tiles holding unknowns (synchronises the stream), then the pool itself.
-int pool_count(const Geometry &G, const int *tile_count, int *scratch_bsum, int *d_total, cudaStream_t s);
+// A report to the host: the context's mailbox, the number it is to carry and
+// the wave-sync words whose errors go with it. mail null: none.
+struct MailSlot {
+  Mailbox *mail = nullptr;
+  unsigned seq = 0;
+  const void *waves = nullptr;
+};
+// Tiles holding unknowns and their unknowns (bsum/usum: one entry per 1024
+// tiles; bsum is left as the offsets pool_assign wants), reported as the
+// pool's or, with macro, the macro tiles' count. The last of a call's counts
+// carries the mail number.
+void launch_pool_count(const Geometry &G, const int *tile_count, int *bsum, long long *usum, bool macro, Mailbox *mail,
+                       unsigned seq, cudaStream_t s);
+// wave-sync error words cleared, limit and fault slot written, n face words of
+// each sweep unset
+void launch_arm_waves(void *ws, int spin_limit, int skip_publish, float *faces_f, float *faces_b, size_t n,
+                      cudaStream_t s);
 // level_count / sched null: no wavefront schedule
 void pool_assign(const Geometry &G, const int *tile_count, int K, const int *scratch_bsum, int *tile_state,
                  int *pool_tile, int *nbr, int *level_count, int *sched, cudaStream_t s);
@@ -59,7 +74,7 @@ void launch_pencil_coefs(const PoolSystem &S, const float *d32, cudaStream_t s);
 void launch_pencil_sweeps(const PoolSystem &S, const float *r, float *z, double *partials, void *ws_f, void *ws_b,
                           const SolverState *st, const SweepUpdate &fu, unsigned *finish, cudaStream_t s);
 void launch_residual64(const PoolSystem &S, const double *b, const double *x, double *r, double *partials,
-                       unsigned *counter, double *out4, cudaStream_t s);
+                       unsigned *counter, const MailSlot &mail, cudaStream_t s);
 void launch_inner_init(int n, const double *r64, double inv_scale, float *r32, float *x32, cudaStream_t s);
 void launch_accumulate(int n, const float *x32, double scale, double *x64, cudaStream_t s);
 // x64 += scale * (x32 + alpha p), the direction chosen as in launch_spmv_update

@@ -1,0 +1,72 @@
+"""The solve loop's host side: iterations queued ahead of the device's reports,
+and the pool's counts it reports. What is queued beyond the last iteration must
+not show in the results."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(sc, **config):
+    from shiokaze_b200.projection import MacGrid, MacPressureSolver3
+    s = MacPressureSolver3(config)
+    s.initialize(sc.shape, sc.dx)
+    vel = MacGrid([v.copy() for v in sc.velocity], [a.copy() for a in sc.velocity_active])
+    res = s.project(sc.dt, vel, sc.solid, sc.solid_velocity, sc.fluid)
+    return res, s.get_pressure().values, vel.values
+
+
+class _Scene:
+    def __init__(self, shape, filled, seed, block):
+        from shiokaze_b200.projection import Grid
+        nx, ny, nz = self.shape = shape
+        self.dx, self.dt = 1.0 / max(shape), 0.01
+        self.solid = self.solid_velocity = None
+        rng = np.random.default_rng(seed)
+        n = [(m + block - 1) // block for m in (nz, ny, nx)]
+        inside = (rng.random(n) < filled).repeat(block, 0).repeat(block, 1).repeat(block, 2)[:nz, :ny, :nx]
+        phi = np.where(inside, -0.7, 0.7).astype(np.float32) * np.float32(self.dx)
+        self.fluid = Grid(phi, np.ones(phi.shape, np.uint8))
+        self.velocity = [rng.standard_normal((nz + (d == 2), ny + (d == 1), nx + (d == 0)), dtype=np.float32)
+                         for d in range(3)]
+        self.velocity_active = [np.ones(v.shape, np.uint8) for v in self.velocity]
+
+
+@pytest.mark.parametrize("precond,block", [("mic0", 16), ("mic0", 8), ("none", 16)])
+@pytest.mark.parametrize("limit", [1, 2, 7, 30000])
+def test_queue_depth_does_not_show(precond, block, limit):
+    sc = _Scene((40, 33, 50), 0.6, 5, 16)
+    config = {"Residual": 1e-5, "MaxIterations": limit, "B200.Preconditioner": precond, "B200.MICBlock": block}
+    res, p, vel = _solve(sc, **config, **{"B200.CheckInterval": 1})
+    assert res["iterations"] <= limit
+    if limit <= 7:
+        assert res["iterations"] == limit
+    else:
+        assert res["reresid"] <= 1e-5
+    for depth in (2, 16):
+        other, po, velo = _solve(sc, **config, **{"B200.CheckInterval": depth})
+        assert other["iterations"] == res["iterations"] and other["reresid"] == res["reresid"]
+        np.testing.assert_array_equal(p, po)
+        for a, b in zip(vel, velo):
+            np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("shape,filled", [
+    ((24, 16, 49152), 0.02),   # 36864 tiles: 37 block sums, levels by the thousand
+    ((264, 32, 16), 0.5),
+    ((8, 8, 8), 1.0),
+])
+@pytest.mark.parametrize("block", [16, 8])
+def test_pool_counts(shape, filled, block):
+    from shiokaze_b200.projection import MacGrid, MacPressureSolver3
+    sc = _Scene(shape, filled, 7, 8)
+    s = MacPressureSolver3({"Residual": 1e-2, "MaxIterations": 2, "B200.MICBlock": block})
+    s.initialize(sc.shape, sc.dx)
+    res = s.project(sc.dt, MacGrid(sc.velocity, sc.velocity_active), None, None, sc.fluid)
+    act = s.get_pressure().active.astype(bool)
+    pad = np.zeros([(m + 7) // 8 * 8 for m in act.shape], bool)
+    pad[:act.shape[0], :act.shape[1], :act.shape[2]] = act
+    nz, ny, nx = (m // 8 for m in pad.shape)
+    assert act.any()
+    assert res["unknowns"] == int(act.sum())
+    assert res["tiles"] == int(pad.reshape(nz, 8, ny, 8, nx, 8).any(axis=(1, 3, 5)).sum())
