@@ -659,9 +659,8 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
   }
   const double scale = bmax;
   const bool reliable = ctx->cfg.refine != 0;
-  launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, s);
-  launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st, tol, s);
-  launch_state_resume(ctx->st, reliable ? kReliableDrop : 0.0, s);
+  launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, nullptr, 0.0, s);
+  launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st, tol, reliable ? kReliableDrop : 0.0, s);
   reset_progress(ctx, 0);
   // z0 = M^-1 r0, rho0, p0 = z0
   if (precond == SHKZ_B200_PRECOND_MIC0) {
@@ -721,8 +720,7 @@ static int solve_system(shkz_b200_ctx *ctx, double tol, int precond, shkz_b200_r
     if (rmax <= tol * bmax) break;
     reset_progress(ctx, hst.iter);
     queued = hst.iter;
-    launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, s);
-    launch_state_resume(ctx->st, kReliableDrop * rmax / scale, s);
+    launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, ctx->st, kReliableDrop * rmax / scale, s);
     true_checked = false;
     // complete the interrupted iteration with the replaced residual (the
     // fused loop leaves the direction update to its next stencil)
@@ -1885,9 +1883,8 @@ static int learned_solve(shkz_b200_ctx *ctx, double tol, shkz_b200_result *res) 
     return 0;
   }
   const double scale = bmax;
-  launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, s);
-  launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st, tol, s);
-  launch_state_resume(ctx->st, kReliableDrop, s);
+  launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, nullptr, 0.0, s);
+  launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st, tol, kReliableDrop, s);
   reset_progress(ctx, 0);
   bool use_mic = false;
   auto precondition = [&](double rmax_scaled) -> int {
@@ -1940,9 +1937,8 @@ static int learned_solve(shkz_b200_ctx *ctx, double tol, shkz_b200_result *res) 
       if (!(rmax_true == rmax_true)) { rc = SHKZ_B200_ERR_NAN; break; }
       if (rmax_true <= tol * bmax) break;
       reset_progress(ctx, hst.iter);
-      launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, s);
       ru_threshold = kReliableDrop * rmax_true / scale;
-      launch_state_resume(ctx->st, ru_threshold, s);
+      launch_inner_init(n, ctx->r64, 1.0 / scale, ctx->r, ctx->x, ctx->st, ru_threshold, s);
       rmax = rmax_true / scale;
     }
     hist.push_back(rmax);
@@ -2189,17 +2185,17 @@ extern "C" int shkz_b200_learned_train(shkz_b200_ctx *ctx, int steps, double lr,
       launch_rand_unknowns(n, ctx->diag, seed * 7919u + (unsigned)i, ctx->t, s);
       launch_spmv(S, ctx->t, ctx->q, ctx->partials, ctx->counter, nullptr, 1, s);
       // balance the two parts by their sizes
-      launch_inner_setup(n, ctx->q, ctx->partials, ctx->counter, ctx->st_scratch, 1.0, s);
+      launch_inner_setup(n, ctx->q, ctx->partials, ctx->counter, ctx->st_scratch, 1.0, 0.0, s);
       SolverState a1;
       cudaMemcpyAsync(&a1, ctx->st_scratch, sizeof(a1), cudaMemcpyDeviceToHost, s);
-      launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st_scratch, 1.0, s);
+      launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st_scratch, 1.0, 0.0, s);
       SolverState a2;
       cudaMemcpyAsync(&a2, ctx->st_scratch, sizeof(a2), cudaMemcpyDeviceToHost, s);
       SHKZ_CUDA_TRY(cudaStreamSynchronize(s));
       const float w = (kind == 1 || a1.rmax0 == 0.0) ? 1.0f : (float)(a2.rmax0 / a1.rmax0);
       launch_axpby_f32(n, w, ctx->q, 1.0f, ctx->r, s);
     }
-    launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st_scratch, 1.0, s);
+    launch_inner_setup(n, ctx->r, ctx->partials, ctx->counter, ctx->st_scratch, 1.0, 0.0, s);
     SolverState a3;
     SHKZ_CUDA_TRY(cudaMemcpyAsync(&a3, ctx->st_scratch, sizeof(a3), cudaMemcpyDeviceToHost, s));
     SHKZ_CUDA_TRY(cudaStreamSynchronize(s));

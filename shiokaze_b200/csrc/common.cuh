@@ -65,6 +65,12 @@ struct SolverState {
   const void *waves;       // the context's wave-sync words, whose errors are reported with it
 };
 
+// A kernel launched by launch_overlapped may start while the kernel before it
+// in the stream runs: it reads and writes global memory only after
+// wait_for_previous, which returns once that kernel (and so, kernel by kernel,
+// everything before it) is complete and its writes are visible.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Block-wide sum of one double; every thread gets the result.
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double *smem) {
@@ -92,6 +98,26 @@ __device__ __forceinline__ double block_max(double v, double *smem) {
   #pragma unroll
   for (int i = 0; i < NT / 32; ++i) s = fmax(s, smem[i]);
   return s;
+}
+
+// Launch of a kernel that begins with wait_for_previous. Its blocks take the
+// place of the previous kernel's as those finish, instead of 2.5 us after the
+// last one: a 64^3 dam break 2.41 -> 2.16 ms a projection, a 256^3 tank 65.8 ->
+// 64.4. (With an explicit launch_dependents at the top of the iteration's
+// kernels, 2.20 and 69: early blocks of the sweeps are in the stencil's way.)
+template <class... P, class... A>
+inline void launch_overlapped(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
 }  // namespace shkz

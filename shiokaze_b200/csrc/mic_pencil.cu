@@ -213,7 +213,8 @@ struct RingOf {
 using Ring = RingOf<NU>;
 
 // Prologue shared by the sweeps: barriers, wait limit.
-__device__ __forceinline__ void begin(Smem &sm, WaveSync *ws, int full_count, int freed_count) {
+// False: the solve has stopped, nothing to do.
+__device__ __forceinline__ bool begin(Smem &sm, WaveSync *ws, const SolverState *st, int full_count, int freed_count) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < NU; ++i) {
       mb_init(&sm.full[i], full_count);
@@ -228,11 +229,16 @@ __device__ __forceinline__ void begin(Smem &sm, WaveSync *ws, int full_count, in
     for (int i = 0; i < SEGQ; ++i) mb_init(&sm.segfull[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async();
+  }
+  wait_for_previous();
+  if (st && *(volatile const int *)&st->done) return false;
+  if (threadIdx.x == 0) {
     sm.dead = 0;
     sm.limit = spin_rounds(ws);
     sm.skip = *((volatile int *)&ws->skip_publish);
   }
   __syncthreads();
+  return true;
 }
 
 // The next pencil of this CTA for one role; false after the last.
@@ -605,10 +611,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_pencil_forward(PoolSystem S, co
                                                                 WaveSync *ws, const SolverState *st, SweepUpdate fu) {
   extern __shared__ __align__(128) unsigned char raw[];
   Smem &sm = *reinterpret_cast<Smem *>(raw);
-  if (st && st->done) return;
+  if (!begin(sm, ws, st, 1 + 4, 1)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nseg = *S.nseg;
-  begin(sm, ws, 1 + 4, 1);
   const int mover = mover_index(warp);
   if (warp == W_SOLVE) {
     solve_pencils<false>(sm, S.mfaces_f, ws);
@@ -776,10 +781,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_pencil_backward(PoolSystem S, c
                                                                  SolverState *st, unsigned *finish) {
   extern __shared__ __align__(128) unsigned char raw[];
   Smem &sm = *reinterpret_cast<Smem *>(raw);
-  if (st && st->done) return;
+  if (!begin(sm, ws, st, 1, 4)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nseg = *S.nseg;
-  begin(sm, ws, 1, 4);
   const int mover = mover_index(warp);
   if (warp == W_SOLVE) {
     solve_pencils<true>(sm, S.mfaces_b, ws);
@@ -891,13 +895,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_pencil_backward(PoolSystem S, c
 // per factorisation, so that the sweeps' staging is plain bulk copies.
 __global__ void __launch_bounds__(256) k_pencil_coefs(PoolSystem S, const float *__restrict__ d32,
                                                       float *__restrict__ cf, float *__restrict__ cb) {
-  const int mt = blockIdx.x, lane = threadIdx.x & 31, j = threadIdx.x >> 5;
+  const int mt = blockIdx.x, x0 = 4 * blockIdx.y, lane = threadIdx.x & 31, j = threadIdx.x >> 5;
   const int field = j >> 1, y = 2 * (lane >> 2) + (j & 1), bz = lane & 3;
   const float *src = field == 0 ? d32 : field == 1 ? S.offx : field == 2 ? S.offy : S.offz;
   __shared__ int sub[8];
   if (threadIdx.x < 8) sub[threadIdx.x] = S.msub[mt * 8 + threadIdx.x];
   __syncthreads();
-  for (int x = 0; x < 16; ++x) {
+  for (int x = x0; x < x0 + 4; ++x) {
     float lo[4], up[4];
     #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -957,7 +961,8 @@ void build_pencils(const Geometry &M, const int *mtile, const int *mnbr, int KM,
 
 void launch_pencil_coefs(const PoolSystem &S, const float *d32, cudaStream_t s) {
   count_launches(1);
-  k_pencil_coefs<<<S.KM, 256, 0, s>>>(S, d32, S.coef_f, S.coef_b);
+  // four x-planes a block: 16 as one block's work took 17 us however small the grid
+  k_pencil_coefs<<<dim3(S.KM, 4), 256, 0, s>>>(S, d32, S.coef_f, S.coef_b);
 }
 
 // one CTA per SM (its ring takes the shared memory), no more than there may be pencils
@@ -979,9 +984,9 @@ void launch_pencil_sweeps(const PoolSystem &S, const float *r, float *z, double 
                           const SolverState *st, const SweepUpdate &fu, unsigned *finish, cudaStream_t s) {
   const int grid = pencil_grid(S);
   count_launches(2);
-  k_pencil_forward<<<grid, NTHREADS, sizeof(Smem), s>>>(S, r, (WaveSync *)ws_f, st, fu);
-  k_pencil_backward<<<grid, NTHREADS, sizeof(Smem), s>>>(S, r, z, partials, (WaveSync *)ws_b,
-                                                         const_cast<SolverState *>(st), finish);
+  launch_overlapped(k_pencil_forward, grid, NTHREADS, sizeof(Smem), s, S, r, (WaveSync *)ws_f, st, fu);
+  launch_overlapped(k_pencil_backward, grid, NTHREADS, sizeof(Smem), s, S, r, z, partials, (WaveSync *)ws_b,
+                    const_cast<SolverState *>(st), finish);
 }
 
 }  // namespace shkz

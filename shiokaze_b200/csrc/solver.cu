@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, co
                                               float *__restrict__ x) {
   __shared__ SpmvSmem sm;
   __shared__ double red[4];
+  wait_for_previous();
   if (st && st->done) return;
   double acc = 0.0;
   const int tid = threadIdx.x;
@@ -417,6 +418,7 @@ __global__ void __launch_bounds__(256) k_update_xr(int n4, const float4 *__restr
 // rho_new from partials (one per pool tile or block), beta = rho_new/rho, rho = rho_new.
 __global__ void __launch_bounds__(1024) k_finish_rho(const double *partials, int n, SolverState *st, int init) {
   __shared__ double red[32];
+  wait_for_previous();
   if (st->done) return;
   const double s = sum_partials<1024>(partials, n, red);
   if (threadIdx.x == 0) {
@@ -468,6 +470,7 @@ __global__ void __launch_bounds__(512) k_mic_colsum(PoolSystem S, double *colsum
   const int pt = blockIdx.x, c = threadIdx.x;
   const int ii = c & 7, jj = (c >> 3) & 7, kk = c >> 6;
   const size_t o = (size_t)pt * SHKZ_TC + c;
+  wait_for_previous();
   double s = 0.0;
   {
     int nb = pt, cell = c + 1;
@@ -568,6 +571,7 @@ __global__ void __launch_bounds__(64) k_mic_factor(PoolSystem S, const int *sche
   __shared__ __align__(16) double D[SHKZ_TC], Sc[SHKZ_TC], A[SHKZ_TC], WX[SHKZ_TC], WY[SHKZ_TC], WZ[SHKZ_TC];
   __shared__ double hx[64], hy[64], hz[64], hsx[64], hsy[64], hsz[64];
   int slot, target;
+  wait_for_previous();
   wave_begin(ws, slot, target);
   const int pt = sched[slot];
   const int tid = threadIdx.x, jj = tid & 7, kk = tid >> 3;
@@ -836,6 +840,7 @@ __global__ void __launch_bounds__(256) k_residual64(PoolSystem S, const double *
   __shared__ double red[8];
   double m = 0.0, s2 = 0.0, bm = 0.0, b2 = 0.0;
   const size_t n = (size_t)S.K * SHKZ_TC;
+  wait_for_previous();
   for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
     const int pt = (int)(o >> 9), c = (int)(o & 511);
     const int ii = c & 7, jj = (c >> 3) & 7, kk = c >> 6;
@@ -911,9 +916,17 @@ __global__ void __launch_bounds__(256) k_residual64(PoolSystem S, const double *
   }
 }
 
-// Start of an inner FP32 solve on r32 = r64 * inv_scale; x32 = 0.
+// Start of an inner FP32 solve on r32 = r64 * inv_scale; x32 = 0. With st the
+// loop that stopped is resumed.
 __global__ void __launch_bounds__(256) k_inner_init(int n, const double *__restrict__ r64, double inv_scale,
-                                                    float *__restrict__ r32, float *__restrict__ x32) {
+                                                    float *__restrict__ r32, float *__restrict__ x32,
+                                                    SolverState *st, double ru_threshold) {
+  wait_for_previous();
+  if (st && blockIdx.x == 0 && threadIdx.x == 0) {
+    st->done = 0;
+    st->x_pending = 0;  // folded in by launch_accumulate_pending
+    st->ru_threshold = ru_threshold;
+  }
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     r32[i] = (float)(r64[i] * inv_scale);
     x32[i] = 0.0f;
@@ -933,6 +946,7 @@ __global__ void __launch_bounds__(256) k_accumulate(int n, const float *__restri
 __global__ void __launch_bounds__(256) k_accumulate_pending(int n, const float *__restrict__ x32,
                                                             const float *p0, const float *p1, const SolverState *st,
                                                             double scale, double *__restrict__ x64) {
+  wait_for_previous();
   const float alpha = st->x_pending ? (float)st->alpha : 0.0f;
   const float *__restrict__ p = (st->iter & 1) ? p1 : p0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -948,9 +962,11 @@ __global__ void __launch_bounds__(256) k_to_float(int n, const double *__restric
 
 // rmax0 and the absolute tolerance of an inner solve from r32 (= its rhs).
 __global__ void __launch_bounds__(256) k_inner_setup(int n, const float *__restrict__ r, double *partials,
-                                                     unsigned *counter, SolverState *st, double tol) {
+                                                     unsigned *counter, SolverState *st, double tol,
+                                                     double ru_threshold) {
   __shared__ double red[8];
   double m = 0.0, s2 = 0.0;
+  wait_for_previous();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     m = fmax(m, fabs((double)r[i]));
     s2 += (double)r[i] * r[i];
@@ -975,13 +991,12 @@ __global__ void __launch_bounds__(256) k_inner_setup(int n, const float *__restr
       st->r2 = ss;
       st->tol_abs = tol * mm;
       st->iter = 0;
-      st->done = (mm == 0.0) ? 1 : 0;
+      st->done = 0;
       st->status = (ss == ss) ? 0 : -5;
-      if (!(ss == ss)) st->done = 3;
       st->rho = 0.0;
       st->beta = 0.0;
       st->x_pending = 0;
-      st->ru_threshold = 0.0;
+      st->ru_threshold = ru_threshold;
       if (st->mail) *(volatile double *)&st->mail->rmax = mm;
       *counter = 0;
     }
@@ -1284,7 +1299,7 @@ void launch_spmv_update(const PoolSystem &S, float *p0, float *p1, const float *
                         double *partials, unsigned *counter, SolverState *st, cudaStream_t s) {
   if (S.K <= 0) return;
   count_launches(1);
-  k_spmv<<<spmv_grid(S.K), 128, 0, s>>>(S, p0, q, partials, counter, st, 0, z, p1, x);
+  launch_overlapped(k_spmv, spmv_grid(S.K), 128, 0, s, S, p0, q, partials, counter, st, 0, z, p1, x);
 }
 
 // one wave of resident CTAs looping over the tiles
@@ -1300,7 +1315,7 @@ void launch_update_xr(int n, const float *p, const float *q, float *x, float *r,
 
 void launch_finish_rho(const double *partials, int n, SolverState *st, int init, cudaStream_t s) {
   count_launches(1);
-  k_finish_rho<<<1, 1024, 0, s>>>(partials, n, st, init);
+  launch_overlapped(k_finish_rho, 1, 1024, 0, s, partials, n, st, init);
 }
 void launch_finish_rho_r2(SolverState *st, int init, cudaStream_t s) {
   count_launches(1);
@@ -1317,9 +1332,9 @@ void launch_mic_factor(const PoolSystem &S, double *colsum, double omega, double
                        int *flags, void *ws, cudaStream_t s) {
   if (S.K <= 0) return;
   count_launches(1);
-  k_mic_colsum<<<S.K, 512, 0, s>>>(S, colsum);
+  launch_overlapped(k_mic_colsum, S.K, 512, 0, s, S, colsum);
   count_launches(1);
-  k_mic_factor<<<S.K, 64, 0, s>>>(S, S.sched, colsum, omega, min_ratio, d64, d32, flags, (WaveSync *)ws);
+  launch_overlapped(k_mic_factor, S.K, 64, 0, s, S, S.sched, colsum, omega, min_ratio, d64, d32, flags, (WaveSync *)ws);
   if (S.KM > 0) launch_pencil_coefs(S, d32, s);
 }
 
@@ -1372,12 +1387,13 @@ void launch_residual64(const PoolSystem &S, const double *b, const double *x, do
                        unsigned *counter, const MailSlot &mail, cudaStream_t s) {
   const long long n = (long long)S.K * SHKZ_TC;
   count_launches(1);
-  k_residual64<<<grid_for(n, 256 * 4, 148 * 8), 256, 0, s>>>(S, b, x, r, partials, counter, mail);
+  launch_overlapped(k_residual64, grid_for(n, 256 * 4, 148 * 8), 256, 0, s, S, b, x, r, partials, counter, mail);
 }
 
-void launch_inner_init(int n, const double *r64, double inv_scale, float *r32, float *x32, cudaStream_t s) {
+void launch_inner_init(int n, const double *r64, double inv_scale, float *r32, float *x32, SolverState *st,
+                       double ru_threshold, cudaStream_t s) {
   count_launches(1);
-  k_inner_init<<<grid_for(n, 256 * 4, 148 * 8), 256, 0, s>>>(n, r64, inv_scale, r32, x32);
+  launch_overlapped(k_inner_init, grid_for(n, 256, 148 * 8), 256, 0, s, n, r64, inv_scale, r32, x32, st, ru_threshold);
 }
 void launch_accumulate(int n, const float *x32, double scale, double *x64, cudaStream_t s) {
   count_launches(1);
@@ -1386,7 +1402,7 @@ void launch_accumulate(int n, const float *x32, double scale, double *x64, cudaS
 void launch_accumulate_pending(int n, const float *x32, const float *p0, const float *p1, const SolverState *st,
                                double scale, double *x64, cudaStream_t s) {
   count_launches(1);
-  k_accumulate_pending<<<grid_for(n, 256 * 4, 148 * 8), 256, 0, s>>>(n, x32, p0, p1, st, scale, x64);
+  launch_overlapped(k_accumulate_pending, grid_for(n, 256, 148 * 8), 256, 0, s, n, x32, p0, p1, st, scale, x64);
 }
 void launch_to_float(int n, const double *a, float *b, cudaStream_t s) {
   count_launches(1);
@@ -1398,9 +1414,10 @@ void launch_state_resume(SolverState *st, double ru_threshold, cudaStream_t s) {
 }
 
 void launch_inner_setup(int n, const float *r, double *partials, unsigned *counter, SolverState *st, double tol,
-                        cudaStream_t s) {
+                        double ru_threshold, cudaStream_t s) {
   count_launches(1);
-  k_inner_setup<<<grid_for(n, 256 * 4, 148 * 8), 256, 0, s>>>(n, r, partials, counter, st, tol);
+  launch_overlapped(k_inner_setup, grid_for(n, 256 * 4, 148 * 8), 256, 0, s, n, r, partials, counter, st, tol,
+                    ru_threshold);
 }
 
 }  // namespace shkz

@@ -75,7 +75,9 @@ void launch_pencil_sweeps(const PoolSystem &S, const float *r, float *z, double 
                           const SolverState *st, const SweepUpdate &fu, unsigned *finish, cudaStream_t s);
 void launch_residual64(const PoolSystem &S, const double *b, const double *x, double *r, double *partials,
                        unsigned *counter, const MailSlot &mail, cudaStream_t s);
-void launch_inner_init(int n, const double *r64, double inv_scale, float *r32, float *x32, cudaStream_t s);
+// st (may be null): also resumes the loop, its next residual replacement below ru_threshold
+void launch_inner_init(int n, const double *r64, double inv_scale, float *r32, float *x32, SolverState *st,
+                       double ru_threshold, cudaStream_t s);
 void launch_accumulate(int n, const float *x32, double scale, double *x64, cudaStream_t s);
 // x64 += scale * (x32 + alpha p), the direction chosen as in launch_spmv_update
 void launch_accumulate_pending(int n, const float *x32, const float *p0, const float *p1, const SolverState *st,
@@ -83,7 +85,7 @@ void launch_accumulate_pending(int n, const float *x32, const float *p0, const f
 void launch_to_float(int n, const double *a, float *b, cudaStream_t s);
 void launch_state_resume(SolverState *st, double ru_threshold, cudaStream_t s);
 void launch_inner_setup(int n, const float *r, double *partials, unsigned *counter, SolverState *st, double tol,
-                        cudaStream_t s);
+                        double ru_threshold, cudaStream_t s);
 
 void launch_apply64(const PoolSystem &S, const double *x, double *y, cudaStream_t s);
 void launch_dots64(int n, const double *a, const double *b, const double *c, const double *d, double *partials,
