@@ -35,6 +35,8 @@
 #include "solver.h"
 #include "wave.cuh"
 #include <math_constants.h>
+
+#include <algorithm>
 #include <atomic>
 
 namespace shkz {
@@ -834,55 +836,83 @@ __global__ void k_macro_sub(Geometry G, Geometry M, const int *macro_tile, int K
 // ---------------------------------------------------------------------------
 // FP64 residual r64 = b64 - A64 x64 (x64 in FP64), its norms, and the FP32
 // scaled copy r32 = r64 / ||r64||inf for the next inner solve.
-__global__ void __launch_bounds__(256) k_residual64(PoolSystem S, const double *__restrict__ b, const double *__restrict__ x,
-                                                    double *__restrict__ r, double *partials, unsigned *counter,
-                                                    MailSlot slot) {
+// One tile a trip, 128 threads, four x-consecutive cells a thread (two 16-byte
+// accesses an array), x staged with its six halo faces as the FP32 stencil
+// does; the upper weights are the neighbour cells' lower ones and come from the
+// lines their owners load. Bound by its 56 bytes a cell: 256^3 tank (8.6 M
+// cells) 100 us, 512^3 rain 291 us; 194 and 586 us with a thread per cell that
+// looked each neighbour up in global memory.
+#define RESIDUAL_CTAS_PER_SM 4  // 126 registers; at 5 and 6 a SM the values spill: 101 and 129 us
+__global__ void __launch_bounds__(128, RESIDUAL_CTAS_PER_SM) k_residual64(PoolSystem S, const double *__restrict__ b,
+                                                    const double *__restrict__ x, double *__restrict__ r,
+                                                    double *partials, unsigned *counter, MailSlot slot) {
   __shared__ double red[8];
+  __shared__ __align__(16) double xs[10][10][12];  // (kk+1, jj+1, ii+2); halos at kk/jj 0,9 and ii 1,10
   double m = 0.0, s2 = 0.0, bm = 0.0, b2 = 0.0;
-  const size_t n = (size_t)S.K * SHKZ_TC;
+  const int tid = threadIdx.x, q4 = tid & 1, jj = (tid >> 1) & 7, kk = tid >> 4;
+  const int c = kk * 64 + jj * 8 + q4 * 4;
+  const int side = tid >> 6, fa = tid & 7, fb = (tid >> 3) & 7;  // halo value of this thread on each axis
   wait_for_previous();
-  for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
-    const int pt = (int)(o >> 9), c = (int)(o & 511);
-    const int ii = c & 7, jj = (c >> 3) & 7, kk = c >> 6;
-    auto xat = [&](int nbslot, int cell, bool inside) -> double {
-      if (inside) return x[(size_t)pt * SHKZ_TC + cell];
-      const int nb = S.nbr[pt * 6 + nbslot];
-      return nb >= 0 ? x[(size_t)nb * SHKZ_TC + cell] : 0.0;
+  for (int pt = blockIdx.x; pt < S.K; pt += gridDim.x) {
+    const size_t o = (size_t)pt * SHKZ_TC + c;
+    const int *nbr = S.nbr + pt * 6;
+    double xv[4], dg[4], lx[4], ly[4], lz[4], ux, uy[4], uz[4], bv[4];
+    auto load4 = [](double *v, const double *p) {
+      const double2 a = reinterpret_cast<const double2 *>(p)[0], e = reinterpret_cast<const double2 *>(p)[1];
+      v[0] = a.x; v[1] = a.y; v[2] = e.x; v[3] = e.y;
     };
-    auto wat = [&](const double *w, int nbslot, int cell, bool inside) -> double {
-      if (inside) return w[(size_t)pt * SHKZ_TC + cell];
-      const int nb = S.nbr[pt * 6 + nbslot];
-      return nb >= 0 ? w[(size_t)nb * SHKZ_TC + cell] : 0.0;
+    auto load4_if = [&](double *v, const double *w, int nb, int cell) {
+      if (nb >= 0) load4(v, w + (size_t)nb * SHKZ_TC + cell);
+      else v[0] = v[1] = v[2] = v[3] = 0.0;
     };
-    const double xc = x[o];
-    double y = S.diag64[o] * xc;
-    y -= S.offx64[o] * xat(NB_XM, ii > 0 ? c - 1 : c + 7, ii > 0);
-    y -= S.offy64[o] * xat(NB_YM, jj > 0 ? c - 8 : c + 56, jj > 0);
-    y -= S.offz64[o] * xat(NB_ZM, kk > 0 ? c - 64 : c + 448, kk > 0);
+    double hal[3];
     {
-      const int cell = ii < 7 ? c + 1 : c - 7;
-      y -= wat(S.offx64, NB_XP, cell, ii < 7) * xat(NB_XP, cell, ii < 7);
+      const int nx = nbr[NB_XM + side], ny = nbr[NB_YM + side], nz = nbr[NB_ZM + side];
+      hal[0] = nx >= 0 ? x[(size_t)nx * SHKZ_TC + (side ? 0 : 7) + 8 * fa + 64 * fb] : 0.0;
+      hal[1] = ny >= 0 ? x[(size_t)ny * SHKZ_TC + fa + (side ? 0 : 56) + 64 * fb] : 0.0;
+      hal[2] = nz >= 0 ? x[(size_t)nz * SHKZ_TC + fa + 8 * fb + (side ? 0 : 448)] : 0.0;
     }
-    {
-      const int cell = jj < 7 ? c + 8 : c - 56;
-      y -= wat(S.offy64, NB_YP, cell, jj < 7) * xat(NB_YP, cell, jj < 7);
+    load4(xv, x + o);
+    load4(dg, S.diag64 + o);
+    load4(lx, S.offx64 + o);
+    load4(ly, S.offy64 + o);
+    load4(lz, S.offz64 + o);
+    load4(bv, b + o);
+    if (q4 == 0) ux = S.offx64[o + 4];
+    else ux = nbr[NB_XP] >= 0 ? S.offx64[(size_t)nbr[NB_XP] * SHKZ_TC + c - 4] : 0.0;
+    load4_if(uy, S.offy64, jj < 7 ? pt : nbr[NB_YP], jj < 7 ? c + 8 : c - 56);
+    load4_if(uz, S.offz64, kk < 7 ? pt : nbr[NB_ZP], kk < 7 ? c + 64 : c - 448);
+    __syncthreads();  // the previous tile's values are read
+    double *row = &xs[kk + 1][jj + 1][2 + q4 * 4];
+    reinterpret_cast<double2 *>(row)[0] = make_double2(xv[0], xv[1]);
+    reinterpret_cast<double2 *>(row)[1] = make_double2(xv[2], xv[3]);
+    xs[fb + 1][fa + 1][side ? 10 : 1] = hal[0];
+    xs[fb + 1][side ? 9 : 0][fa + 2] = hal[1];
+    xs[side ? 9 : 0][fb + 1][fa + 2] = hal[2];
+    __syncthreads();
+    double rv[4];
+    #pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      // roundings spelt out: which product of the first two is fused is the compiler's choice
+      double y = __fma_rn(-lx[e], row[e - 1], __dmul_rn(dg[e], xv[e]));
+      y = __fma_rn(-ly[e], row[e - 12], y);
+      y = __fma_rn(-lz[e], row[e - 120], y);
+      y = __fma_rn(-(e < 3 ? lx[e + 1] : ux), row[e + 1], y);
+      y = __fma_rn(-uy[e], row[e + 12], y);
+      y = __fma_rn(-uz[e], row[e + 120], y);
+      rv[e] = dg[e] != 0.0 ? bv[e] - y : 0.0;
+      m = fmax(m, fabs(rv[e]));
+      s2 += rv[e] * rv[e];
+      bm = fmax(bm, fabs(bv[e]));
+      b2 += bv[e] * bv[e];
     }
-    {
-      const int cell = kk < 7 ? c + 64 : c - 448;
-      y -= wat(S.offz64, NB_ZP, cell, kk < 7) * xat(NB_ZP, cell, kk < 7);
-    }
-    const double bv = b[o];
-    const double rv = S.diag64[o] != 0.0 ? bv - y : 0.0;
-    r[o] = rv;
-    m = fmax(m, fabs(rv));
-    s2 += rv * rv;
-    bm = fmax(bm, fabs(bv));
-    b2 += bv * bv;
+    reinterpret_cast<double2 *>(r + o)[0] = make_double2(rv[0], rv[1]);
+    reinterpret_cast<double2 *>(r + o)[1] = make_double2(rv[2], rv[3]);
   }
-  const double v0 = block_max<256>(m, red);
-  const double v1 = block_sum<256>(s2, red);
-  const double v2 = block_max<256>(bm, red);
-  const double v3 = block_sum<256>(b2, red);
+  const double v0 = block_max<128>(m, red);
+  const double v1 = block_sum<128>(s2, red);
+  const double v2 = block_max<128>(bm, red);
+  const double v3 = block_sum<128>(b2, red);
   if (threadIdx.x == 0) {
     partials[4 * blockIdx.x + 0] = v0;
     partials[4 * blockIdx.x + 1] = v1;
@@ -891,16 +921,16 @@ __global__ void __launch_bounds__(256) k_residual64(PoolSystem S, const double *
   }
   if (last_block(counter)) {
     double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += 256) {
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 128) {
       a0 = fmax(a0, partials[4 * i]);
       a1 += partials[4 * i + 1];
       a2 = fmax(a2, partials[4 * i + 2]);
       a3 += partials[4 * i + 3];
     }
-    a0 = block_max<256>(a0, red);
-    a1 = block_sum<256>(a1, red);
-    a2 = block_max<256>(a2, red);
-    a3 = block_sum<256>(a3, red);
+    a0 = block_max<128>(a0, red);
+    a1 = block_sum<128>(a1, red);
+    a2 = block_max<128>(a2, red);
+    a3 = block_sum<128>(a3, red);
     if (threadIdx.x == 0) {
       *counter = 0;
       if (slot.mail) {
@@ -1385,9 +1415,9 @@ void launch_macro_count(const Geometry &G, const int *tile_count, const Geometry
 
 void launch_residual64(const PoolSystem &S, const double *b, const double *x, double *r, double *partials,
                        unsigned *counter, const MailSlot &mail, cudaStream_t s) {
-  const long long n = (long long)S.K * SHKZ_TC;
   count_launches(1);
-  launch_overlapped(k_residual64, grid_for(n, 256 * 4, 148 * 8), 256, 0, s, S, b, x, r, partials, counter, mail);
+  const int grid = std::max(1, std::min(S.K, 148 * RESIDUAL_CTAS_PER_SM));
+  launch_overlapped(k_residual64, grid, 128, 0, s, S, b, x, r, partials, counter, mail);
 }
 
 void launch_inner_init(int n, const double *r64, double inv_scale, float *r32, float *x32, SolverState *st,
