@@ -110,7 +110,7 @@ struct shkz_b200_ctx {
   size_t cap_sp_raw = 0;
   float4 *sp_posm = nullptr, *sp_vc[3] = {};
   int *sp_key = nullptr, *sp_rank = nullptr, *sp_list = nullptr;
-  float4 *sp_sposm = nullptr, *sp_svc = nullptr;
+  float4 *sp_srec = nullptr;
   long long cap_sp_particles = 0;
   int *sp_faces = nullptr, *sp_sorted = nullptr, *sp_face_bin = nullptr, *sp_nfaces = nullptr, *sp_work = nullptr;
   long long cap_sp_list = 0;
@@ -472,8 +472,8 @@ extern "C" void shkz_b200_destroy(shkz_b200_ctx *ctx) {
                   ctx->prev, ctx->rank_pool, ctx->rank_cnt, ctx->rank_total, ctx->xw, ctx->h_dens[0],
                   ctx->h_dens[1], ctx->h_dens[2], ctx->flush, ctx->pb, ctx->ext_bits, ctx->ext_solid,
                   ctx->ext_flag, ctx->ext_list, ctx->sp_raw, ctx->sp_posm,
-                  ctx->sp_vc[0], ctx->sp_vc[1], ctx->sp_vc[2], ctx->sp_key, ctx->sp_rank, ctx->sp_list, ctx->sp_sposm,
-                  ctx->sp_svc, ctx->sp_faces, ctx->sp_sorted, ctx->sp_face_bin, ctx->sp_nfaces, ctx->sp_work,
+                  ctx->sp_vc[0], ctx->sp_vc[1], ctx->sp_vc[2], ctx->sp_key, ctx->sp_rank, ctx->sp_list, ctx->sp_srec,
+                  ctx->sp_faces, ctx->sp_sorted, ctx->sp_face_bin, ctx->sp_nfaces, ctx->sp_work,
                   ctx->sp_count, ctx->sp_tile_start, ctx->sp_tile_act, ctx->sp_tiles, ctx->sp_act[0],
                   ctx->sp_act[1], ctx->sp_act[2], ctx->sp_mass[0], ctx->sp_mass[1], ctx->sp_mass[2], ctx->sp_mom[0],
                   ctx->sp_mom[1], ctx->sp_mom[2],
@@ -1315,8 +1315,7 @@ static int splat_device(shkz_b200_ctx *ctx, const shkz_b200_splat_args *a, const
     GROW(sp_key, 3 * n);
     GROW(sp_rank, 3 * n);
     GROW(sp_list, 3 * n);
-    GROW(sp_sposm, 3 * n);
-    GROW(sp_svc, 3 * n);
+    GROW(sp_srec, 6 * n);
     ctx->cap_sp_particles = n;
   }
   if (!ctx->sp_nfaces) GROW(sp_nfaces, 4);
@@ -1365,8 +1364,7 @@ static int splat_device(shkz_b200_ctx *ctx, const shkz_b200_splat_args *a, const
   B.tile_act = ctx->sp_tile_act;
   B.tile_start = ctx->sp_tile_start;
   B.list = ctx->sp_list;
-  B.sposm = ctx->sp_sposm;
-  B.svc = ctx->sp_svc;
+  B.srec = ctx->sp_srec;
   B.faces = ctx->sp_faces;
   B.sorted = ctx->sp_sorted;
   B.face_bin = ctx->sp_face_bin;

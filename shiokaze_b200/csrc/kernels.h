@@ -105,7 +105,7 @@ struct SplatBuffers {
   uint8_t *tile_act;       // [tiles] the tile holds a particle
   int *tile_start;         // [tiles + 1], exclusive scan of the tiles' particle counts
   int *list;               // [3 count] d * count + particle index, bucket by bucket, arrival order inside one
-  float4 *sposm, *svc;     // [3 count] posm and vc[d] bucket by bucket, index order inside one
+  float4 *srec;            // [3 count][2] posm and vc[d] bucket by bucket, index order inside one
   uint8_t *act[3];         // faces activated by the splat
   int *faces;              // active faces of each axis, listed from face_off[d]
   int *sorted;             // the same lists, faces with more particles to visit first

@@ -20,8 +20,8 @@
 //   scatter  every particle index into its bucket's slot;
 //   sort     one thread per slot: the slot's particle goes to the rank its
 //            index has in the bucket (the atomic slots are in arrival order)
-//            and its packed data is copied there, so each bucket is
-//            contiguous and in the reference's order;
+//            and its packed data is copied there as one 32-byte record, so
+//            each bucket is contiguous and in the reference's order;
 //   compact  the activated faces of each axis into a list, then the list
 //            ordered by work class (particle visits per face);
 //   gather   one thread per listed face: visits the 16 buckets of the
@@ -37,6 +37,7 @@
 // three axes' tiles are numbered one after another. Only tiles that hold a
 // particle are scanned and cleared, so the bucket bookkeeping costs in
 // proportion to the particles' band, not to the grid.
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -49,37 +50,50 @@ namespace {
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 __device__ __forceinline__ float rec_f(const unsigned char *rec, int off, int k) {
-  return __ldg(reinterpret_cast<const float *>(rec + off) + k);
+  return reinterpret_cast<const float *>(rec + off)[k];
 }
 
-// Division by the cell size. When dx is a power of two, a / dx and
-// a * (1 / dx) are the same real number, so their correctly rounded results
-// are equal: the multiply stands in for the FP64 divide, bit for bit.
+// Division by the cell size, correctly rounded in each mode.
+//  DIV_POW2: dx is a power of two, so a / dx and a * (1 / dx) are the same real
+//    number.
+//  DIV_FMA: two corrections of a * y, y the rounded reciprocal. The first
+//    leaves a quotient within one unit in the last place, from which the second
+//    gives the rounded one (Markstein 1990: needs y rounded to nearest and a
+//    mantissa of dx that is not all ones; make_dxdiv checks both, and that
+//    nothing here over- or underflows). Five FP64 operations for three divides
+//    a visit: a 200^3 gather took 620 us with them and takes 412.
+//  DIV_ANY: the divide.
+enum { DIV_ANY = 0, DIV_POW2 = 1, DIV_FMA = 2 };
 struct DxDiv {
   double dx, inv;
-  int pow2;
+  int mode;
 };
 
-template <bool POW2>
+template <int MODE>
 __device__ __forceinline__ double div_dx(double a, const DxDiv &X) {
-  return POW2 ? a * X.inv : a / X.dx;
+  if (MODE == DIV_POW2) return a * X.inv;
+  if (MODE == DIV_FMA) {
+    double q = a * X.inv;
+    q = __fma_rn(__fma_rn(-q, X.dx, a), X.inv, q);
+    return __fma_rn(__fma_rn(-q, X.dx, a), X.inv, q);
+  }
+  return a / X.dx;
+}
+
+// the same for a position, which may be infinite
+template <int MODE>
+__device__ __forceinline__ double position_dx(float p, const DxDiv &X) {
+  const double q = div_dx<MODE>((double)p, X);
+  return MODE == DIV_FMA && !(q == q) ? (double)p : q;
 }
 
 // shape3::find_edge(p/dx, dim) on one axis (include/shiokaze/math/shape.h:
 // 748-750): p/dx rounded to FP32, plus 0.5 off the edge's own axis rounded to
 // FP32, truncated, clamped to the edge grid.
-__device__ __forceinline__ int edge_axis(float pc, const DxDiv &X, bool half, int extent) {
-  const double pd = X.pow2 ? div_dx<true>((double)pc, X) : div_dx<false>((double)pc, X);
+__device__ __forceinline__ int edge_axis(double pd, bool half, int extent) {
   const float q = __double2float_rn(pd);
   const float t = __double2float_rn((double)q + (half ? 0.5 : 0.0));
   return clampi((int)t, 0, extent - 1);
-}
-
-// one factor of macnbflip3::grid_kernel (macnbflip3.cpp:44-49)
-template <bool POW2>
-__device__ __forceinline__ double tent(float r, const DxDiv &X) {
-  const double v = 1.0 - div_dx<POW2>(fabs((double)r), X);
-  return 0.0 < v ? v : 0.0;
 }
 
 // Slot of the edge bucket e (edge coordinates on axis d, extents E): the
@@ -101,14 +115,30 @@ __device__ __forceinline__ int2 bucket_range(const SplatBuffers &B, int slot) {
   return make_int2(first, end);
 }
 
-__global__ void k_splat_bin(SplatRecords R, int nx, int ny, int nz, DxDiv X, SplatBuffers B) {
-  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+constexpr int kBinThreads = 128;
+constexpr int kStageStride = 96;
+template <int MODE>
+__global__ void __launch_bounds__(kBinThreads) k_splat_bin(SplatRecords R, int nx, int ny, int nz, DxDiv X, SplatBuffers B) {
+  // Records up to kStageStride bytes come through shared memory: read in place,
+  // each of a record's 17 words is a line of its own for every lane of a warp
+  // (1.6 M particles: 143 -> 129 us, most of it the bucket counters' atomics)
+  __shared__ unsigned stage[kBinThreads * kStageStride / 4];
+  const long long n0 = (long long)blockIdx.x * kBinThreads, n = n0 + threadIdx.x;
+  const bool staged = R.stride <= kStageStride && (R.stride & 3) == 0;
+  if (staged) {
+    const int words = (int)min((long long)kBinThreads, R.count - n0) * (R.stride >> 2);
+    const unsigned *src = reinterpret_cast<const unsigned *>(R.base + (size_t)n0 * R.stride);
+    for (int w = threadIdx.x; w < words; w += kBinThreads) stage[w] = __ldg(src + w);
+    __syncthreads();
+  }
   if (n >= R.count) return;
-  const unsigned char *rec = R.base + (size_t)n * R.stride;
+  const unsigned char *rec = staged ? reinterpret_cast<const unsigned char *>(stage) + threadIdx.x * R.stride
+                                    : R.base + (size_t)n * R.stride;
   const float p[3] = {rec_f(rec, R.off_p, 0), rec_f(rec, R.off_p, 1), rec_f(rec, R.off_p, 2)};
   B.posm[n] = make_float4(p[0], p[1], p[2], rec_f(rec, R.off_m, 0));
   const bool splats = R.splat_bullet || R.off_bullet < 0 || rec[R.off_bullet] == 0;
   const int n3[3] = {nx, ny, nz};
+  const double pd[3] = {position_dx<MODE>(p[0], X), position_dx<MODE>(p[1], X), position_dx<MODE>(p[2], X)};
   #pragma unroll
   for (int d = 0; d < 3; ++d) {
     float4 vc = make_float4(rec_f(rec, R.off_v, d), 0.f, 0.f, 0.f);
@@ -123,32 +153,28 @@ __global__ void k_splat_bin(SplatRecords R, int nx, int ny, int nz, DxDiv X, Spl
       B.key[slot] = -1;
       continue;
     }
-    int e[3], E[3];
+    int e[3], E[3], lo[3], hi[3];
     #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      E[c] = n3[c] + (c != d);
-      e[c] = edge_axis(p[c], X, c != d, E[c]);
+      const bool half = c != d;
+      E[c] = n3[c] + half;
+      e[c] = edge_axis(pd[c], half, E[c]);
+      // faces this particle activates (macnbflip3.cpp:109-120): the cell below
+      // the face-centred position and its +1 neighbours, clamped to the cells
+      const int pi = (int)(pd[c] - (half ? 0.5 : 0.0));
+      lo[c] = clampi(pi, 0, n3[c] - 1);
+      hi[c] = clampi(pi + 1, 0, n3[c] - 1);
     }
     const int key = bucket_slot(B, d, E, e);
     B.key[slot] = key;
     const int rank = atomicAdd(&B.count[key], 1);
     B.rank[slot] = rank;
     if (rank == 0) B.tile_act[key >> 9] = 1;
-    // faces this particle activates (macnbflip3.cpp:109-120): the cell below
-    // the face-centred position and its +1 neighbours, clamped to the cells
-    int pi[3];
-    #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const double pd = X.pow2 ? div_dx<true>((double)p[c], X) : div_dx<false>((double)p[c], X);
-      pi[c] = (int)(pd - (c != d ? 0.5 : 0.0));
-    }
     const int fw = nx + (d == 0), fh = ny + (d == 1);
     uint8_t *act = B.act[d];
     #pragma unroll
     for (int o = 0; o < 8; ++o) {
-      const int i = clampi(pi[0] + (o >> 2), 0, nx - 1);
-      const int j = clampi(pi[1] + ((o >> 1) & 1), 0, ny - 1);
-      const int k = clampi(pi[2] + (o & 1), 0, nz - 1);
+      const int i = o >> 2 ? hi[0] : lo[0], j = (o >> 1) & 1 ? hi[1] : lo[1], k = o & 1 ? hi[2] : lo[2];
       act[(size_t)i + (size_t)fw * ((size_t)j + (size_t)fh * k)] = 1;
     }
   }
@@ -328,6 +354,18 @@ __global__ void k_splat_scatter(long long count, SplatBuffers B) {
   }
 }
 
+// A sorted record, 32 bytes: (p, mass) and (u_d, c_d), in one access.
+__device__ __forceinline__ void store_record(float4 *p, const float4 &a, const float4 &b) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+               "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+__device__ __forceinline__ void load_record(const float4 *p, float4 &a, float4 &b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(p));
+}
+
 // One thread per bucket slot: the slot's particle goes to the position its
 // index takes among its bucket's particles (the atomic slots are in arrival
 // order), and its packed data is copied there, so that the gather reads each
@@ -337,7 +375,7 @@ __global__ void k_splat_sort_copy(long long count, SplatBuffers B) {
   const int total = B.tile_start[B.tiles];
   if (s >= total) return;
   const int sl = B.list[s];  // d * count + particle
-  const int d = (int)(sl / count);
+  const int d = (sl >= count) + (sl >= 2 * count);
   const long long n = sl - d * count;
   const int2 range = bucket_range(B, B.key[sl]);
   const int s0 = range.x, s1 = range.y;
@@ -349,8 +387,7 @@ __global__ void k_splat_sort_copy(long long count, SplatBuffers B) {
   // one bucket holds one axis' entries, so d * count + particle orders them by particle
   int r = 0;
   for (int t = s0; t < s1; ++t) r += B.list[t] < sl;
-  B.sposm[s0 + r] = B.posm[n];
-  B.svc[s0 + r] = B.vc[d][n];
+  store_record(B.srec + 2 * (size_t)(s0 + r), B.posm[n], B.vc[d][n]);
 }
 
 // active faces of axis D into a list: 16 faces a thread, one atomic a block
@@ -359,7 +396,7 @@ __global__ void k_splat_sort_copy(long long count, SplatBuffers B) {
 constexpr int kCompactThreads = 256;
 
 template <int D>
-__global__ void __launch_bounds__(kCompactThreads) k_splat_compact(int nx, int ny, int nz, SplatBuffers B) {
+__device__ __forceinline__ void compact_axis(int nx, int ny, int nz, SplatBuffers B) {
   __shared__ int warp_sums[kCompactThreads / 32];
   __shared__ int block_base;
   const size_t nf = (size_t)(nx + (D == 0)) * (ny + (D == 1)) * (nz + (D == 2));
@@ -419,7 +456,7 @@ __device__ __forceinline__ int face_visits(size_t f, int nx, int ny, int nz, con
 }
 
 template <int D>
-__global__ void __launch_bounds__(256) k_splat_face_work(int nx, int ny, int nz, SplatBuffers B) {
+__device__ __forceinline__ void face_work_axis(int nx, int ny, int nz, SplatBuffers B) {
   __shared__ int hist[kSplatWorkBins];
   for (int i = threadIdx.x; i < kSplatWorkBins; i += blockDim.x) hist[i] = 0;
   __syncthreads();
@@ -460,7 +497,7 @@ __global__ void k_splat_work_scan(SplatBuffers B) {
 // faces with shared-memory cursors (the global cursors would serialise on a
 // few addresses).
 template <int D>
-__global__ void __launch_bounds__(256) k_splat_face_sort(SplatBuffers B) {
+__device__ __forceinline__ void face_sort_axis(SplatBuffers B) {
   __shared__ int cnt[kSplatWorkBins];
   __shared__ int cur[kSplatWorkBins];
   const int nact = B.nfaces[D];
@@ -482,6 +519,23 @@ __global__ void __launch_bounds__(256) k_splat_face_sort(SplatBuffers B) {
   }
 }
 
+// the three axes in one launch each, blockIdx.y the axis
+__global__ void __launch_bounds__(kCompactThreads) k_splat_compact(int nx, int ny, int nz, SplatBuffers B) {
+  if (blockIdx.y == 0) compact_axis<0>(nx, ny, nz, B);
+  else if (blockIdx.y == 1) compact_axis<1>(nx, ny, nz, B);
+  else compact_axis<2>(nx, ny, nz, B);
+}
+__global__ void __launch_bounds__(256) k_splat_face_work(int nx, int ny, int nz, SplatBuffers B) {
+  if (blockIdx.y == 0) face_work_axis<0>(nx, ny, nz, B);
+  else if (blockIdx.y == 1) face_work_axis<1>(nx, ny, nz, B);
+  else face_work_axis<2>(nx, ny, nz, B);
+}
+__global__ void __launch_bounds__(256) k_splat_face_sort(SplatBuffers B) {
+  if (blockIdx.y == 0) face_sort_axis<0>(B);
+  else if (blockIdx.y == 1) face_sort_axis<1>(B);
+  else face_sort_axis<2>(B);
+}
+
 // The 16 visits of get_face_neighbors (pointgridhash3.cpp:218-231), in its
 // loop order dir, ri, rj, rk, reach the 8 distinct buckets of bucket_coords:
 // the loop variable of the face's own axis D does not move the bucket.
@@ -494,23 +548,102 @@ __device__ __forceinline__ int visit_bucket(int v) {
 }
 
 constexpr int kGatherThreads = 256;
-constexpr int kGatherBatch = 4;
+constexpr int kGatherBatch = 3;
+
+// a rounded to FP32, as a double
+__device__ __forceinline__ double round_fp32(double a) { return (double)__double2float_rn(a); }
+
+// The visits of one face, summed in order. FAR: dx is a power of two and the
+// face lies two cells or more from the axis planes. Its position is then an
+// FP32 value; the FP64 difference of two FP32 values rounded to FP32 is their
+// FP32 difference (2 * 24 + 2 <= 53 bits), and inside the tent, where the two
+// are within a factor of two, it is exact, so it stands for both.
+template <int D, int MODE, bool FAR>
+__device__ __forceinline__ void sum_visits(bool has, const int2 (*range)[kGatherThreads], const double pos[3],
+                                           const DxDiv &X, const float4 *__restrict__ srec, bool apic, double &m, double &mom) {
+  const float posf[3] = {(float)pos[0], (float)pos[1], (float)pos[2]};
+  int v = -1, s = 0, e = 0;
+  bool live = has;
+  while (true) {
+    // the lane's next kGatherBatch particles of its visit sequence: their
+    // loads go out together so the L2 latencies overlap, and they are
+    // summed in sequence order
+    int at[kGatherBatch];
+    #pragma unroll
+    for (int u = 0; u < kGatherBatch; ++u) {
+      while (live && s == e) {
+        if (++v == 16) {
+          live = false;
+          break;
+        }
+        const int2 r = range[visit_bucket<D>(v)][threadIdx.x];
+        s = r.x;
+        e = r.y;
+      }
+      at[u] = live ? s++ : -1;
+    }
+    if (!__any_sync(0xffffffffu, at[0] >= 0)) break;
+    float4 pmb[kGatherBatch], ub[kGatherBatch];
+    #pragma unroll
+    for (int u = 0; u < kGatherBatch; ++u) {
+      load_record(srec + 2 * (size_t)max(at[u], 0), pmb[u], ub[u]);
+    }
+    #pragma unroll
+    for (int u = 0; u < kGatherBatch; ++u) {
+      if (at[u] < 0) continue;
+      const float4 pm = pmb[u], uv = ub[u];
+      // factors of macnbflip3::grid_kernel (macnbflip3.cpp:44-49); one that is
+      // not positive makes the weight zero
+      double o0, o1, o2, f0, f1, f2;  // particle - face, and as the reference's FP32 vector
+      if (FAR) {
+        o0 = f0 = __fsub_rn(pm.x, posf[0]);
+        o1 = f1 = __fsub_rn(pm.y, posf[1]);
+        o2 = f2 = __fsub_rn(pm.z, posf[2]);
+      } else {
+        o0 = (double)pm.x - pos[0];
+        o1 = (double)pm.y - pos[1];
+        o2 = (double)pm.z - pos[2];
+        f0 = round_fp32(o0);
+        f1 = round_fp32(o1);
+        f2 = round_fp32(o2);
+      }
+      const double t0 = 1.0 - div_dx<MODE>(fabs(f0), X);
+      const double t1 = 1.0 - div_dx<MODE>(fabs(f1), X);
+      const double t2 = 1.0 - div_dx<MODE>(fabs(f2), X);
+      const double w = t0 * t1 * t2;
+      if (t0 > 0.0 && t1 > 0.0 && t2 > 0.0 && w != 0.0) {
+        const double wm = w * (double)pm.w;
+        mom = round_fp32(mom + wm * (double)uv.x);
+        m = round_fp32(m + wm);
+        if (apic) {
+          double dot = 0.0;
+          dot += (double)uv.y * -o0;
+          dot += (double)uv.z * -o1;
+          dot += (double)uv.w * -o2;
+          mom = round_fp32(mom + wm * dot);
+        }
+      }
+    }
+  }
+}
 
 // One lane per listed face, a warp over 32 of them. A lane first loads the
 // ranges of its face's 8 distinct buckets (into shared memory, all at once),
 // then walks the 16 visits as one flat sequence of particles, so the lanes of
-// a warp stay busy until the longest sequence ends.
-template <int D, bool POW2>
-__global__ void __launch_bounds__(kGatherThreads) k_splat_gather(int nx, int ny, int nz, DxDiv X, SplatBuffers B,
-                                                                 SplatGrid G) {
-  __shared__ int2 range[8][kGatherThreads];
-  if (B.nfaces[3]) return;  // a bucket was over the limit: leave the grids as they are
+// a warp stay busy until the longest sequence ends. The lanes' records lie
+// apart, so each is a pass of its own through L1's data pipe; that bound the
+// gather at 92 % of its rate while a record was two 16-byte loads. As one of
+// 32 bytes, three of them in flight (four spill), and with the conversions of
+// the exact case gone, L1 is at 76 %, the FP64 conversions at 69 %: 256^3 tank,
+// three axes 3.1e5 faces each, 769 -> 555 us. Tiles of 8^3 faces ordered by
+// work within, for locality, took 1074 (uneven tiles).
+template <int D, int MODE>
+__device__ __forceinline__ void gather_axis(int2 (*range)[kGatherThreads], int nx, int ny, int nz, const DxDiv &X,
+                                            const SplatBuffers &B, const SplatGrid &G) {
   const int fw = nx + (D == 0), fh = ny + (D == 1);
   const int E[3] = {nx + (D != 0), ny + (D != 1), nz + (D != 2)};
   const int nact = B.nfaces[D];
   const int *__restrict__ faces = B.sorted + B.face_off[D];
-  const float4 *__restrict__ sposm = B.sposm;
-  const float4 *__restrict__ svc = B.svc;
   const bool apic = B.apic;
   const double dx = X.dx;
   const int tid = threadIdx.x;
@@ -526,6 +659,9 @@ __global__ void __launch_bounds__(kGatherThreads) k_splat_gather(int nx, int ny,
     double pos[3];
     #pragma unroll
     for (int c = 0; c < 3; ++c) pos[c] = ((double)fi[c] + (c != D ? 0.5 : 0.0)) * dx;
+    bool near = false;
+    #pragma unroll
+    for (int c = 0; c < 3; ++c) near |= pos[c] < 2.0 * dx;
     // the 8 distinct buckets (empty where out of the edge grid)
     #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -535,74 +671,40 @@ __global__ void __launch_bounds__(kGatherThreads) k_splat_gather(int nx, int ny,
       const int2 r = out ? make_int2(0, 0) : bucket_range(B, bucket_slot(B, D, E, q));
       range[k][tid] = r;
     }
-    float m = 0.0f, mom = 0.0f;
-    int v = -1, s = 0, e = 0;
-    bool live = has;
-    while (true) {
-      // the lane's next kGatherBatch particles of its visit sequence: their
-      // loads go out together so the L2 latencies overlap, and they are
-      // summed in sequence order
-      int at[kGatherBatch];
-      #pragma unroll
-      for (int u = 0; u < kGatherBatch; ++u) {
-        while (live && s == e) {
-          if (++v == 16) {
-            live = false;
-            break;
-          }
-          const int2 r = range[visit_bucket<D>(v)][tid];
-          s = r.x;
-          e = r.y;
-        }
-        at[u] = live ? s++ : -1;
-      }
-      if (!__any_sync(0xffffffffu, at[0] >= 0)) break;
-      float4 pmb[kGatherBatch], ub[kGatherBatch];
-      #pragma unroll
-      for (int u = 0; u < kGatherBatch; ++u) {
-        pmb[u] = at[u] >= 0 ? __ldg(sposm + at[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
-        ub[u] = at[u] >= 0 ? __ldg(svc + at[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      #pragma unroll
-      for (int u = 0; u < kGatherBatch; ++u) {
-        if (at[u] < 0) continue;
-        const float4 pm = pmb[u], uv = ub[u];
-        const float r0 = __double2float_rn((double)pm.x - pos[0]);
-        const float r1 = __double2float_rn((double)pm.y - pos[1]);
-        const float r2 = __double2float_rn((double)pm.z - pos[2]);
-        const double w = tent<POW2>(r0, X) * tent<POW2>(r1, X) * tent<POW2>(r2, X);
-        if (w != 0.0) {
-          const double wm = w * (double)pm.w;
-          mom = __double2float_rn((double)mom + wm * (double)uv.x);
-          m = __double2float_rn((double)m + wm);
-          if (apic) {
-            double dot = 0.0;
-            dot += (double)uv.y * (pos[0] - (double)pm.x);
-            dot += (double)uv.z * (pos[1] - (double)pm.y);
-            dot += (double)uv.w * (pos[2] - (double)pm.z);
-            mom = __double2float_rn((double)mom + wm * dot);
-          }
-        }
-      }
-    }
+    double m = 0.0, mom = 0.0;  // FP32 values
+    if (MODE == DIV_POW2 && !__any_sync(0xffffffffu, near))
+      sum_visits<D, MODE, true>(has, range, pos, X, B.srec, apic, m, mom);
+    else
+      sum_visits<D, MODE, false>(has, range, pos, X, B.srec, apic, m, mom);
     if (!has) continue;
-    const bool on = m != 0.0f;
+    const float mass = (float)m, momentum = (float)mom;
+    const bool on = mass != 0.0f;
     if (G.mass[D]) {
-      G.mass[D][f] = on ? m : 0.0f;
-      G.momentum[D][f] = on ? mom : 0.0f;
+      G.mass[D][f] = on ? mass : 0.0f;
+      G.momentum[D][f] = on ? momentum : 0.0f;
       G.splat_active[D][f] = on ? 1 : 0;
     }
     if (on && G.velocity[D]) {
       // combined grid velocity (macflipliquid3.cpp:141-150)
       float *u = G.velocity[D];
       uint8_t *ua = G.velocity_active[D];
-      const double g64 = 1.0 - (double)m;
+      const double g64 = 1.0 - m;
       const float gm = ua[f] ? __double2float_rn(0.0 < g64 ? g64 : 0.0) : 0.0f;
-      const float num = __fadd_rn(__fmul_rn(gm, u[f]), mom);
-      u[f] = __fdiv_rn(num, __fadd_rn(gm, m));
+      const float num = __fadd_rn(__fmul_rn(gm, u[f]), momentum);
+      u[f] = __fdiv_rn(num, __fadd_rn(gm, mass));
       ua[f] = 1;
     }
   }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kGatherThreads, 4) k_splat_gather(int nx, int ny, int nz, DxDiv X, SplatBuffers B,
+                                                                 SplatGrid G) {
+  __shared__ int2 range[8][kGatherThreads];
+  if (B.nfaces[3]) return;  // a bucket was over the limit: leave the grids as they are
+  if (blockIdx.y == 0) gather_axis<0, MODE>(range, nx, ny, nz, X, B, G);
+  else if (blockIdx.y == 1) gather_axis<1, MODE>(range, nx, ny, nz, X, B, G);
+  else gather_axis<2, MODE>(range, nx, ny, nz, X, B, G);
 }
 
 // The splat grid of axis D is zero and inactive wherever no particle
@@ -610,7 +712,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_splat_gather(int nx, int ny,
 // rest is cleared first (not after a refused bucket: then the call leaves
 // every grid as it was).
 template <int D>
-__global__ void k_splat_clear_grid(int nx, int ny, int nz, SplatBuffers B, SplatGrid G) {
+__device__ __forceinline__ void clear_grid_axis(int nx, int ny, int nz, SplatBuffers B, SplatGrid G) {
   if (B.nfaces[3]) return;
   const size_t nf = (size_t)(nx + (D == 0)) * (ny + (D == 1)) * (nz + (D == 2));
   for (size_t f = (size_t)blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += (size_t)gridDim.x * blockDim.x) {
@@ -620,21 +722,35 @@ __global__ void k_splat_clear_grid(int nx, int ny, int nz, SplatBuffers B, Splat
   }
 }
 
+__global__ void __launch_bounds__(256) k_splat_clear_grid(int nx, int ny, int nz, SplatBuffers B, SplatGrid G) {
+  if (blockIdx.y == 0) clear_grid_axis<0>(nx, ny, nz, B, G);
+  else if (blockIdx.y == 1) clear_grid_axis<1>(nx, ny, nz, B, G);
+  else clear_grid_axis<2>(nx, ny, nz, B, G);
+}
+
 }  // namespace
 
 static DxDiv make_dxdiv(double dx) {
   int ex = 0;
   const double mant = std::frexp(dx, &ex);
   const double inv = 1.0 / dx;
-  const bool pow2 = mant == 0.5 && std::isnormal(dx) && std::isfinite(inv) && inv * dx == 1.0;
-  return DxDiv{dx, inv, pow2 ? 1 : 0};
+  if (mant == 0.5 && std::isnormal(dx) && std::isfinite(inv) && inv * dx == 1.0 &&
+      dx > 1e-30 && dx < 1e30)
+    return DxDiv{dx, inv, DIV_POW2};  // (face positions are then FP32 values)
+  // the operands are FP32 values (0, or 2^-149 to 2^128) and their residuals
+  // 2^53 times smaller; the largest mantissa below 2 is 1 - 2^-53 in frexp's
+  if (dx > 1e-100 && dx < 1e100 && mant != 1.0 - 0x1p-53) return DxDiv{dx, inv, DIV_FMA};
+  return DxDiv{dx, inv, DIV_ANY};
 }
 
 void launch_splat_bin(const SplatRecords &R, int nx, int ny, int nz, double dx, const SplatBuffers &B,
                       cudaStream_t s) {
   if (R.count <= 0) return;
-  const unsigned blocks = (unsigned)((R.count + 255) / 256);
-  k_splat_bin<<<blocks, 256, 0, s>>>(R, nx, ny, nz, make_dxdiv(dx), B);
+  const unsigned blocks = (unsigned)((R.count + kBinThreads - 1) / kBinThreads);
+  const DxDiv X = make_dxdiv(dx);
+  if (X.mode == DIV_POW2) k_splat_bin<DIV_POW2><<<blocks, kBinThreads, 0, s>>>(R, nx, ny, nz, X, B);
+  else if (X.mode == DIV_FMA) k_splat_bin<DIV_FMA><<<blocks, kBinThreads, 0, s>>>(R, nx, ny, nz, X, B);
+  else k_splat_bin<DIV_ANY><<<blocks, kBinThreads, 0, s>>>(R, nx, ny, nz, X, B);
 }
 
 size_t scan_tile_count(long long n) { return (size_t)((n + kScanTile - 1) / kScanTile); }
@@ -666,40 +782,24 @@ void launch_splat_scatter(long long count, const SplatBuffers &B, cudaStream_t s
 
 void launch_splat_gather(int nx, int ny, int nz, double dx, const SplatBuffers &B, const SplatGrid &G,
                          cudaStream_t s) {
-  for (int d = 0; d < 3; ++d) {
-    const size_t nf = (size_t)(nx + (d == 0)) * (ny + (d == 1)) * (nz + (d == 2));
-    const unsigned blocks = (unsigned)((nf + 16 * kCompactThreads - 1) / (16 * kCompactThreads));
-    if (d == 0) k_splat_compact<0><<<blocks, kCompactThreads, 0, s>>>(nx, ny, nz, B);
-    if (d == 1) k_splat_compact<1><<<blocks, kCompactThreads, 0, s>>>(nx, ny, nz, B);
-    if (d == 2) k_splat_compact<2><<<blocks, kCompactThreads, 0, s>>>(nx, ny, nz, B);
-  }
+  size_t most = 0;
+  for (int d = 0; d < 3; ++d)
+    most = std::max(most, (size_t)(nx + (d == 0)) * (ny + (d == 1)) * (nz + (d == 2)));
+  const unsigned chunks = (unsigned)((most + 16 * kCompactThreads - 1) / (16 * kCompactThreads));
+  k_splat_compact<<<dim3(chunks, 3), kCompactThreads, 0, s>>>(nx, ny, nz, B);
   // the face lists' lengths stay on the device: a fixed grid strides over them
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const unsigned blocks = (unsigned)sms * 8;
-  k_splat_face_work<0><<<blocks, 256, 0, s>>>(nx, ny, nz, B);
-  k_splat_face_work<1><<<blocks, 256, 0, s>>>(nx, ny, nz, B);
-  k_splat_face_work<2><<<blocks, 256, 0, s>>>(nx, ny, nz, B);
+  const dim3 blocks((unsigned)sms * 8, 3);
+  k_splat_face_work<<<blocks, 256, 0, s>>>(nx, ny, nz, B);
   k_splat_work_scan<<<1, 96, 0, s>>>(B);
-  k_splat_face_sort<0><<<blocks, 256, 0, s>>>(B);
-  k_splat_face_sort<1><<<blocks, 256, 0, s>>>(B);
-  k_splat_face_sort<2><<<blocks, 256, 0, s>>>(B);
-  if (G.mass[0]) {
-    k_splat_clear_grid<0><<<blocks, 256, 0, s>>>(nx, ny, nz, B, G);
-    k_splat_clear_grid<1><<<blocks, 256, 0, s>>>(nx, ny, nz, B, G);
-    k_splat_clear_grid<2><<<blocks, 256, 0, s>>>(nx, ny, nz, B, G);
-  }
+  k_splat_face_sort<<<blocks, 256, 0, s>>>(B);
+  if (G.mass[0]) k_splat_clear_grid<<<blocks, 256, 0, s>>>(nx, ny, nz, B, G);
   const DxDiv X = make_dxdiv(dx);
-  if (X.pow2) {
-    k_splat_gather<0, true><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
-    k_splat_gather<1, true><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
-    k_splat_gather<2, true><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
-  } else {
-    k_splat_gather<0, false><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
-    k_splat_gather<1, false><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
-    k_splat_gather<2, false><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
-  }
+  if (X.mode == DIV_POW2) k_splat_gather<DIV_POW2><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
+  else if (X.mode == DIV_FMA) k_splat_gather<DIV_FMA><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
+  else k_splat_gather<DIV_ANY><<<blocks, kGatherThreads, 0, s>>>(nx, ny, nz, X, B, G);
 }
 
 }  // namespace shkz

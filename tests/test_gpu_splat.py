@@ -192,3 +192,40 @@ def test_splat_grid_alone_without_velocity(golden_splat):
         assert np.array_equal(mom[d].view(np.uint32), np.asarray(want["momentum"][d], np.float32).view(np.uint32))
     b = native.splat_args(nx, ny, nz, float(g["dx"]), P.ctypes.data, len(P), P.dtype)
     assert L.shkz_b200_splat_host(ctx.handle, ctypes.byref(b)) == -1
+
+
+@pytest.mark.parametrize("dx", [
+    2.0 ** -6, 2.0 ** -40,              # exact reciprocal, FP32 face positions
+    1.0 / 48, 0.1, 1.0 / 3, 3.0e-7,     # reciprocal with two corrections
+    float(np.nextafter(2.0, 0)) / 64,   # its exception: a mantissa of ones
+])
+@pytest.mark.parametrize("stride", [84, 96, 100])  # staged, the longest that is, read in place
+def test_splat_divisions_and_record_strides(dx, stride):
+    """Positions on and next to the planes where a particle changes bucket or
+    face, next to the axis planes and slightly outside: bit-identical to the
+    reference-pinned CPU restatement."""
+    from shiokaze_b200 import native, scenes
+    base = scenes.PARTICLE_DTYPE
+    dtype = np.dtype({"names": list(base.names), "formats": [base.fields[k][0] for k in base.names],
+                      "offsets": [base.fields[k][1] for k in base.names], "itemsize": stride})
+    nx, ny, nz = 9, 13, 17
+    rng = np.random.default_rng(17)
+    n = 6000 + 77
+    P = np.zeros(n, dtype)
+    q = rng.uniform(-0.25, 1.0, (n, 3)) * (np.array([nx, ny, nz]) + 0.25)
+    snap = rng.random((n, 3)) < 0.3
+    q[snap] = np.round(2 * q[snap]) / 2
+    p = (q * dx).astype(np.float32)
+    step = rng.integers(-1, 2, (n, 3))
+    p = np.where(step < 0, np.nextafter(p, np.float32(-9)), np.where(step > 0, np.nextafter(p, np.float32(9e9)), p))
+    P["p"] = p
+    P["velocity"] = rng.standard_normal((n, 3))
+    P["c"] = rng.standard_normal((n, 3, 3)) / dx
+    P["mass"] = rng.uniform(0.05, 0.2, n)
+    P["bullet"] = rng.random(n) < 0.05
+    vel = [rng.standard_normal((nz + (d == 2), ny + (d == 1), nx + (d == 0))).astype(np.float32) for d in range(3)]
+    act = [(rng.random(v.shape) < 0.7).astype(np.uint8) for v in vel]
+    got = native.splat(native.Context(native.default_config()), nx, ny, nz, dx, P, vel, act)
+    want = oracle.splat(nx, ny, nz, dx, P, vel, act)
+    assert_bitexact(got, dict(zip(("velocity", "velocity_active", "mass", "momentum", "splat_active"), want)))
+    assert all(int(s.sum()) > 500 for s in got[4])
