@@ -1656,7 +1656,7 @@ extern "C" int shkz_b200_solve_csr(shkz_b200_ctx *ctx, long long n, const long l
   if (ctx->cfg.spin_limit > 0) M.set_wait_limit(ctx->cfg.spin_limit);
   if (ctx->cfg.fault_skip_publish > 0) M.set_fault_skip(ctx->cfg.fault_skip_publish - 1);
   if (mic) {
-    int rc = M.build((int)n, hp.data(), hi.data(), dp, di, s);
+    int rc = M.build((int)n, nnz, hp.data(), hi.data(), dp, di, s);
     if (!rc) rc = M.factor(dd, ctx->cfg.mic_omega, ctx->cfg.mic_min_diag_ratio, s);
     if (rc) {
       cleanup();

@@ -18,9 +18,10 @@ struct CsrMicDevice {
 class CsrMic0 {
  public:
   ~CsrMic0();
-  // Pattern analysis on the host (row-sorted, symmetric pattern, 0-based);
-  // d_indptr/d_indices: the same pattern on the device (kept by the caller).
-  int build(int n, const int *indptr, const int *indices, const int *d_indptr, const int *d_indices,
+  // Pattern analysis (0-based; on the device for sorted rows and a symmetric
+  // pattern, else on the host); d_indptr/d_indices: the same pattern on the
+  // device (kept by the caller).
+  int build(int n, long long nnz, const int *indptr, const int *indices, const int *d_indptr, const int *d_indices,
             cudaStream_t s);
   // Factor the values of A (device, CSR order) with the header's parameters.
   int factor(const double *d_data, double omega, double min_ratio, cudaStream_t s);
@@ -34,16 +35,23 @@ class CsrMic0 {
   // fault injection for tests: the forward solve's row at level-order
   // position pos (-1: none) never stores its value
   void set_fault_skip(int pos) { skip_pos = pos; }
-  int levels() const { return (int)level_start.size() - 1; }
+  int levels() const { return nlev; }
 
  private:
+  static constexpr int kNotSymmetric = 1;
   void release();
+  bool allocate(long long entries);
+  int build_device(long long nnz, cudaStream_t s);
+  int build_host(const int *indptr, const int *indices, cudaStream_t s);
   CsrMicDevice device() const;
-  int n = 0, nnzl = 0, nchunks = 0, wait_limit = 1 << 22, skip_pos = -1;
-  std::vector<int> level_start;
+  int n = 0, nnzl = 0, nlev = 0, wait_limit = 1 << 22, skip_pos = -1;
+  char *arena = nullptr;  // holds all of the following
   int *d_colstart = nullptr, *d_rowindex = nullptr, *d_lrow_start = nullptr, *d_lrow_col = nullptr,
       *d_lrow_pos = nullptr, *d_src = nullptr, *d_dpos = nullptr, *d_cols = nullptr, *d_chunks = nullptr;
-  int *d_sync = nullptr;  // two chunk counters, the wait error word
+  int *d_ready = nullptr;  // levels, then the factorisation's flags
+  int *d_count = nullptr, *d_chunk = nullptr, *d_sums = nullptr;  // scratch of the analysis
+  int *d_sync = nullptr;  // two chunk counters, the wait error word, the factorisation's counter, the analysis' results
+  int *d_nchunks = nullptr;
   double *d_val = nullptr, *d_invdiag = nullptr, *d_adiag = nullptr, *d_t = nullptr;
   const int *a_ptr = nullptr, *a_idx = nullptr;
 };
