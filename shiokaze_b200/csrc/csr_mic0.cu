@@ -641,7 +641,7 @@ int CsrMic0::factor(const double *d_data, double omega, double min_ratio, cudaSt
     return SHKZ_B200_ERR_CUDA;
   count_launches(1);
   k_csrmic_factor<<<solve_blocks(), 128, 0, s>>>(device(), d_cols, d_chunks, d_nchunks, omega, min_ratio, d_ready,
-                                                 reinterpret_cast<unsigned *>(d_sync) + 3, d_sync + 2, wait_limit);
+                                                 reinterpret_cast<unsigned *>(d_sync) + 3, d_sync + 2, 1 << 22);
   return cudaGetLastError() == cudaSuccess ? 0 : SHKZ_B200_ERR_CUDA;
 }
 
