@@ -530,21 +530,24 @@ __global__ void k_pool_grad(const float *Gc, int C, int hx, int hy, int hz, cons
   }
 }
 
-// Weight gradient on the tensor cores (tcgen05, kind::f16, M = 64, N = 16,
+// Weight gradient on the tensor cores (tcgen05, kind::f16, M = 64, N = 24,
 // K = voxels): for one active block (8 x 16 x 8 voxels) and one 16-channel
 // input chunk,
 //   D_t[co][ci] = sum_v gpre[v][co] * X(v + off_t)[ci]      for the 27 taps t,
-// accumulated in TMEM (tap t in columns 16 t .. 16 t + 15) over four
-// sub-blocks of two z planes (256 voxels). Both operands are MN-major, so the
-// staged data keep their channels-last order:
+// accumulated in TMEM over the CTA's share of the block's four sub-blocks of
+// two z planes (256 voxels). An MMA takes the three x taps of one (dy, dz) and
+// 8 input channels, a row of 8-channel groups 16 bytes apart in the halo
+// (columns 24 (2 (3 dz + dy) + half) + 8 dx): an MMA's time is that of its A
+// operand, so 18 of them in place of 27 of N = 16: a block 88 -> 70 us. Both
+// operands are MN-major, so the staged data keep their channels-last order:
 //   A = gpre: 8-channel groups g of 256 voxels x 16 B, byte g * 4096 + k * 16
 //       (k = x + 8 y + 128 z); SBO = 4096 B between channel groups, LBO = 128 B
 //       between the 8-voxel groups of a K step;
 //   B = the input halo of the sub-block, (4 z) x 18 x 10 voxels x 16 B per
 //       8-channel half, the canonical layout of the forward kernel; a tap is
-//       the same layout shifted, so only the start address changes; SBO = the
-//       half's size between the channel halves, LBO = 160 B (one y row)
-//       between the 8-voxel groups of a K step.
+//       the same layout shifted, so only the start address changes; SBO = 16 B
+//       (one voxel) between the x taps, LBO = 160 B (one y row) between the
+//       8-voxel groups of a K step.
 // The next sub-block is staged (cp.async) while the tensor cores work on the
 // current one. Row co of D sits in TMEM lane (co % 16) + 32 (co / 16), so warp
 // w reads output channels 16 w .. 16 w + 15 in its first 16 lanes, adds them
@@ -552,8 +555,8 @@ __global__ void k_pool_grad(const float *Gc, int C, int hx, int hy, int hz, cons
 __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __nv_bfloat16 *gpre, int cout_pad, int cout_real,
                                                      const __nv_bfloat16 *in0, int c0, const __nv_bfloat16 *in1,
                                                      int c1, int nx, int ny, int nz, int hx, int hy, int hz,
-                                                     const uint8_t *blk, int gbx, int gby, int gbz, float *dW,
-                                                     float *db, int *err) {
+                                                     const uint8_t *blk, int gbx, int gby, int gbz, int split,
+                                                     float *dW, float *db, int *err) {
   constexpr uint32_t kG = 8 * 256 * 16;        // staged gpre of a sub-block
   constexpr uint32_t kHH = 4 * 18 * 10 * 16;   // one 8-channel half of the halo
   constexpr uint32_t kBuf = kG + 2 * kHH;      // one stage (55,808 bytes)
@@ -563,6 +566,8 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __nv_bfloat16 *gpre, 
   const int cin = c0 + c1;
   const int nchunk = cin / 16;
   int bid = blockIdx.x;
+  const int subs = 4 / split, first = bid % split * subs, last = first + subs;
+  bid /= split;
   const int chunk = bid % nchunk;
   bid /= nchunk;
   const int bxi = bid % gbx, byi = (bid / gbx) % gby, bzi = bid / (gbx * gby);
@@ -584,8 +589,8 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __nv_bfloat16 *gpre, 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  // D FP32, A/B BF16, both MN-major, N = 16, M = 64
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(16 >> 3) << 17) |
+  // D FP32, A/B BF16, both MN-major, N = 24, M = 64
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(24 >> 3) << 17) |
                          ((uint32_t)(64 >> 4) << 24);
   auto stage = [&](int sb, uint32_t buf) {
     for (int e = tid; e < 2048; e += 128) {
@@ -619,26 +624,26 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __nv_bfloat16 *gpre, 
   bool ok = true;
   float bsum = 0.0f;
   const bool bias = chunk == 0 && db != nullptr;
-  stage(0, s0);
+  stage(first, s0 + (uint32_t)(first & 1) * kBuf);
   cp_async_wait_all();
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
-  for (int sb = 0; sb < 4; ++sb) {
+  for (int sb = first; sb < last; ++sb) {
     const uint32_t buf = s0 + (uint32_t)(sb & 1) * kBuf;
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int t = 0; t < 27; ++t) {
-        const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
+      for (int t = 0; t < 18; ++t) {
+        const int half = t & 1, dy = (t >> 1) % 3, dz = t / 6;
         #pragma unroll 4
         for (int j = 0; j < 16; ++j) {
           const int y0 = (2 * j) & 15, zl = j >> 3;
           const uint64_t da = umma_desc(buf + 256u * (uint32_t)j, 128, 4096);
-          const uint64_t dbd =
-              umma_desc(buf + kG + (uint32_t)(((zl + dz) * 18 + (y0 + dy)) * 10 + dx) * 16, 160, kHH);
-          const uint32_t acc = (sb > 0 || j > 0) ? 1u : 0u;
+          const uint64_t dbd = umma_desc(
+              buf + kG + (uint32_t)half * kHH + (uint32_t)(((zl + dz) * 18 + (y0 + dy)) * 10) * 16, 160, 16);
+          const uint32_t acc = (sb > first || j > 0) ? 1u : 0u;
           asm volatile(
               "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + (uint32_t)(t * 16)),
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + (uint32_t)(t * 24)),
               "l"(da), "l"(dbd), "r"(idesc), "r"(acc)
               : "memory");
         }
@@ -648,7 +653,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __nv_bfloat16 *gpre, 
     }
     __syncwarp();
     // the next sub-block into the other stage while the tensor cores read this one
-    if (sb + 1 < 4) stage(sb + 1, s0 + (uint32_t)((sb + 1) & 1) * kBuf);
+    if (sb + 1 < last) stage(sb + 1, s0 + (uint32_t)((sb + 1) & 1) * kBuf);
     if (bias) {
       // bias gradient: thread (co, half) sums half of the sub-block's voxels
       const int co = tid & 63, half = tid >> 6;
@@ -657,7 +662,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __nv_bfloat16 *gpre, 
         for (int k = half * 128; k < half * 128 + 128; ++k) bsum += __bfloat162float(G[(co >> 3) * 2048 + k * 8 + (co & 7)]);
       }
     }
-    if (!mbar_wait(bar_s, (uint32_t)(sb & 1))) {
+    if (!mbar_wait(bar_s, (uint32_t)((sb - first) & 1))) {
       ok = false;
       break;
     }
@@ -670,13 +675,14 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __nv_bfloat16 *gpre, 
     const int co = 16 * warp + (lane & 15);
     for (int t = 0; t < 27; ++t) {
       uint32_t r[16];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * 16);
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(taddr)
-          : "memory");
+      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t / 3 * 48 + t % 3 * 8);
+      #pragma unroll
+      for (int half = 0; half < 2; ++half)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[8 * half]), "=r"(r[8 * half + 1]), "=r"(r[8 * half + 2]), "=r"(r[8 * half + 3]),
+                       "=r"(r[8 * half + 4]), "=r"(r[8 * half + 5]), "=r"(r[8 * half + 6]), "=r"(r[8 * half + 7])
+                     : "r"(taddr + 24u * half)
+                     : "memory");
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (lane < 16 && co < cout_real) {
         float *dst = dW + ((size_t)t * cout_real + co) * cin + chunk * 16;
@@ -1100,11 +1106,16 @@ static int backward(LearnedModel *m, cudaStream_t s) {
       cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       const int nb = m->gb[lv][0] * m->gb[lv][1] * m->gb[lv][2] * (cin / 16);
       count_launches(1);
-      k_wgrad_tc<<<nb, 128, smem, s>>>(m->gpre, P.n_pad, P.cout, m->T[D.in0], D.c0,
+      // A block's sub-blocks over 4 or 2 CTAs (36 and 47 us each, 70 whole)
+      // where that still is one wave, or evens out the second of two: 16
+      // blocks 78 -> 37 us, 64 71 -> 50, 256 135 -> 112; but 192, fewer of
+      // them active, 77 -> 88.
+      const int split = 4 * nb <= 148 ? 4 : 2 * nb <= 148 || (nb > 222 && nb <= 296) ? 2 : 1;
+      k_wgrad_tc<<<nb * split, 128, smem, s>>>(m->gpre, P.n_pad, P.cout, m->T[D.in0], D.c0,
                                        D.in1 >= 0 ? m->T[D.in1] : nullptr, D.c1, m->NX[lv], m->NY[lv], m->NZ[lv],
                                        lv < 2 ? m->NX[lv + 1] : 0, lv < 2 ? m->NY[lv + 1] : 0,
                                        lv < 2 ? m->NZ[lv + 1] : 0, m->blk[lv], m->gb[lv][0], m->gb[lv][1],
-                                       m->gb[lv][2], P.gw, P.gb, m->err);
+                                       m->gb[lv][2], split, P.gw, P.gb, m->err);
     }
     if (li == 0) break;  // no input gradient needed for the first layer
     // input gradient: conv of gpre with the flipped, transposed weights

@@ -200,3 +200,26 @@ def test_training_gains_over_unpreconditioned_direction():
     e_trained = _step_energy(s, r, s.learned_apply(r))
     assert e_trained < e_identity, (e_trained, e_identity)
     assert e_trained < e_untrained, (e_trained, e_untrained)
+
+
+@pytest.mark.parametrize("n", [48, 64])
+def test_weight_gradients_over_block_counts(n):
+    """Grids whose layers' blocks go to one, two and four CTAs each (the 32^3
+    one above: mostly four): weight gradients against the oracle's on the
+    activations the GPU stored, to BF16's few per cent."""
+    sc, s, _ = _projected(n=n)
+    s.learned_init(seed=4)
+    rng = np.random.default_rng(2)
+    unk = s.get_pressure().active.astype(bool)
+    s.learned_apply(np.where(unk, rng.standard_normal(unk.shape), 0).astype(np.float32))
+    X0 = s.learned_tensor("X0")
+    masks = cn.level_masks(_pool_cells(s, X0.shape[:3]))
+    gZ = rng.standard_normal(X0.shape[:3]).astype(np.float32) * masks[0]
+    got = _unpack(s.learned_backward(gZ))
+    T = {name: s.learned_tensor(name) for name in s.TENSORS[:-1]}
+    pre = {name: T[cn.OUTPUT[name]] for name, lvl, in0, in1, cout, relu in cn.LAYERS if relu}
+    want = cn.backward(_unpack(s.learned_params()), T, pre, masks, gZ)
+    for name, *_ in cn.LAYERS:
+        den = np.linalg.norm(want[name + ".w"])
+        if den > 0:
+            assert np.linalg.norm(got[name + ".w"] - want[name + ".w"]) <= 0.05 * den, name
