@@ -324,11 +324,11 @@ def run_splat(args):
     achieved = algo / (call_ms * 1e-3) / 1e9
     t0 = (ncu_traffic() or {}).get("splat_call")
     traffic = t0["dram_bytes_per_launch"] * len(P) / t0["particles"] if t0 else None
-    roofline = {"kernel": "shkz_b200_splat_device (bin, scan, bucket sort, face lists, k_splat_gather x3)",
+    roofline = {"kernel": "shkz_b200_splat_device (bin, scan, bucket sort, face lists, k_splat_gather)",
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "ms": call_ms, "algo_bytes_per_launch": algo, "traffic": traffic,
-                "note": ("not HBM-bound: the gather (about 3/5 of the call) is bound by FP64 issue and latency, "
-                         "each face summing its particles serially in the reference's order; traffic is 9.5x the "
+                "note": ("not HBM-bound: the gather (about 3/5 of the call) is bound by L1 passes and FP64 conversions, "
+                         "each face summing its particles serially in the reference's order; traffic was 9.5x the "
                          "algorithmic bytes because of the hash (packed and bucket-ordered particle copies, the "
                          "gather's L2 re-reads)")}
     # end to end through the host-buffer entry point, pinned host arrays
