@@ -374,6 +374,7 @@ __global__ void __launch_bounds__(256) k_update_xr(int n4, const float4 *__restr
                                                    float4 *__restrict__ x, float4 *__restrict__ r, double *partials,
                                                    unsigned *counter, SolverState *st, int max_iterations) {
   __shared__ double red[8];
+  wait_for_previous();
   if (st->done) return;
   const float alpha = (float)st->alpha;
   double m = 0.0, s2 = 0.0;
@@ -454,6 +455,7 @@ __global__ void k_finish_rho_r2(SolverState *st, int init) {
 // p = z + beta p (beta from st; init: p = z)
 __global__ void __launch_bounds__(256) k_update_p(int n4, const float4 *__restrict__ z, float4 *__restrict__ p,
                                                   const SolverState *st) {
+  wait_for_previous();
   if (st->done) return;
   const float beta = (float)st->beta;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
@@ -1202,6 +1204,7 @@ __global__ void __launch_bounds__(256) k_fpcg_dots(int n4, const float4 *__restr
                                                    const float4 *__restrict__ q, double *partials, unsigned *counter,
                                                    SolverState *st, int init) {
   __shared__ double red[8];
+  wait_for_previous();
   if (st->done) return;
   double a = 0.0, b = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
@@ -1322,7 +1325,7 @@ void launch_spmv(const PoolSystem &S, const float *p, float *q, double *partials
                  int mode, cudaStream_t s) {
   if (S.K <= 0) return;
   count_launches(1);
-  k_spmv<<<spmv_grid(S.K), 128, 0, s>>>(S, p, q, partials, counter, st, mode, nullptr, nullptr, nullptr);
+  launch_overlapped(k_spmv, spmv_grid(S.K), 128, 0, s, S, p, q, partials, counter, st, mode, nullptr, nullptr, nullptr);
 }
 
 void launch_spmv_update(const PoolSystem &S, float *p0, float *p1, const float *z, float *q, float *x,
@@ -1339,8 +1342,8 @@ void launch_update_xr(int n, const float *p, const float *q, float *x, float *r,
                       SolverState *st, int max_iterations, cudaStream_t s) {
   const int n4 = n / 4;
   count_launches(1);
-  k_update_xr<<<grid_for(n4, 256 * 4, 148 * 8), 256, 0, s>>>(n4, (const float4 *)p, (const float4 *)q, (float4 *)x,
-                                                               (float4 *)r, partials, counter, st, max_iterations);
+  launch_overlapped(k_update_xr, grid_for(n4, 256 * 4, 148 * 8), 256, 0, s, n4, (const float4 *)p, (const float4 *)q,
+                    (float4 *)x, (float4 *)r, partials, counter, st, max_iterations);
 }
 
 void launch_finish_rho(const double *partials, int n, SolverState *st, int init, cudaStream_t s) {
@@ -1355,7 +1358,7 @@ void launch_finish_rho_r2(SolverState *st, int init, cudaStream_t s) {
 void launch_update_p(int n, const float *z, float *p, const SolverState *st, cudaStream_t s) {
   const int n4 = n / 4;
   count_launches(1);
-  k_update_p<<<grid_for(n4, 256 * 4, 148 * 8), 256, 0, s>>>(n4, (const float4 *)z, (float4 *)p, st);
+  launch_overlapped(k_update_p, grid_for(n4, 256 * 4, 148 * 8), 256, 0, s, n4, (const float4 *)z, (float4 *)p, st);
 }
 
 void launch_mic_factor(const PoolSystem &S, double *colsum, double omega, double min_ratio, double *d64, float *d32,
@@ -1500,8 +1503,8 @@ void launch_fpcg_dots(int n, const float *z, const float *r, const float *q, dou
                       SolverState *st, int init, cudaStream_t s) {
   const int n4 = n / 4;
   count_launches(1);
-  k_fpcg_dots<<<grid_for(n4, 256 * 4, 148 * 8), 256, 0, s>>>(n4, (const float4 *)z, (const float4 *)r,
-                                                               (const float4 *)q, partials, counter, st, init);
+  launch_overlapped(k_fpcg_dots, grid_for(n4, 256 * 4, 148 * 8), 256, 0, s, n4, (const float4 *)z, (const float4 *)r,
+                    (const float4 *)q, partials, counter, st, init);
 }
 void launch_rand_unknowns(int n, const float *diag, unsigned seed, float *e, cudaStream_t s) {
   count_launches(1);

@@ -70,3 +70,32 @@ def test_pool_counts(shape, filled, block):
     assert act.any()
     assert res["unknowns"] == int(act.sum())
     assert res["tiles"] == int(pad.reshape(nz, 8, ny, 8, nx, 8).any(axis=(1, 3, 5)).sum())
+
+
+@pytest.mark.parametrize("zero", [True, False])   # breakdown of the network at once, and a stall after some iterations
+@pytest.mark.parametrize("limit", [12, 30000])
+def test_queue_depth_does_not_show_after_the_fallback(zero, limit):
+    """The learned solver's MIC(0) iterations are queued ahead, the network's
+    are not: the answer is that of one iteration at a time."""
+    from shiokaze_b200.projection import MacGrid, MacPressureSolver3
+    sc = _Scene((40, 33, 50), 0.6, 5, 16)
+    runs = []
+    for depth in (1, 2, 16):
+        s = MacPressureSolver3({"Residual": 1e-6, "B200.CheckInterval": depth})
+        s.initialize(sc.shape, sc.dx)
+        vel = lambda: MacGrid([v.copy() for v in sc.velocity], [a.copy() for a in sc.velocity_active])
+        s.project(sc.dt, vel(), None, None, sc.fluid)
+        s.learned_init(seed=3)
+        if zero:
+            s.learned_set_params(np.zeros_like(s.learned_params()))
+        s.configure({"B200.Preconditioner": "learned", "MaxIterations": limit})
+        v = vel()
+        runs.append((s.project(sc.dt, v, None, None, sc.fluid), s.get_pressure().values, v.values))
+    first, p, vel0 = runs[0]
+    assert first["fallbacks"] == 1
+    assert first["iterations"] == limit if limit == 12 else first["reresid"] <= 1e-6
+    for res, q, v in runs[1:]:
+        assert (res["iterations"], res["reresid"], res["fallbacks"]) == (first["iterations"], first["reresid"], 1)
+        np.testing.assert_array_equal(p, q)
+        for a, b in zip(vel0, v):
+            np.testing.assert_array_equal(a, b)
