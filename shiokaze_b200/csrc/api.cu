@@ -187,7 +187,9 @@ extern "C" void shkz_b200_host_free(void *p) {
 // Grid and tile-pool buffers of the context: freed and reallocated when a
 // call needs more. Their bytes are counted against cfg.device_mem_limit_mb
 // (when set), which refuses an allocation with SHKZ_B200_ERR_NOMEM before
-// cudaMalloc is asked.
+// cudaMalloc is asked. A refused buffer is left null, so whoever grows a group
+// of them sets the group's capacity to zero first: a smaller call after a
+// refused one then allocates anew instead of finding the capacity it had.
 static void release(shkz_b200_ctx *ctx, void *p) {
   if (!p) return;
   auto it = ctx->held.find(p);
@@ -243,10 +245,12 @@ static Geometry make_geometry(int nx, int ny, int nz) {
 static int ensure_grid(shkz_b200_ctx *ctx, const Geometry &G) {
   const size_t cells = (size_t)G.nx * G.ny * G.nz;
   if (cells > ctx->cap_cells) {
+    ctx->cap_cells = 0;
     GROW(unk, cells);
     ctx->cap_cells = cells;
   }
   if (G.ntiles > ctx->cap_tiles) {
+    ctx->cap_tiles = 0;
     GROW(tile_count, G.ntiles);
     GROW(tile_state, G.ntiles);
     // block sums of the tiles and, after them, of the macro tiles
@@ -267,6 +271,7 @@ static int ensure_host_staging(shkz_b200_ctx *ctx, const Geometry &G, bool solid
   const size_t cells = (size_t)G.nx * G.ny * G.nz;
   const size_t nodes = (size_t)(G.nx + 1) * (G.ny + 1) * (G.nz + 1);
   if (cells > ctx->cap_h_cells) {
+    ctx->cap_h_cells = 0;
     GROW(h_fluid, cells);
     GROW(h_fluid_active, cells);
     GROW(h_pressure, cells);
@@ -274,6 +279,7 @@ static int ensure_host_staging(shkz_b200_ctx *ctx, const Geometry &G, bool solid
     ctx->cap_h_cells = cells;
   }
   if (solid && nodes > ctx->cap_h_nodes) {
+    ctx->cap_h_nodes = 0;
     GROW(h_solid, nodes);
     GROW(h_solid_active, nodes);
     ctx->cap_h_nodes = nodes;
@@ -281,6 +287,7 @@ static int ensure_host_staging(shkz_b200_ctx *ctx, const Geometry &G, bool solid
   for (int d = 0; d < 3; ++d) {
     const size_t nf = (size_t)(G.nx + (d == 0)) * (G.ny + (d == 1)) * (G.nz + (d == 2));
     if (nf > ctx->cap_h_faces[d]) {
+      ctx->cap_h_faces[d] = 0;
       GROW(h_vel[d], nf);
       GROW(h_vact[d], nf);
       if (ctx->h_svel[d]) { release(ctx, ctx->h_svel[d]); ctx->h_svel[d] = nullptr; }
@@ -295,6 +302,7 @@ static int ensure_pool(shkz_b200_ctx *ctx, int K) {
   if (K <= ctx->cap_pool) return 0;
   int cap = K + K / 4 + 16;
   const size_t n = (size_t)cap * SHKZ_TC;
+  ctx->cap_pool = 0;
   GROW(pool_tile, cap);
   GROW(nbr, (size_t)cap * 6);
   GROW(sched, cap);
@@ -321,6 +329,7 @@ static int ensure_pool(shkz_b200_ctx *ctx, int K) {
 static int ensure_macro(shkz_b200_ctx *ctx, int KM) {
   if (KM <= ctx->cap_macro) return 0;
   const int cap = KM + KM / 4 + 16;
+  ctx->cap_macro = 0;
   GROW(mtile, cap);
   GROW(mnbr, (size_t)cap * 6);
   GROW(seg, cap);
@@ -842,12 +851,14 @@ static float ms_between(cudaEvent_t a, cudaEvent_t b) {
 // previous vector (kept across growth)
 static int ensure_warm(shkz_b200_ctx *ctx, const Geometry &G, int T, long long unknowns_bound) {
   if (ctx->cap_warm_pool < ctx->cap_pool) {
+    ctx->cap_warm_pool = 0;
     GROW(rank_pool, (size_t)ctx->cap_pool * SHKZ_TC);
     GROW(xw, (size_t)ctx->cap_pool * SHKZ_TC);
     ctx->cap_warm_pool = ctx->cap_pool;
   }
   const size_t nref = unknown_rank_scratch(G, T);
   if (nref > ctx->cap_rank_cnt) {
+    ctx->cap_rank_cnt = 0;
     GROW(rank_cnt, nref);
     ctx->cap_rank_cnt = nref;
   }
@@ -907,6 +918,7 @@ static int project_device(shkz_b200_ctx *ctx, const shkz_b200_project_args *a, s
     // velocity += surface tension force before the system is built (it reads the new velocity)
     const size_t cells = (size_t)G.nx * G.ny * G.nz;
     if (cells > ctx->cap_curv) {
+      ctx->cap_curv = 0;
       GROW(curv, cells);
       ctx->cap_curv = cells;
     }
@@ -1042,6 +1054,7 @@ extern "C" int shkz_b200_project_host(shkz_b200_ctx *ctx, const shkz_b200_projec
   const Geometry G = make_geometry(a->nx, a->ny, a->nz);
   const bool svel[3] = {a->solid_velocity[0] != nullptr, a->solid_velocity[1] != nullptr,
                         a->solid_velocity[2] != nullptr};
+  ctx->has_system = 0;  // as project_device: the previous system's buffers may be regrown
   rc = ensure_grid(ctx, G);
   if (rc) return res->status = rc;
   rc = ensure_host_staging(ctx, G, a->solid != nullptr, svel);
@@ -1065,6 +1078,7 @@ extern "C" int shkz_b200_project_host(shkz_b200_ctx *ctx, const shkz_b200_projec
       SHKZ_CUDA_TRY(cudaMemcpyAsync(ctx->h_svel[d], a->solid_velocity[d], nf[d] * 4, cudaMemcpyHostToDevice, s));
     if (a->solid_density[d]) {
       if (nf[d] > ctx->cap_h_dens[d]) {
+        ctx->cap_h_dens[d] = 0;
         GROW(h_dens[d], nf[d]);
         ctx->cap_h_dens[d] = nf[d];
       }
@@ -1164,6 +1178,7 @@ static int extend_device(shkz_b200_ctx *ctx, const shkz_b200_extend_args *a) {
     if (a->solid) {
       const size_t nodes = (size_t)(a->nx + 1) * (a->ny + 1) * (a->nz + 1);
       if (nodes > ctx->cap_ext_solid) {
+        ctx->cap_ext_solid = 0;
         GROW(ext_solid, (nodes + 31) / 32);
         ctx->cap_ext_solid = nodes;
       }
@@ -1310,6 +1325,7 @@ static int splat_device(shkz_b200_ctx *ctx, const shkz_b200_splat_args *a, const
   B.apic = a->offset_apic >= 0;
   const long long n = a->count;
   if (n > ctx->cap_sp_particles) {
+    ctx->cap_sp_particles = 0;
     GROW(sp_posm, n);
     for (int d = 0; d < 3; ++d) GROW(sp_vc[d], n);
     GROW(sp_key, 3 * n);
@@ -1321,6 +1337,7 @@ static int splat_device(shkz_b200_ctx *ctx, const shkz_b200_splat_args *a, const
   if (!ctx->sp_nfaces) GROW(sp_nfaces, 4);
   if (!ctx->sp_work) GROW(sp_work, 3 * kSplatWorkBins);
   if (B.tiles > ctx->cap_sp_tiles) {
+    ctx->cap_sp_tiles = 0;
     GROW(sp_count, 512 * B.tiles);
     GROW(sp_tile_act, B.tiles);
     GROW(sp_tile_start, B.tiles + 1);
@@ -1343,6 +1360,7 @@ static int splat_device(shkz_b200_ctx *ctx, const shkz_b200_splat_args *a, const
     listed += std::min((long long)nf[d], 8 * n);
   }
   if (listed > ctx->cap_sp_list) {
+    ctx->cap_sp_list = 0;
     GROW(sp_faces, listed);
     GROW(sp_sorted, listed);
     GROW(sp_face_bin, listed);
@@ -1350,6 +1368,7 @@ static int splat_device(shkz_b200_ctx *ctx, const shkz_b200_splat_args *a, const
   }
   for (int d = 0; d < 3; ++d) {
     if (nf[d] > ctx->cap_sp_faces[d]) {
+      ctx->cap_sp_faces[d] = 0;
       GROW(sp_act[d], nf[d]);
       ctx->cap_sp_faces[d] = nf[d];
     }
@@ -1421,6 +1440,7 @@ extern "C" int shkz_b200_splat_host(shkz_b200_ctx *ctx, const shkz_b200_splat_ar
   if (rc) return rc;
   const size_t raw = (size_t)a->count * (size_t)(a->count ? a->stride : 0);
   if (raw > ctx->cap_sp_raw) {
+    ctx->cap_sp_raw = 0;
     GROW(sp_raw, raw);
     ctx->cap_sp_raw = raw;
   }
@@ -1439,6 +1459,7 @@ extern "C" int shkz_b200_splat_host(shkz_b200_ctx *ctx, const shkz_b200_splat_ar
     }
     if (outs) {
       if (nf[d] > ctx->cap_sp_out[d]) {
+        ctx->cap_sp_out[d] = 0;
         GROW(sp_mass[d], nf[d]);
         GROW(sp_mom[d], nf[d]);
         GROW(sp_sact[d], nf[d]);
