@@ -1780,6 +1780,7 @@ extern "C" int shkz_b200_time_kernel(shkz_b200_ctx *ctx, int which, int reps, do
   init.tol_abs = -1.0;
   const int arm = arm_waves(ctx);
   if (arm) return arm;
+  init.x_pending = 1;  // as in an iteration's stencil, which clears it: set again before each
   SHKZ_CUDA_TRY(cudaMemcpyAsync(ctx->st_scratch, &init, sizeof(init), cudaMemcpyHostToDevice, s));
   auto launch = [&]() {
     switch (which) {
@@ -1836,6 +1837,8 @@ extern "C" int shkz_b200_time_kernel(shkz_b200_ctx *ctx, int which, int reps, do
   double total = 0.0;
   for (int i = 0; i < reps; ++i) {
     SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->flush, i & 0xff, flush_bytes, s));
+    if (which == 9)
+      SHKZ_CUDA_TRY(cudaMemcpyAsync(ctx->st_scratch, &init, sizeof(init), cudaMemcpyHostToDevice, s));
     cudaEventRecord(ctx->ev[4], s);
     launch();
     cudaEventRecord(ctx->ev[5], s);

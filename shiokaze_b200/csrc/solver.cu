@@ -185,8 +185,8 @@ struct SpmvSmem {
 };
 
 // zu != null: the pending updates of the previous iteration are applied on the
-// fly: x += alpha p with the old p (k_update_xr's arithmetic), then the
-// direction p <- z + beta p (k_update_p's) to the tile and its halo. The
+// fly: x += alpha p with the old p (k_update_xr's arithmetic; x null: not
+// pending), then the direction p <- z + beta p (k_update_p's) to the tile and its halo. The
 // tile's new p is written to pout (a different buffer: other CTAs still read
 // the old p for their halos). The x update costs 8 B per cell here, where the
 // old p is in registers, against 12 B in the forward sweep.
@@ -200,9 +200,11 @@ __device__ __forceinline__ void stage_tile(const PoolSystem &S, const float *__r
   xv = ld4(p + base);
   if (zu) {
     const float4 zv = ld4(zu + base);
-    float4 sol = ld4(x + base);
-    sol.x += alpha * xv.x; sol.y += alpha * xv.y; sol.z += alpha * xv.z; sol.w += alpha * xv.w;
-    st4(x + base, sol);
+    if (x) {
+      float4 sol = ld4(x + base);
+      sol.x += alpha * xv.x; sol.y += alpha * xv.y; sol.z += alpha * xv.z; sol.w += alpha * xv.w;
+      st4(x + base, sol);
+    }
     xv.x = zv.x + beta * xv.x; xv.y = zv.y + beta * xv.y; xv.z = zv.z + beta * xv.z; xv.w = zv.w + beta * xv.w;
     st4(pout + base, xv);
   }
@@ -334,8 +336,10 @@ __global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, co
   const int tid = threadIdx.x;
   const int q4 = tid & 1, jj = (tid >> 1) & 7, kk = tid >> 4;
   const float beta = zu ? (float)st->beta : 0.0f;
-  // alpha of the previous iteration, until the last block replaces it
-  const float alpha = zu && st->x_pending ? (float)st->alpha : 0.0f;
+  // alpha of the previous iteration, until the last block replaces it. Nothing
+  // is added where nothing is pending: p may hold a NaN, which 0 * p keeps.
+  if (zu && !st->x_pending) x = nullptr;
+  const float alpha = zu ? (float)st->alpha : 0.0f;
   if (zu && (st->iter & 1)) {
     float *t = const_cast<float *>(p);
     p = pout;
@@ -359,6 +363,7 @@ __global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, co
     if (tid == 0) {
       st->pq = pq;
       st->alpha = st->rho / pq;
+      if (zu) st->x_pending = 0;  // added above, also when the solve breaks down here
       if (!(pq == pq) || pq == 0.0) {
         st->done = 3;
         if (!(pq == pq)) st->status = -5;
@@ -979,11 +984,12 @@ __global__ void __launch_bounds__(256) k_accumulate_pending(int n, const float *
                                                             const float *p0, const float *p1, const SolverState *st,
                                                             double scale, double *__restrict__ x64) {
   wait_for_previous();
-  const float alpha = st->x_pending ? (float)st->alpha : 0.0f;
+  const bool pending = st->x_pending;
+  const float alpha = (float)st->alpha;
   const float *__restrict__ p = (st->iter & 1) ? p1 : p0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float x = x32[i];
-    x += alpha * p[i];
+    if (pending) x += alpha * p[i];
     x64[i] += scale * (double)x;
   }
 }

@@ -142,3 +142,28 @@ def test_zero_network_falls_back_to_mic0_and_reaches_its_answer():
     assert res1["fallbacks"] == 1, res1
     assert res1["reresid"] <= sc.tol
     assert np.abs(p1.astype(np.float64) - p0).max() / np.abs(p0).max() < 1e-4
+
+
+@pytest.mark.parametrize("block", [16, 8])
+@pytest.mark.parametrize("refine", [1, 0])
+def test_breakdown_leaves_the_last_finite_iterate(block, refine):
+    """A cell at minus infinity beside one outside the liquid gives a NaN
+    weight and a finite right-hand side, so the solve breaks down in its first
+    iteration. The call says so; the pressure it hands back is the iterate
+    before that (zero) and only the face between the two cells has no value."""
+    from shiokaze_b200.projection import Grid, MacGrid, MacPressureSolver3
+    nx, ny, nz = 40, 33, 50
+    rng = np.random.default_rng(5)
+    dx = 1.0 / nz
+    phi = np.where(rng.random((4, 3, 3)) < 0.6, -0.7, 0.7).repeat(16, 0).repeat(16, 1).repeat(16, 2)[:nz, :ny, :nx] * dx
+    k, j, i = np.argwhere((phi[:, :, :-1] < 0) & (phi[:, :, 1:] > 0))[100]
+    phi[k, j, i] = -np.inf
+    vel = [rng.standard_normal((nz + (d == 2), ny + (d == 1), nx + (d == 0))).astype(np.float32) for d in range(3)]
+    s = MacPressureSolver3({"Residual": 1e-6, "B200.MICBlock": block, "B200.Refine": refine})
+    s.initialize((nx, ny, nz), dx)
+    grid = MacGrid([v.copy() for v in vel], [np.ones(v.shape, np.uint8) for v in vel])
+    res = s.project(0.01, grid, None, None, Grid(phi.astype(np.float32), np.ones(phi.shape, np.uint8)))
+    assert res["status"] == -5 and res["iterations"] == 0
+    assert not s.get_pressure().values.any()
+    bad = [np.argwhere(np.isnan(v)) for v in grid.values]
+    assert bad[0].tolist() == [[k, j, i + 1]] and not len(bad[1]) and not len(bad[2])
