@@ -1676,6 +1676,7 @@ extern "C" int shkz_b200_solve_csr(shkz_b200_ctx *ctx, long long n, const long l
   CsrMic0 M;
   if (ctx->cfg.spin_limit > 0) M.set_wait_limit(ctx->cfg.spin_limit);
   if (ctx->cfg.fault_skip_publish > 0) M.set_fault_skip(ctx->cfg.fault_skip_publish - 1);
+  if (ctx->cfg.fault_skip_publish < 0) M.set_fault_skip_column(-1 - ctx->cfg.fault_skip_publish);
   if (mic) {
     int rc = M.build((int)n, nnz, hp.data(), hi.data(), dp, di, s);
     if (!rc) rc = M.factor(dd, ctx->cfg.mic_omega, ctx->cfg.mic_min_diag_ratio, s);
@@ -1751,7 +1752,7 @@ extern "C" int shkz_b200_solve_csr(shkz_b200_ctx *ctx, long long n, const long l
   if (cudaMemcpyAsync(x, xv, sizeof(double) * n, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     rc = SHKZ_B200_ERR_CUDA;
-  // a triangular solve's bounded wait that ran out outranks the NaN it left
+  // a bounded wait that ran out outranks the NaN it left
   if (mic && (!rc || rc == SHKZ_B200_ERR_NAN)) {
     const int we = M.wait_error(s);
     if (we) rc = we;

@@ -58,7 +58,7 @@ __device__ __forceinline__ int load_flag(const int *p) {
 __global__ void __launch_bounds__(128) k_csrmic_factor(CsrMicDevice M, const int *__restrict__ cols,
                                                        const int *__restrict__ chunks, const int *__restrict__ nchunks,
                                                        double omega, double min_ratio, int *ready, unsigned *counter,
-                                                       int *err, int limit) {
+                                                       int *err, int limit, int skip) {
   const int lane = threadIdx.x & 31, total = *nchunks;
   while (true) {
     int chunk = 0;
@@ -148,7 +148,9 @@ __global__ void __launch_bounds__(128) k_csrmic_factor(CsrMicDevice M, const int
     }
     M.invdiag[j] = inv;
     __threadfence();
-    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(ready + j), "r"(1) : "memory");
+    // fault injection (tests only): the column at level-order position skip
+    // never says that it is done, so the waits on it run out
+    if (first + lane != skip) asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(ready + j), "r"(1) : "memory");
   }
 }
 
@@ -642,7 +644,8 @@ int CsrMic0::factor(const double *d_data, double omega, double min_ratio, cudaSt
     return SHKZ_B200_ERR_CUDA;
   count_launches(1);
   k_csrmic_factor<<<solve_blocks(), 128, 0, s>>>(device(), d_cols, d_chunks, d_nchunks, omega, min_ratio, d_ready,
-                                                 reinterpret_cast<unsigned *>(d_sync) + 3, d_sync + 2, 1 << 22);
+                                                 reinterpret_cast<unsigned *>(d_sync) + 3, d_sync + 2, wait_limit,
+                                                 skip_column);
   return cudaGetLastError() == cudaSuccess ? 0 : SHKZ_B200_ERR_CUDA;
 }
 

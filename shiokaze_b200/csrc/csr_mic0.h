@@ -28,13 +28,16 @@ class CsrMic0 {
   // z = (L L^T)^-1 r (z must not alias r); every launch returns at once
   // while *done != 0
   int apply(const double *r, double *z, cudaStream_t s, const int *done = nullptr);
-  // SHKZ_B200_ERR_TIMEOUT when a triangular solve's wait ran out (since build)
+  // SHKZ_B200_ERR_TIMEOUT when a wait of the factorisation or of a triangular
+  // solve since it ran out
   int wait_error(cudaStream_t s) const;
-  // polling rounds of each wait in the triangular solves
+  // polling rounds of each wait in the factorisation and the triangular solves
   void set_wait_limit(int limit) { wait_limit = limit; }
   // fault injection for tests: the forward solve's row at level-order
   // position pos (-1: none) never stores its value
   void set_fault_skip(int pos) { skip_pos = pos; }
+  // the same for the factorisation: the column there never says it is done
+  void set_fault_skip_column(int pos) { skip_column = pos; }
   int levels() const { return nlev; }
 
  private:
@@ -44,7 +47,7 @@ class CsrMic0 {
   int build_device(long long nnz, cudaStream_t s);
   int build_host(const int *indptr, const int *indices, cudaStream_t s);
   CsrMicDevice device() const;
-  int n = 0, nnzl = 0, nlev = 0, wait_limit = 1 << 22, skip_pos = -1;
+  int n = 0, nnzl = 0, nlev = 0, wait_limit = 1 << 22, skip_pos = -1, skip_column = -1;
   char *arena = nullptr;  // holds all of the following
   int *d_colstart = nullptr, *d_rowindex = nullptr, *d_lrow_start = nullptr, *d_lrow_col = nullptr,
       *d_lrow_pos = nullptr, *d_src = nullptr, *d_dpos = nullptr, *d_cols = nullptr, *d_chunks = nullptr;

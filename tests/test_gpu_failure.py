@@ -167,3 +167,41 @@ def test_breakdown_leaves_the_last_finite_iterate(block, refine):
     assert not s.get_pressure().values.any()
     bad = [np.argwhere(np.isnan(v)) for v in grid.values]
     assert bad[0].tolist() == [[k, j, i + 1]] and not len(bad[1]) and not len(bad[2])
+
+
+def test_csr_factor_wait_timeout_returns_error_and_context_recovers():
+    """A column of the MIC(0) factorisation that never says it is done: the
+    columns that wait on it give up after the configured rounds (the default,
+    2^22, takes seconds)."""
+    import ctypes
+    import time
+    from conftest import golden_names, load_golden
+    from shiokaze_b200 import native
+    g = load_golden(golden_names()[0])
+    n = int(g["rhs"].size)
+    arrays = [np.ascontiguousarray(g[k], t) for k, t in
+              (("indptr", np.int64), ("indices", np.int64), ("data", np.float64), ("rhs", np.float64))]
+
+    def solve(ctx):
+        x = np.zeros(n, np.float64)
+        res = native.Result()
+        t0 = time.perf_counter()
+        rc = native.load().shkz_b200_solve_csr(ctx.handle, n, *[a.ctypes.data for a in arrays], x.ctypes.data,
+                                               ctypes.byref(res))
+        return rc, time.perf_counter() - t0, res.iterations, x
+
+    cfg = native.default_config()
+    cfg.residual = float(g["tol"])
+    cfg.csr_preconditioner = native.PRECOND_MIC0
+    ctx = native.Context(cfg)
+    rc0, _, it0, x0 = solve(ctx)
+    assert rc0 == 0 and it0 > 0
+    cfg.spin_limit, cfg.fault_skip_publish = 20000, -1
+    ctx.set_config(cfg)
+    rc, seconds, _, _ = solve(ctx)
+    assert rc == ERR_TIMEOUT and seconds < 1.0, (rc, seconds)
+    cfg.spin_limit, cfg.fault_skip_publish = 0, 0
+    ctx.set_config(cfg)
+    rc1, _, it1, x1 = solve(ctx)
+    assert rc1 == 0 and it1 == it0
+    assert np.array_equal(x1, x0)
