@@ -68,9 +68,12 @@ struct shkz_b200_ctx {
   unsigned *counter = nullptr;
   SolverState *st = nullptr;
   int *wflags = nullptr;  // factor wavefront flags [cap_pool]
-  unsigned long long *faces_f = nullptr, *faces_b = nullptr;  // [cap_pool][3][64] epoch-tagged sweep faces
-  // 16^3 macro tiles and pencils of the MIC(0) sweeps
-  int KM = 0, cap_macro = 0;
+  int cap_faces = 0;
+  unsigned long long *faces_f = nullptr, *faces_b = nullptr;  // [cap_faces][3][64] epoch-tagged faces of the 8^3 sweeps
+  int cap_fp64 = 0;       // tiles that xref64, p64, q64 and z64 hold
+  // 16^3 macro tiles and pencils of the MIC(0) sweeps: the system's macro
+  // tiles (0 with mic_block 8), and how many have their pencils built
+  int macro_tiles = 0, KM = 0, cap_macro = 0;
   int *mcount = nullptr, *mstate = nullptr, *mtile = nullptr, *mnbr = nullptr, *msub = nullptr, *nseg = nullptr;
   int2 *seg = nullptr, *mseg = nullptr;
   float *mfaces_f = nullptr, *mfaces_b = nullptr;  // [cap_macro][kFaceRows][32]
@@ -190,6 +193,9 @@ extern "C" void shkz_b200_host_free(void *p) {
 // cudaMalloc is asked. A refused buffer is left null, so whoever grows a group
 // of them sets the group's capacity to zero first: a smaller call after a
 // refused one then allocates anew instead of finding the capacity it had.
+// Before a refusal, the pencils of the MIC(0) sweeps (which have slower
+// stand-ins, see prepare_sweeps) give their memory back.
+static bool drop_pencils(shkz_b200_ctx *ctx);
 static void release(shkz_b200_ctx *ctx, void *p) {
   if (!p) return;
   auto it = ctx->held.find(p);
@@ -207,16 +213,19 @@ static int grow(shkz_b200_ctx *ctx, T **ptr, size_t need, const char *what) {
   if (need == 0) return 0;
   const size_t bytes = need * sizeof(T);
   const size_t cap = (size_t)(ctx->cfg.device_mem_limit_mb > 0 ? ctx->cfg.device_mem_limit_mb : 0) << 20;
-  if (cap && ctx->held_bytes + bytes > cap) {
-    std::snprintf(g_last_error, sizeof(g_last_error),
-                  "device memory cap of %d MiB reached: %zu bytes held, %zu more requested for %s",
-                  ctx->cfg.device_mem_limit_mb, ctx->held_bytes, bytes, what);
-    return SHKZ_B200_ERR_NOMEM;
-  }
-  cudaError_t e = cudaMalloc((void **)ptr, bytes);
-  if (e != cudaSuccess) {
-    shkz_set_cuda_error(e, "cudaMalloc", __FILE__, __LINE__);
+  for (;;) {
+    cudaError_t e = cudaErrorMemoryAllocation;
+    const bool capped = cap && ctx->held_bytes + bytes > cap;
+    if (!capped && (e = cudaMalloc((void **)ptr, bytes)) == cudaSuccess) break;
     *ptr = nullptr;
+    if (!capped) cudaGetLastError();  // reported here, not by the next launch
+    if (drop_pencils(ctx)) continue;
+    if (capped)
+      std::snprintf(g_last_error, sizeof(g_last_error),
+                    "device memory cap of %d MiB reached: %zu bytes held, %zu more requested for %s",
+                    ctx->cfg.device_mem_limit_mb, ctx->held_bytes, bytes, what);
+    else
+      shkz_set_cuda_error(e, "cudaMalloc", __FILE__, __LINE__);
     return SHKZ_B200_ERR_NOMEM;
   }
   ctx->held[*ptr] = bytes;
@@ -308,22 +317,56 @@ static int ensure_pool(shkz_b200_ctx *ctx, int K) {
   GROW(sched, cap);
   GROW(diag, n); GROW(offx, n); GROW(offy, n); GROW(offz, n); GROW(d32, n);
   GROW(diag64, n); GROW(offx64, n); GROW(offy64, n); GROW(offz64, n); GROW(rhs64, n);
-  GROW(colsum, n); GROW(dmic64, n); GROW(x64, n); GROW(r64, n); GROW(xref64, n);
-  GROW(p64, n); GROW(q64, n); GROW(z64, n);
+  GROW(colsum, n); GROW(dmic64, n); GROW(x64, n); GROW(r64, n);
   GROW(x, n); GROW(r, n); GROW(p, n); GROW(q, n); GROW(z, n); GROW(t, n); GROW(p32, n); GROW(pb, n);
   GROW(partials, (size_t)2 * cap + 4 * 8192);
   GROW(wflags, (size_t)cap);
-  GROW(faces_f, (size_t)cap * 3 * 64);
-  GROW(faces_b, (size_t)cap * 3 * 64);
   SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->wflags, 0, sizeof(int) * (size_t)cap, ctx->stream));
-  SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->faces_f, 0, sizeof(unsigned long long) * (size_t)cap * 3 * 64, ctx->stream));
-  SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->faces_b, 0, sizeof(unsigned long long) * (size_t)cap * 3 * 64, ctx->stream));
   if (ctx->ws) {
-    // flags were reset: restart the epochs
+    // flags were reset: restart the epochs, which face tags must not outlive
     SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->ws, 0, 3 * wave_sync_bytes(), ctx->stream));
+    ctx->cap_faces = 0;
   }
   ctx->cap_pool = cap;
   return 0;
+}
+
+// the FP64 reference solve's own vectors
+static int ensure_fp64(shkz_b200_ctx *ctx) {
+  if (ctx->cap_pool <= ctx->cap_fp64) return 0;
+  const size_t n = (size_t)ctx->cap_pool * SHKZ_TC;
+  ctx->cap_fp64 = 0;
+  GROW(xref64, n); GROW(p64, n); GROW(q64, n); GROW(z64, n);
+  ctx->cap_fp64 = ctx->cap_pool;
+  return 0;
+}
+
+// faces of the sweeps on 8^3 tiles; tag 0 is no epoch's
+static int ensure_faces(shkz_b200_ctx *ctx) {
+  if (ctx->cap_pool <= ctx->cap_faces) return 0;
+  const size_t n = (size_t)ctx->cap_pool * 3 * 64;
+  ctx->cap_faces = 0;
+  GROW(faces_f, n);
+  GROW(faces_b, n);
+  SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->faces_f, 0, sizeof(unsigned long long) * n, ctx->stream));
+  SHKZ_CUDA_TRY(cudaMemsetAsync(ctx->faces_b, 0, sizeof(unsigned long long) * n, ctx->stream));
+  ctx->cap_faces = ctx->cap_pool;
+  return 0;
+}
+
+static void release_pencils(shkz_b200_ctx *ctx) {
+  ctx->cap_macro = ctx->KM = 0;
+  auto give = [&](auto *&p) {
+    release(ctx, p);
+    p = nullptr;
+  };
+  give(ctx->mtile); give(ctx->mnbr); give(ctx->seg); give(ctx->mseg); give(ctx->nseg); give(ctx->msub);
+  give(ctx->mfaces_f); give(ctx->mfaces_b); give(ctx->coef_f); give(ctx->coef_b); give(ctx->tp);
+}
+static bool drop_pencils(shkz_b200_ctx *ctx) {
+  if (!ctx->cap_macro) return false;
+  release_pencils(ctx);
+  return true;
 }
 
 static int ensure_macro(shkz_b200_ctx *ctx, int KM) {
@@ -380,7 +423,7 @@ static unsigned next_mail(shkz_b200_ctx *ctx) {
 
 // Tiles and macro tiles that hold unknowns, and the unknowns: counted by four
 // small kernels and read by the host in one go.
-static int count_pool(shkz_b200_ctx *ctx, const Geometry &G, int *K, int *KM, long long *unknowns) {
+static int count_pool(shkz_b200_ctx *ctx, const Geometry &G, int *K, int *macro_tiles, long long *unknowns) {
   cudaStream_t s = ctx->stream;
   const bool macro = ctx->cfg.mic_block != 8;
   const unsigned seq = next_mail(ctx);
@@ -394,16 +437,17 @@ static int count_pool(shkz_b200_ctx *ctx, const Geometry &G, int *K, int *KM, lo
   const int rc = wait_mail(ctx, seq);
   if (rc) return rc;
   *K = ctx->mail->tiles;
-  *KM = macro ? ctx->mail->macro_tiles : 0;
+  *macro_tiles = macro ? ctx->mail->macro_tiles : 0;
   *unknowns = ctx->mail->unknowns;
   return 0;
 }
 
 static int build_macro_tiles(shkz_b200_ctx *ctx, const Geometry &G, int KM, cudaStream_t s) {
-  ctx->KM = 0;
-  if (KM <= 0) return 0;
   const int rc = ensure_macro(ctx, KM);
-  if (rc) return rc;
+  if (rc) {
+    release_pencils(ctx);
+    return rc;
+  }
   build_macro(G, macro_geometry(G), ctx->tile_count, ctx->tile_state, ctx->mcount, ctx->mstate, ctx->mtile, ctx->mnbr,
               ctx->level_count, ctx->seg, ctx->mseg, ctx->nseg, ctx->msub, KM, macro_bsum(ctx, G), s);
   SHKZ_CUDA_TRY(cudaGetLastError());
@@ -546,6 +590,35 @@ static int arm_waves(shkz_b200_ctx *ctx) {
                    ctx->cfg.fault_skip_publish > 0 ? ctx->cfg.fault_skip_publish : 0, ctx->mfaces_f, ctx->mfaces_b,
                    faces, ctx->stream);
   SHKZ_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
+// Buffers and structures for the MIC(0) sweeps of the current system, and the
+// waves armed; before any of them. Sweeps run on pencils, whose coefficients in
+// sweep order and other arrays take 154 KB a 16^3 macro tile, where one of its
+// 8^3 tiles takes 64 in the pool: a dense pool (eight a macro tile) holds 1.3
+// times as much with them, one with a tile in each 3.4 times. Where they are not
+// to be had, the sweeps on 8^3 tiles give the same z in 3 KB a tile (256^3 tank:
+// 618 us a pair for 254).
+static int prepare_sweeps(shkz_b200_ctx *ctx) {
+  if (ctx->K > 0 && ctx->cfg.mic_block != 8 && ctx->macro_tiles > 0 && !ctx->KM) {
+    const int rc = build_macro_tiles(ctx, ctx->G, ctx->macro_tiles, ctx->stream);
+    if (rc && rc != SHKZ_B200_ERR_NOMEM) return rc;
+    if (!rc && ctx->mic_ready) launch_pencil_coefs(pool_system(ctx), ctx->d32, ctx->stream);
+  }
+  if (ctx->K > 0 && !pool_system(ctx).KM)
+    if (const int rc = ensure_faces(ctx)) return rc;
+  return arm_waves(ctx);
+}
+
+// the same, and the factor if the projection did not need one
+static int prepare_mic(shkz_b200_ctx *ctx) {
+  if (const int rc = prepare_sweeps(ctx)) return rc;
+  if (ctx->K <= 0 || ctx->mic_ready) return 0;
+  launch_mic_factor(pool_system(ctx), ctx->colsum, ctx->cfg.mic_omega, ctx->cfg.mic_min_diag_ratio, ctx->dmic64,
+                    ctx->d32, ctx->wflags, wsync(ctx, 0), ctx->stream);
+  SHKZ_CUDA_TRY(cudaGetLastError());
+  ctx->mic_ready = 1;
   return 0;
 }
 
@@ -927,19 +1000,17 @@ static int project_device(shkz_b200_ctx *ctx, const shkz_b200_project_args *a, s
     launch_surface_tension(in, ctx->flags, ctx->curv, a->surface_tension, vel, vact, s);
   }
   // pool size (one small host read), then the pool itself
-  int K = 0, KM = 0;
+  int K = 0;
   long long unknowns = 0;
-  rc = count_pool(ctx, G, &K, &KM, &unknowns);
+  ctx->KM = 0;
+  rc = count_pool(ctx, G, &K, &ctx->macro_tiles, &unknowns);
   if (rc) return rc;
   rc = ensure_pool(ctx, K > 0 ? K : 1);
+  if (!rc && ctx->cfg.fp64_reference) rc = ensure_fp64(ctx);
   if (rc) return rc;
   pool_assign(G, ctx->tile_count, K, ctx->bsum, ctx->tile_state, ctx->pool_tile, ctx->nbr, ctx->level_count,
               ctx->sched, s);
   SHKZ_CUDA_TRY(cudaGetLastError());
-  rc = build_macro_tiles(ctx, G, KM, s);
-  if (rc) return rc;
-  rc = arm_waves(ctx);
-  if (rc) return rc;
   cudaEventRecord(ctx->ev[9], s);
   ctx->K = K;
   ctx->G = G;
@@ -975,13 +1046,11 @@ static int project_device(shkz_b200_ctx *ctx, const shkz_b200_project_args *a, s
                                   cudaMemcpyDeviceToDevice, s));
   }
   const int precond = ctx->cfg.preconditioner;
-  const PoolSystem S = pool_system(ctx);
   ctx->mic_ready = 0;
-  if (K > 0 && (precond == SHKZ_B200_PRECOND_MIC0 || precond == SHKZ_B200_PRECOND_LEARNED)) {
-    launch_mic_factor(S, ctx->colsum, ctx->cfg.mic_omega, ctx->cfg.mic_min_diag_ratio, ctx->dmic64, ctx->d32,
-                      ctx->wflags, wsync(ctx, 0), s);
-    ctx->mic_ready = 1;
-  }
+  // (the FP64 reference solve's preconditioner is MIC(0) as well)
+  const bool mic = precond == SHKZ_B200_PRECOND_MIC0 || precond == SHKZ_B200_PRECOND_LEARNED || ctx->cfg.fp64_reference;
+  rc = mic ? prepare_mic(ctx) : arm_waves(ctx);
+  if (rc) return rc;
   SHKZ_CUDA_TRY(cudaGetLastError());
   cudaEventRecord(ctx->ev[1], s);
   ctx->has_system = 1;
@@ -1534,6 +1603,11 @@ extern "C" int shkz_b200_inspect(shkz_b200_ctx *ctx, int what, void *host_out, s
   SHKZ_CUDA_TRY(cudaMalloc(&dense, cells * (f64 ? 8 : 4)));
   const float *src32 = nullptr;
   const double *src64 = nullptr;
+  if (what == 7 && ctx->K > ctx->cap_fp64) {  // no reference solve has run on a system of this size
+    cudaFree(dense);
+    std::memset(host_out, 0, cells * 8);
+    return 0;
+  }
   switch (what) {
     case 0: src32 = ctx->diag; break;
     case 1: src32 = ctx->offx; break;
@@ -1567,7 +1641,9 @@ static int dense_roundtrip(shkz_b200_ctx *ctx, const float *in_cells, float *out
   const size_t cells = (size_t)G.nx * G.ny * G.nz;
   const int n = ctx->K * SHKZ_TC;
   float *dense = nullptr;
-  int rc = arm_waves(ctx);
+  const bool mic = op == 1 && (ctx->cfg.preconditioner == SHKZ_B200_PRECOND_MIC0 ||
+                               ctx->cfg.preconditioner == SHKZ_B200_PRECOND_LEARNED);
+  int rc = mic ? prepare_mic(ctx) : arm_waves(ctx);
   if (rc) return rc;
   SHKZ_CUDA_TRY(cudaMalloc(&dense, cells * 4));
   cudaMemcpyAsync(dense, in_cells, cells * 4, cudaMemcpyHostToDevice, s);
@@ -1577,7 +1653,7 @@ static int dense_roundtrip(shkz_b200_ctx *ctx, const float *in_cells, float *out
     const PoolSystem S = pool_system(ctx);
     if (op == 0) {
       launch_spmv(S, ctx->r, ctx->z, ctx->partials, ctx->counter, nullptr, 1, s);
-    } else if (ctx->cfg.preconditioner == SHKZ_B200_PRECOND_MIC0 || ctx->cfg.preconditioner == SHKZ_B200_PRECOND_LEARNED) {
+    } else if (mic) {
       launch_mic_apply(S, ctx->d32, ctx->r, ctx->t, ctx->z, nullptr, ctx->faces_f,
                        ctx->faces_b, wsync(ctx, 1), wsync(ctx, 2), nullptr, s);
     } else {
@@ -1772,6 +1848,9 @@ extern "C" int shkz_b200_time_kernel(shkz_b200_ctx *ctx, int which, int reps, do
   if (!ctx->has_system) return SHKZ_B200_ERR_STATE;
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
+  const bool mic = which == 1 || which == 2 || which == 7 || which == 10;
+  const int arm = mic ? prepare_mic(ctx) : arm_waves(ctx);
+  if (arm) return arm;
   const PoolSystem S = pool_system(ctx);
   const int n = ctx->K * SHKZ_TC;
   SolverState init{};
@@ -1779,8 +1858,6 @@ extern "C" int shkz_b200_time_kernel(shkz_b200_ctx *ctx, int which, int reps, do
   init.alpha = 1e-30;  // keeps x and r unchanged to rounding while timing the update
   init.beta = 0.0;
   init.tol_abs = -1.0;
-  const int arm = arm_waves(ctx);
-  if (arm) return arm;
   init.x_pending = 1;  // as in an iteration's stencil, which clears it: set again before each
   SHKZ_CUDA_TRY(cudaMemcpyAsync(ctx->st_scratch, &init, sizeof(init), cudaMemcpyHostToDevice, s));
   auto launch = [&]() {
@@ -2208,14 +2285,10 @@ extern "C" int shkz_b200_learned_train(shkz_b200_ctx *ctx, int steps, double lr,
   if (rc) return rc;
   if (ctx->K == 0) return 0;
   cudaStream_t s = ctx->stream;
+  if ((rc = prepare_mic(ctx))) return rc;
   const PoolSystem S = pool_system(ctx);
   const LearnedSystem LS = learned_system(ctx);
   const int n = ctx->K * SHKZ_TC;
-  if (!ctx->mic_ready) {
-    launch_mic_factor(S, ctx->colsum, ctx->cfg.mic_omega, ctx->cfg.mic_min_diag_ratio, ctx->dmic64, ctx->d32,
-                      ctx->wflags, wsync(ctx, 0), s);
-    ctx->mic_ready = 1;
-  }
   const int np = mic_partial_count(S);
   std::vector<double> hp((size_t)np);
   for (int i = 0; i < steps; ++i) {
