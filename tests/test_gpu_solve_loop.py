@@ -99,3 +99,53 @@ def test_queue_depth_does_not_show_after_the_fallback(zero, limit):
         np.testing.assert_array_equal(p, q)
         for a, b in zip(vel0, v):
             np.testing.assert_array_equal(a, b)
+
+
+_BLOCKING = r"""
+import ctypes, sys, time
+cu = ctypes.CDLL("libcuda.so.1")
+dev = ctypes.c_int()
+assert cu.cuInit(0) == 0 and cu.cuDeviceGet(ctypes.byref(dev), 0) == 0
+assert cu.cuDevicePrimaryCtxSetFlags_v2(dev, 4) == 0  # CU_CTX_SCHED_BLOCKING_SYNC
+import torch
+from shiokaze_b200 import native
+n = 192
+T = lambda shape, fill, dtype=torch.float32: torch.full(shape, fill, dtype=dtype, device="cuda")
+g = torch.Generator(device="cuda").manual_seed(3)
+phi, phia = T((n, n, n), -0.7 / n), T((n, n, n), 1, torch.uint8)
+vel = [torch.randn((n + (d == 2), n + (d == 1), n + (d == 0)), device="cuda", generator=g) for d in range(3)]
+act = [T(tuple(v.shape), 1, torch.uint8) for v in vel]
+phi[n // 2:] = 0.7 / n
+cfg = native.default_config()
+cfg.residual = 1e-9
+ctx = native.Context(cfg)
+a = native.ProjectArgs()
+a.nx = a.ny = a.nz = n
+a.dx, a.dt, a.fluid, a.fluid_active = 1.0 / n, 0.01, phi.data_ptr(), phia.data_ptr()
+torch.cuda.synchronize()
+for _ in range(4):
+    work = [v.clone() for v in vel]
+    for d in range(3):
+        a.velocity[d], a.velocity_active[d] = work[d].data_ptr(), act[d].data_ptr()
+    torch.cuda.synchronize()
+    res = native.Result()
+    t, c = time.perf_counter(), time.thread_time()
+    assert native.load().shkz_b200_project_device(ctx.handle, ctypes.byref(a), ctypes.byref(res)) == 0
+    wall, cpu = time.perf_counter() - t, time.thread_time() - c
+    assert res.ms_solve > 5
+print(cpu / wall)
+"""
+
+
+def test_waits_sleep_under_blocking_synchronisation():
+    """An application that has asked for cudaDeviceScheduleBlockingSync gets its
+    core back while the solve runs: launches and looks are a small part of an
+    iteration's 0.1 ms and more here, so well under half of the call is CPU time."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", _BLOCKING], cwd=root, env=dict(os.environ, PYTHONPATH=root),
+                         capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
+    assert float(out.stdout.split()[-1]) < 0.5, out.stdout
