@@ -105,6 +105,9 @@ __device__ __forceinline__ double block_max(double v, double *smem) {
 // last one: a 64^3 dam break 2.41 -> 2.16 ms a projection, a 256^3 tank 65.8 ->
 // 64.4. (With an explicit launch_dependents at the top of the iteration's
 // kernels, 2.20 and 69: early blocks of the sweeps are in the stencil's way.)
+// Such a kernel's pointer parameters are not __restrict__: the promise would
+// cover the time before wait_for_previous returns, when the previous kernel is
+// still writing what they point to, and let loads be moved above it.
 template <class... P, class... A>
 inline void launch_overlapped(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A &&...args) {
   cudaLaunchConfig_t c = {};

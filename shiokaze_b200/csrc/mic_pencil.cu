@@ -776,8 +776,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_pencil_forward(PoolSystem S, co
 
 // Backward sweep with the fused z.r (r: the residual the forward sweep used);
 // with finish the last CTA also turns the partials into rho and beta.
-__global__ void __launch_bounds__(NTHREADS, 1) k_pencil_backward(PoolSystem S, const float *__restrict__ r,
-                                                                 float *__restrict__ z, double *partials, WaveSync *ws,
+__global__ void __launch_bounds__(NTHREADS, 1) k_pencil_backward(PoolSystem S, const float *r, float *z,
+                                                                 double *partials, WaveSync *ws,
                                                                  SolverState *st, unsigned *finish) {
   extern __shared__ __align__(128) unsigned char raw[];
   Smem &sm = *reinterpret_cast<Smem *>(raw);

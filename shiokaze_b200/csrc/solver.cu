@@ -324,10 +324,9 @@ __device__ __forceinline__ float4 stencil4(const SpmvSmem &sm, float4 xv, const 
 // holding the current direction is chosen by the parity of the completed
 // iteration count on the device, so launches that the loop control retires
 // (done != 0) do not flip it.
-__global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, const float *p, float *__restrict__ q,
+__global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, const float *p, float *q,
                                               double *partials, unsigned *counter, SolverState *st, int mode,
-                                              const float *__restrict__ zu, float *pout,
-                                              float *__restrict__ x) {
+                                              const float *zu, float *pout, float *x) {
   __shared__ SpmvSmem sm;
   __shared__ double red[4];
   wait_for_previous();
@@ -375,9 +374,8 @@ __global__ void __launch_bounds__(128, SPMV_CTAS_PER_SM) k_spmv(PoolSystem S, co
 }
 
 // x += alpha p; r -= alpha q; ||r||inf, ||r||2^2 -> st; convergence check.
-__global__ void __launch_bounds__(256) k_update_xr(int n4, const float4 *__restrict__ p, const float4 *__restrict__ q,
-                                                   float4 *__restrict__ x, float4 *__restrict__ r, double *partials,
-                                                   unsigned *counter, SolverState *st, int max_iterations) {
+__global__ void __launch_bounds__(256) k_update_xr(int n4, const float4 *p, const float4 *q, float4 *x, float4 *r,
+                                                   double *partials, unsigned *counter, SolverState *st, int max_iterations) {
   __shared__ double red[8];
   wait_for_previous();
   if (st->done) return;
@@ -458,7 +456,7 @@ __global__ void k_finish_rho_r2(SolverState *st, int init) {
 }
 
 // p = z + beta p (beta from st; init: p = z)
-__global__ void __launch_bounds__(256) k_update_p(int n4, const float4 *__restrict__ z, float4 *__restrict__ p,
+__global__ void __launch_bounds__(256) k_update_p(int n4, const float4 *z, float4 *p,
                                                   const SolverState *st) {
   wait_for_previous();
   if (st->done) return;
@@ -850,8 +848,8 @@ __global__ void k_macro_sub(Geometry G, Geometry M, const int *macro_tile, int K
 // cells) 100 us, 512^3 rain 291 us; 194 and 586 us with a thread per cell that
 // looked each neighbour up in global memory.
 #define RESIDUAL_CTAS_PER_SM 4  // 126 registers; at 5 and 6 a SM the values spill: 101 and 129 us
-__global__ void __launch_bounds__(128, RESIDUAL_CTAS_PER_SM) k_residual64(PoolSystem S, const double *__restrict__ b,
-                                                    const double *__restrict__ x, double *__restrict__ r,
+__global__ void __launch_bounds__(128, RESIDUAL_CTAS_PER_SM) k_residual64(PoolSystem S, const double *b,
+                                                    const double *x, double *r,
                                                     double *partials, unsigned *counter, MailSlot slot) {
   __shared__ double red[8];
   __shared__ __align__(16) double xs[10][10][12];  // (kk+1, jj+1, ii+2); halos at kk/jj 0,9 and ii 1,10
@@ -955,8 +953,8 @@ __global__ void __launch_bounds__(128, RESIDUAL_CTAS_PER_SM) k_residual64(PoolSy
 
 // Start of an inner FP32 solve on r32 = r64 * inv_scale; x32 = 0. With st the
 // loop that stopped is resumed.
-__global__ void __launch_bounds__(256) k_inner_init(int n, const double *__restrict__ r64, double inv_scale,
-                                                    float *__restrict__ r32, float *__restrict__ x32,
+__global__ void __launch_bounds__(256) k_inner_init(int n, const double *r64, double inv_scale,
+                                                    float *r32, float *x32,
                                                     SolverState *st, double ru_threshold) {
   wait_for_previous();
   if (st && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -980,13 +978,13 @@ __global__ void __launch_bounds__(256) k_accumulate(int n, const float *__restri
 // The same with the last iteration's x update, which the fused iteration
 // leaves to its next stencil: x64 += scale * (x32 + alpha p). p0 holds the
 // direction after an even number of completed iterations, p1 after an odd one.
-__global__ void __launch_bounds__(256) k_accumulate_pending(int n, const float *__restrict__ x32,
+__global__ void __launch_bounds__(256) k_accumulate_pending(int n, const float *x32,
                                                             const float *p0, const float *p1, const SolverState *st,
-                                                            double scale, double *__restrict__ x64) {
+                                                            double scale, double *x64) {
   wait_for_previous();
   const bool pending = st->x_pending;
   const float alpha = (float)st->alpha;
-  const float *__restrict__ p = (st->iter & 1) ? p1 : p0;
+  const float *p = (st->iter & 1) ? p1 : p0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float x = x32[i];
     if (pending) x += alpha * p[i];
@@ -999,7 +997,7 @@ __global__ void __launch_bounds__(256) k_to_float(int n, const double *__restric
 }
 
 // rmax0 and the absolute tolerance of an inner solve from r32 (= its rhs).
-__global__ void __launch_bounds__(256) k_inner_setup(int n, const float *__restrict__ r, double *partials,
+__global__ void __launch_bounds__(256) k_inner_setup(int n, const float *r, double *partials,
                                                      unsigned *counter, SolverState *st, double tol,
                                                      double ru_threshold) {
   __shared__ double red[8];
@@ -1206,8 +1204,8 @@ __global__ void __launch_bounds__(256) k_scale_f32_f64(int n, const float *__res
 
 // z.r and z.q (FP64); init: rho = z.r, beta = 0; else Polak-Ribiere
 // beta = z.(r_new - r_old)/rho = -alpha z.q / rho (r_old = r_new + alpha q).
-__global__ void __launch_bounds__(256) k_fpcg_dots(int n4, const float4 *__restrict__ z, const float4 *__restrict__ r,
-                                                   const float4 *__restrict__ q, double *partials, unsigned *counter,
+__global__ void __launch_bounds__(256) k_fpcg_dots(int n4, const float4 *z, const float4 *r,
+                                                   const float4 *q, double *partials, unsigned *counter,
                                                    SolverState *st, int init) {
   __shared__ double red[8];
   wait_for_previous();
