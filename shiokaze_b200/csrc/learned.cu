@@ -809,6 +809,7 @@ struct LearnedModel {
   int *err = nullptr;
   double *partials = nullptr;
   size_t params_total = 0;
+  int sms = 148;
   long long nactive[3] = {0, 0, 0};  // active 8x16x8 blocks per level (last prepare)
 };
 
@@ -858,6 +859,7 @@ static int repack(LearnedModel *m, int li, cudaStream_t s) {
 LearnedModel *learned_create(int device) {
   LearnedModel *m = new LearnedModel();
   m->device = device;
+  cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
   bool ok = cudaMalloc(&m->err, sizeof(int)) == cudaSuccess &&
             cudaMalloc(&m->partials, sizeof(double) * 8192) == cudaSuccess;
   size_t total = 0;
@@ -1075,6 +1077,27 @@ static int forward(LearnedModel *m, cudaStream_t s) {
 }
 
 // Backward of sum(gZ * Z): weight/bias gradients into L[].gw/gb (zeroed first).
+// How many CTAs share a block's four sub-blocks: whichever of 1, 2 and 4 takes
+// the fewest waves times the time of one, with one CTA an SM and `work` (block,
+// chunk) pairs that do anything (the CTAs of inactive blocks return at once).
+// A CTA takes 70 us with all four sub-blocks, 42 with two, 29 with one (32 to 64
+// input channels; what does not shrink is TMEM, staging and the atomics).
+// Measured with 1 / 2 / 4, work 16: 78 / 50 / 38 us; 72: 76 / 66 / 82; 114:
+// 76 / 83 / 90; 160: 135 / 117 / 131; 228: 148 / 164 / 187; 342: 199 / 189 /
+// 226; 646: 331 / 339 / 417.
+static int wgrad_split(long long work, int sms) {
+  int best = 1;
+  long long least = 0;
+  for (int split = 1; split <= 4; split *= 2) {
+    const long long us = (work * split + sms - 1) / sms * (split == 1 ? 70 : split == 2 ? 42 : 29);
+    if (split == 1 || us < least) {
+      best = split;
+      least = us;
+    }
+  }
+  return best;
+}
+
 static int backward(LearnedModel *m, cudaStream_t s) {
   for (int li = 0; li < 11; ++li) {
     cudaMemsetAsync(m->L[li].gw, 0, m->L[li].nw * 4, s);
@@ -1106,11 +1129,7 @@ static int backward(LearnedModel *m, cudaStream_t s) {
       cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       const int nb = m->gb[lv][0] * m->gb[lv][1] * m->gb[lv][2] * (cin / 16);
       count_launches(1);
-      // A block's sub-blocks over 4 or 2 CTAs (36 and 47 us each, 70 whole)
-      // where that still is one wave, or evens out the second of two: 16
-      // blocks 78 -> 37 us, 64 71 -> 50, 256 135 -> 112; but 192, fewer of
-      // them active, 77 -> 88.
-      const int split = 4 * nb <= 148 ? 4 : 2 * nb <= 148 || (nb > 222 && nb <= 296) ? 2 : 1;
+      const int split = wgrad_split(m->nactive[lv] * (cin / 16), m->sms);
       k_wgrad_tc<<<nb * split, 128, smem, s>>>(m->gpre, P.n_pad, P.cout, m->T[D.in0], D.c0,
                                        D.in1 >= 0 ? m->T[D.in1] : nullptr, D.c1, m->NX[lv], m->NY[lv], m->NZ[lv],
                                        lv < 2 ? m->NX[lv + 1] : 0, lv < 2 ? m->NY[lv + 1] : 0,
