@@ -91,6 +91,7 @@ struct SplatRecords {
   long long count;
   int stride, off_p, off_v, off_m, off_c, off_bullet;  // off_c / off_bullet < 0: absent
   int splat_bullet;
+  int used;  // bytes of a record up to the end of its last field (set by launch_splat_bin)
 };
 struct SplatBuffers {
   float4 *posm;            // per particle: p, mass

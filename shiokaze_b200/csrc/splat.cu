@@ -121,12 +121,15 @@ template <int MODE>
 __global__ void __launch_bounds__(kBinThreads) k_splat_bin(SplatRecords R, int nx, int ny, int nz, DxDiv X, SplatBuffers B) {
   // Records up to kStageStride bytes come through shared memory: read in place,
   // each of a record's 17 words is a line of its own for every lane of a warp
-  // (1.6 M particles: 143 -> 129 us, most of it the bucket counters' atomics)
+  // (1.6 M particles: 143 -> 129 us, most of it the bucket counters' atomics).
+  // Nothing past the last record's last field is read: the caller's array may
+  // start inside its first record and so end before the last one's stride.
   __shared__ unsigned stage[kBinThreads * kStageStride / 4];
   const long long n0 = (long long)blockIdx.x * kBinThreads, n = n0 + threadIdx.x;
   const bool staged = R.stride <= kStageStride && (R.stride & 3) == 0;
   if (staged) {
-    const int words = (int)min((long long)kBinThreads, R.count - n0) * (R.stride >> 2);
+    const int records = (int)min((long long)kBinThreads, R.count - n0);
+    const int words = ((records - 1) * R.stride + R.used + 3) >> 2;
     const unsigned *src = reinterpret_cast<const unsigned *>(R.base + (size_t)n0 * R.stride);
     for (int w = threadIdx.x; w < words; w += kBinThreads) stage[w] = __ldg(src + w);
     __syncthreads();
@@ -743,9 +746,11 @@ static DxDiv make_dxdiv(double dx) {
   return DxDiv{dx, inv, DIV_ANY};
 }
 
-void launch_splat_bin(const SplatRecords &R, int nx, int ny, int nz, double dx, const SplatBuffers &B,
+void launch_splat_bin(const SplatRecords &records, int nx, int ny, int nz, double dx, const SplatBuffers &B,
                       cudaStream_t s) {
-  if (R.count <= 0) return;
+  if (records.count <= 0) return;
+  SplatRecords R = records;
+  R.used = std::max({R.off_p + 12, R.off_v + 12, R.off_m + 4, R.off_c >= 0 ? R.off_c + 36 : 0, R.off_bullet + 1});
   const unsigned blocks = (unsigned)((R.count + kBinThreads - 1) / kBinThreads);
   const DxDiv X = make_dxdiv(dx);
   if (X.mode == DIV_POW2) k_splat_bin<DIV_POW2><<<blocks, kBinThreads, 0, s>>>(R, nx, ny, nz, X, B);

@@ -229,3 +229,47 @@ def test_splat_divisions_and_record_strides(dx, stride):
     want = oracle.splat(nx, ny, nz, dx, P, vel, act)
     assert_bitexact(got, dict(zip(("velocity", "velocity_active", "mass", "momentum", "splat_active"), want)))
     assert all(int(s.sum()) > 500 for s in got[4])
+
+
+@pytest.mark.parametrize("count", [1, 128, 129, 1000])
+@pytest.mark.parametrize("bullet", [True, False])
+def test_records_that_end_before_their_last_stride(count, bullet):
+    """A device array given from inside its first record (the fields of a
+    larger struct), so that it ends with the last record's last field."""
+    import torch
+    from shiokaze_b200 import native, scenes
+    names = ["lead", "mass", "velocity", "c", "p"] + (["bullet"] if bullet else [])
+    formats = [("u1", 24), "f4", ("f4", 3), ("f4", (3, 3)), ("f4", 3)] + (["u1"] if bullet else [])
+    offsets = [0, 24, 28, 40, 76] + ([88] if bullet else [])
+    dtype = np.dtype({"names": names, "formats": formats, "offsets": offsets, "itemsize": 92 if bullet else 88})
+    n, dx = 12, 1.0 / 12
+    rng = np.random.default_rng(count)
+    rec = np.zeros(count, dtype)
+    rec["p"] = rng.random((count, 3))
+    rec["velocity"] = rng.standard_normal((count, 3))
+    rec["c"] = rng.standard_normal((count, 3, 3))
+    rec["mass"] = rng.uniform(0.05, 0.2, count)
+    P = np.zeros(count, scenes.PARTICLE_DTYPE)
+    for k in ("p", "velocity", "c", "mass"):
+        P[k] = rec[k]
+    if bullet:
+        P["bullet"] = rec["bullet"] = rng.random(count) < 0.2
+    vel = [rng.standard_normal((n + (d == 2), n + (d == 1), n + (d == 0))).astype(np.float32) for d in range(3)]
+    act = [(rng.random(v.shape) < 0.7).astype(np.uint8) for v in vel]
+    want = oracle.splat(n, n, n, dx, P, vel, act)
+    T = lambda arr: torch.from_numpy(np.ascontiguousarray(arr)).to("cuda:0")
+    raw = T(rec.view(np.uint8).reshape(-1)[24:len(rec) * dtype.itemsize - (3 if bullet else 0)])
+    v, a_ = [T(x) for x in vel], [T(x) for x in act]
+    mass, mom, sact = [torch.zeros_like(x) for x in v], [torch.zeros_like(x) for x in v], [torch.zeros_like(x) for x in a_]
+    torch.cuda.synchronize()
+    ctx = native.Context(native.default_config())
+    a = native.splat_args(n, n, n, dx, raw.data_ptr(), count, dtype)
+    for field in ("offset_position", "offset_velocity", "offset_mass", "offset_apic", "offset_bullet"):
+        if getattr(a, field) >= 0:
+            setattr(a, field, getattr(a, field) - 24)
+    for d in range(3):
+        a.velocity[d], a.velocity_active[d] = v[d].data_ptr(), a_[d].data_ptr()
+        a.mass[d], a.momentum[d], a.splat_active[d] = mass[d].data_ptr(), mom[d].data_ptr(), sact[d].data_ptr()
+    ctx.check(native.load().shkz_b200_splat_device(ctx.handle, ctypes.byref(a)), "splat_device")
+    got = [[x.cpu().numpy() for x in part] for part in (v, a_, mass, mom, sact)]
+    assert_bitexact(got, dict(zip(("velocity", "velocity_active", "mass", "momentum", "splat_active"), want)))
