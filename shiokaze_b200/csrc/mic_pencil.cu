@@ -70,7 +70,6 @@ constexpr int CUNIT = UX * CROW, RUNIT = UX * RROW;
 constexpr int NG = 8;               // units of upstream face rows in their ring
 constexpr int GROW = 32;            // floats of a face row: [z 16] of the y face, [y 16] of the z face
 constexpr int PREFETCH = 6;         // units ahead of a copy into the ring that L2 is told of
-constexpr int SKEW = 10;            // steps the last lane trails the first
 constexpr int SEGQ = 16;            // pencils known ahead (a pencil has >= 4 units, the roles are < 2 NU units apart)
 constexpr int REDS = 8;             // macro tiles whose sums may be under way (the ring holds fewer)
 constexpr int NWARPS = 12;           // three to a sub-partition, so that the solver may have 168 registers
@@ -94,6 +93,7 @@ struct __align__(128) Smem {
   unsigned long long full[NU], empty[NU], freed[NU], gfull[NG], gempty[NG], segfull[SEGQ];
   int arrived[REDS];
   int limit, skip, dead;
+  long long patience;                  // clocks of a wait inside the CTA
 };
 
 static_assert(sizeof(Smem) <= 227 * 1024, "the ring fits one CTA's shared memory");
@@ -109,10 +109,12 @@ __device__ __forceinline__ void mb_expect(unsigned long long *b, int bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(b)), "r"(bytes) : "memory");
 }
 // Bounded wait for the phase with this parity. The roles wait for one another
-// inside the CTA and the pollers' own waits are bounded, so the limit (a few
-// seconds of clock) is not met; if it were, the sweep reports its error, the
-// CTA's remaining waits return at once and it issues no more copies.
+// inside the CTA and, in the end, for its pollers, whose rounds (0.24 us, 470
+// clocks each) are bounded by the configured limit. This limit is several times
+// theirs, and 4 s at least, so it is not met; if it were, the sweep reports its
+// error, the CTA's remaining waits return at once, and it loads nothing more.
 constexpr long long kWaitClocks = 1ll << 33;
+constexpr int kWaitClocksPerRound = 1 << 12;
 __device__ __forceinline__ bool mb_try(uint32_t a, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -130,7 +132,7 @@ __device__ __forceinline__ void mb_wait(Smem &sm, unsigned long long *b, uint32_
   const long long t0 = clock64();
   while (!mb_try(a, parity)) {
     if (*(volatile int *)&sm.dead) return;
-    if (clock64() - t0 > kWaitClocks) {
+    if (clock64() - t0 > *(volatile long long *)&sm.patience) {
       *(volatile int *)&sm.dead = 1;
       atomicCAS(&ws->error, 0, 1);
       return;
@@ -235,6 +237,7 @@ __device__ __forceinline__ bool begin(Smem &sm, WaveSync *ws, const SolverState 
   if (threadIdx.x == 0) {
     sm.dead = 0;
     sm.limit = spin_rounds(ws);
+    sm.patience = max(kWaitClocks, (long long)sm.limit * kWaitClocksPerRound);
     sm.skip = *((volatile int *)&ws->skip_publish);
   }
   __syncthreads();
@@ -488,7 +491,7 @@ __device__ __forceinline__ void solve_pencils(Smem &sm, float *faces, WaveSync *
     fr.next();
     Plane P, N;
     load_plane(L.at, P);
-    // one unit a trip; the skewed lanes end SKEW (< 12) steps after lane 0. The
+    // one unit a trip; the skewed lanes end 10 (< 12) steps after lane 0. The
     // first and last three trips, where lanes start and stop, are loops of
     // their own, so that the main one is free of branches.
     bool ready = false;
@@ -515,7 +518,7 @@ __device__ __forceinline__ void solve_pencils(Smem &sm, float *faces, WaveSync *
       __syncwarp();
       if (lane == 0) {
         mb_arrive(&sm.gempty[used]);
-        // after trip u + 3 every lane has left unit u (step 4 u + 3 + SKEW)
+        // after trip u + 3 every lane has left unit u (step 4 u + 3 + 10)
         if (!EDGE || g >= 3) mb_arrive(&sm.empty[er.slot]);
       }
       if (!EDGE || g >= 3) er.next();

@@ -205,3 +205,24 @@ def test_csr_factor_wait_timeout_returns_error_and_context_recovers():
     rc1, _, it1, x1 = solve(ctx)
     assert rc1 == 0 and it1 == it0
     assert np.array_equal(x1, x0)
+
+
+def test_a_longer_wait_limit_is_not_cut_short():
+    """Waits inside a CTA of the pencil sweeps end with an error after 4 s at
+    the earliest, but not before a longer configured limit of the waits they
+    depend on has run out: 2^25 rounds, 6 to 8 s."""
+    import time
+    from shiokaze_b200 import scenes
+    from shiokaze_b200.projection import MacPressureSolver3
+    sc = scenes.dambreak_sphere(n=48, seed=1, tol=1e-6)
+    res0, p0, _ = _reference_solution(sc)
+    s = MacPressureSolver3({"Residual": sc.tol, "B200.SpinLimit": 1 << 25, "B200.FaultSkipPublish": 1})
+    s.initialize((sc.nx, sc.ny, sc.nz), sc.dx)
+    t0 = time.perf_counter()
+    res, _, _ = _run(s, sc)
+    assert res["status"] == ERR_TIMEOUT
+    assert time.perf_counter() - t0 > 5.2
+    s.configure({"B200.SpinLimit": 0, "B200.FaultSkipPublish": 0})
+    res1, p1, _ = _run(s, sc)
+    assert res1["status"] == 0 and res1["iterations"] == res0["iterations"]
+    assert np.array_equal(p1, p0)
