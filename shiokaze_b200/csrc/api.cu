@@ -91,6 +91,7 @@ struct shkz_b200_ctx {
   LearnedModel *model = nullptr;
   int model_ready = 0;  // block activity computed for the current system
   AssemblyInputs last_in{};
+  bool inputs_gone = false;        // its arrays were the context's staging buffers, regrown since
   SolverState *st_scratch = nullptr;
   // optional terms: surface tension curvature, volume correction, warm start
   float *curv = nullptr;
@@ -279,11 +280,19 @@ static int ensure_grid(shkz_b200_ctx *ctx, const Geometry &G) {
   return 0;
 }
 
+// The last system may have been assembled from these (project_host): once one
+// of them is regrown for another call, its inputs can no longer be read.
 static int ensure_host_staging(shkz_b200_ctx *ctx, const Geometry &G, bool solid, const bool svel[3]) {
+  auto regrown = [&](const float *p) {
+    const AssemblyInputs &in = ctx->last_in;
+    if (p && (p == in.fluid || p == in.solid || p == in.vel[0] || p == in.vel[1] || p == in.vel[2]))
+      ctx->inputs_gone = true;
+  };
   const size_t cells = (size_t)G.nx * G.ny * G.nz;
   const size_t nodes = (size_t)(G.nx + 1) * (G.ny + 1) * (G.nz + 1);
   if (cells > ctx->cap_h_cells) {
     ctx->cap_h_cells = 0;
+    regrown(ctx->h_fluid);
     GROW(h_fluid, cells);
     GROW(h_fluid_active, cells);
     GROW(h_pressure, cells);
@@ -292,6 +301,7 @@ static int ensure_host_staging(shkz_b200_ctx *ctx, const Geometry &G, bool solid
   }
   if (solid && nodes > ctx->cap_h_nodes) {
     ctx->cap_h_nodes = 0;
+    regrown(ctx->h_solid);
     GROW(h_solid, nodes);
     GROW(h_solid_active, nodes);
     ctx->cap_h_nodes = nodes;
@@ -300,6 +310,7 @@ static int ensure_host_staging(shkz_b200_ctx *ctx, const Geometry &G, bool solid
     const size_t nf = (size_t)(G.nx + (d == 0)) * (G.ny + (d == 1)) * (G.nz + (d == 2));
     if (nf > ctx->cap_h_faces[d]) {
       ctx->cap_h_faces[d] = 0;
+      regrown(ctx->h_vel[d]);
       GROW(h_vel[d], nf);
       GROW(h_vact[d], nf);
       if (ctx->h_svel[d]) { release(ctx, ctx->h_svel[d]); ctx->h_svel[d] = nullptr; }
@@ -1009,6 +1020,7 @@ static int project_device(shkz_b200_ctx *ctx, const shkz_b200_project_args *a, s
   in.rhs_add = 0.0;
 
   ctx->last_in = in;
+  ctx->inputs_gone = false;
   const long long launches0 = launches_so_far();
   cudaEventRecord(ctx->ev[0], s);
   launch_label(in, ctx->flags, ctx->unk, ctx->tile_count, s);
@@ -1920,6 +1932,7 @@ extern "C" int shkz_b200_time_kernel(shkz_b200_ctx *ctx, int which, int reps, do
     }
   };
   if (which < 0 || which > 10) return SHKZ_B200_ERR_ARG;
+  if ((which == 5 || which == 6 || which == 8) && ctx->inputs_gone) return SHKZ_B200_ERR_STATE;
   if (which >= 9 && (!ctx->pb || S.KM <= 0)) return SHKZ_B200_ERR_STATE;
   if (which == 8) {
     const int rc = learned_ready(ctx);
@@ -2212,6 +2225,7 @@ extern "C" int shkz_b200_learned_apply(shkz_b200_ctx *ctx, const float *r_cells,
   cudaSetDevice(ctx->device);
   int rc = learned_ready(ctx);
   if (rc) return rc;
+  if (ctx->inputs_gone) return SHKZ_B200_ERR_STATE;
   cudaStream_t s = ctx->stream;
   const Geometry &G = ctx->G;
   const size_t cells = (size_t)G.nx * G.ny * G.nz;
@@ -2309,6 +2323,7 @@ extern "C" int shkz_b200_learned_train(shkz_b200_ctx *ctx, int steps, double lr,
   cudaSetDevice(ctx->device);
   int rc = learned_ready(ctx);
   if (rc) return rc;
+  if (ctx->inputs_gone) return SHKZ_B200_ERR_STATE;
   if (ctx->K == 0) return 0;
   cudaStream_t s = ctx->stream;
   if ((rc = prepare_mic(ctx))) return rc;

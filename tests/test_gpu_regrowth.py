@@ -124,3 +124,23 @@ def test_scenes_fit_under_a_memory_cap(n, filled, block, cap, config):
         # and again on pencils, built for the system that was solved without
         s.configure({"B200.DeviceMemoryLimitMB": 0})
         np.testing.assert_array_equal(s.apply_preconditioner(r), z)
+
+
+def test_network_after_its_inputs_were_regrown():
+    """The network reads the level sets the last projection was given; through
+    the host entry point those are staged in buffers that a larger extension
+    replaces. It is then refused until the next projection."""
+    from shiokaze_b200 import native
+    from shiokaze_b200.projection import MacPressureSolver3
+    s = MacPressureSolver3({"Residual": 1e-5})
+    _project(s, 24)
+    s.learned_init(seed=1)
+    r = np.random.default_rng(3).standard_normal((24, 24, 24)).astype(np.float32)
+    z = s.learned_apply(r)
+    _extend(s.context, 48)
+    with pytest.raises(native.ShkzError) as e:
+        s.learned_apply(r)
+    assert e.value.code == -7
+    s.inspect(0)  # the assembled system itself is still there
+    _project(s, 24)
+    np.testing.assert_array_equal(s.learned_apply(r), z)
