@@ -39,3 +39,45 @@ def _z(shape, blocks, block, seed):
 ])
 def test_pencil_sweeps_equal_tile_sweeps(shape, blocks):
     np.testing.assert_array_equal(_z(shape, blocks, 16, 3), _z(shape, blocks, 8, 3))
+
+
+@pytest.mark.parametrize("shape,blocks", [
+    ((8, 8, 8), 1.0),
+    ((16, 16, 16), 1.0),
+    ((17, 33, 15), 1.0),
+    ((150, 20, 50), 1.0),
+    ((96, 80, 64), 0.5),
+    ((64, 208, 224), 0.8),
+])
+@pytest.mark.parametrize("limit", [1, 2, 3, 30000])
+def test_fused_iteration_equals_the_separate_kernels(shape, blocks, limit):
+    """The loop every projection runs (r update, norms, z.r, rho and beta inside
+    the pencil sweeps, x and p updates in the next stencil) against the loop of
+    separate kernels on 8^3 tiles, at the shapes above and stopped after one,
+    two and three iterations, where an update is pending and the direction is in
+    either buffer. Per cell the FP32 arithmetic is the same; alpha and beta
+    differ by the order in which FP64 sums are added, some 1e-13."""
+    from shiokaze_b200.projection import Grid, MacGrid, MacPressureSolver3
+    nx, ny, nz = shape
+    dx = 1.0 / max(shape)
+    rng = np.random.default_rng(3)
+    pick = rng.random(((nz + 15) // 16, (ny + 15) // 16, (nx + 15) // 16)) < blocks
+    inside = pick.repeat(16, 0).repeat(16, 1).repeat(16, 2)[:nz, :ny, :nx]
+    inside[-1] = False  # a free surface
+    phi = (np.where(inside, -1.0, 1.0) * rng.uniform(0.2, 1.7, (nz, ny, nx)) * dx).astype(np.float32)
+    vel = [rng.standard_normal((nz + (d == 2), ny + (d == 1), nx + (d == 0))).astype(np.float32) for d in range(3)]
+    runs = []
+    for block in (16, 8):
+        s = MacPressureSolver3({"Residual": 1e-6, "MaxIterations": limit, "B200.MICBlock": block})
+        s.initialize(shape, dx)
+        grid = MacGrid([v.copy() for v in vel], [np.ones(v.shape, np.uint8) for v in vel])
+        res = s.project(0.01, grid, None, None, Grid(phi, np.ones(phi.shape, np.uint8)))
+        runs.append((res, s.get_pressure().values.astype(np.float64)))
+    (res, p), (other, want) = runs
+    assert res["status"] == 0 and res["iterations"] == other["iterations"]
+    assert res["iterations"] == limit if limit < 4 else res["reresid"] <= 1e-6
+    # FP32 vectors of the same cells: a last bit of alpha or beta is 6e-8, a few
+    # of them an iteration, summed over the iterations done
+    tol = 5e-7 * (res["iterations"] + 1)
+    assert np.abs(p - want).max() <= tol * np.abs(want).max()
+    assert abs(res["reresid"] - other["reresid"]) <= max(tol * other["reresid"], 1e-8)
