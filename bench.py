@@ -60,9 +60,9 @@ ALGO_BYTES = {
 ITER_BYTES = 100
 
 # library kernels one splat call launches: bin, tile scan, three scan passes,
-# scatter, sort, three face compactions, three work counts, work scan, three
-# face sorts, three gathers, clear
-SPLAT_LAUNCHES = 21
+# scatter, sort, face compaction, work count, work scan, face sort, gather,
+# clear (the three axes share each)
+SPLAT_LAUNCHES = 13
 
 # FLIP splat workload (--workload flip_splat): the splat and combined grid
 # velocity before a projection, on the 256^3 sloshing tank with particles in

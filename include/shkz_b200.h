@@ -75,10 +75,13 @@ typedef struct shkz_b200_config {
   int refine;                 /* FP64 outer refinement of the FP32 solve (default 1) */
   int fp64_reference;         /* also run an FP64 tight solve and report the error (default 0) */
   double fp64_tol;            /* tolerance of that solve (default 1e-12) */
-  int check_interval;         /* at most so many iterations queued beyond the last the device reported (default 16; the solve queues 3) */
+  int check_interval;         /* at most so many iterations queued beyond the last the device reported: 1 or 2
+                                 hold the queue shorter than the 3 the solve keeps, any other value (the
+                                 default is 16) changes nothing */
   int stall_window;           /* learned FPCG: iterations without progress before MIC(0) fallback */
   int device;                 /* CUDA device ordinal (default 0) */
-  int mic_block;              /* MIC(0) sweep block edge: 16 (default, 2x2x2 tiles per CTA) or 8 */
+  int mic_block;              /* MIC(0) sweeps on x-pencils of 16^3 macro tiles, a pencil per CTA (16, default),
+                                 or on 8^3 tiles, a tile per CTA (8): the same result */
   double gain;                /* Gain of the volume correction (default 1.0) */
   int warm_start;             /* WarmStart (default 0) */
   int index_tile;             /* tile edge of the caller's grids (TileSize, default 16): unknown numbering of

@@ -737,8 +737,8 @@ static void reset_progress(shkz_b200_ctx *ctx, int iter) {
   __atomic_store_n(&ctx->mail->progress, (unsigned long long)(unsigned)iter, __ATOMIC_RELEASE);
 }
 
-// Iterations queued beyond the last one reported. A retired launch costs 4 us
-// (12 an iteration) whenever the loop stops, which it does once per reliable
+// Iterations queued beyond the last one reported. A retired launch costs 1.5 us
+// (4.5 an iteration) whenever the loop stops, which it does once per reliable
 // update; too few queued and the device waits for the host.
 static const int kQueueAhead = 3;
 

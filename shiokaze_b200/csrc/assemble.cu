@@ -176,7 +176,6 @@ __global__ void k_levelset_exist(const float *fluid, const uint8_t *fluid_active
 }
 
 // ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // Strips: four 8^3 tiles along x, one CTA each. A warp takes rows of 32 cells,
 // 8 of the strip's 64, so that every access is a row's. (A thread per cell of
 // a tile, or of the grid with its coordinates from divisions, left HBM idle:
