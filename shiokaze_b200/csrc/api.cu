@@ -68,6 +68,7 @@ struct shkz_b200_ctx {
   double *partials = nullptr, *out4 = nullptr;
   Mailbox *mail = nullptr;         // pinned host memory the device reports to
   unsigned mail_seq = 0;           // number of the last report asked for
+  bool sleeps = false;             // waits for reports sleep (this call; see poll_mail)
   unsigned *counter = nullptr;
   SolverState *st = nullptr;
   int *wflags = nullptr;  // factor wavefront flags [cap_pool]
@@ -423,8 +424,7 @@ static int *macro_bsum(shkz_b200_ctx *ctx, const Geometry &G) { return ctx->bsum
 // projection of 36 ms: 36 ms of CPU time spinning, 5 sleeping and 1 ms longer).
 constexpr unsigned kTightLooks = 1000;
 template <class F>
-static bool poll_mail(cudaStream_t s, F arrived) {
-  bool sleeps = false;
+static bool poll_mail(const shkz_b200_ctx *ctx, F arrived) {
   for (unsigned looks = 1;; ++looks) {
     if (arrived()) return true;
     if (looks < kTightLooks) {
@@ -433,13 +433,9 @@ static bool poll_mail(cudaStream_t s, F arrived) {
 #endif
       continue;
     }
-    if (looks == kTightLooks) {
-      unsigned flags = 0;
-      sleeps = cudaGetDeviceFlags(&flags) == cudaSuccess &&
-               (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
-    }
-    if ((looks & (sleeps ? 0xfu : 0xfffu)) == 0 && cudaStreamQuery(s) != cudaErrorNotReady) return arrived();
-    if (sleeps) {
+    if ((looks & (ctx->sleeps ? 0xfu : 0xfffu)) == 0 && cudaStreamQuery(ctx->stream) != cudaErrorNotReady)
+      return arrived();
+    if (ctx->sleeps) {
       const timespec nap = {0, 50000};
       nanosleep(&nap, nullptr);
     } else {
@@ -448,7 +444,7 @@ static bool poll_mail(cudaStream_t s, F arrived) {
   }
 }
 static int wait_mail(shkz_b200_ctx *ctx, unsigned seq) {
-  if (poll_mail(ctx->stream, [&] { return __atomic_load_n(&ctx->mail->seq, __ATOMIC_ACQUIRE) == seq; })) return 0;
+  if (poll_mail(ctx, [&] { return __atomic_load_n(&ctx->mail->seq, __ATOMIC_ACQUIRE) == seq; })) return 0;
   shkz_set_cuda_error(cudaGetLastError(), "report of a kernel", __FILE__, __LINE__);
   return SHKZ_B200_ERR_CUDA;
 }
@@ -462,6 +458,9 @@ static unsigned next_mail(shkz_b200_ctx *ctx) {
 // small kernels and read by the host in one go.
 static int count_pool(shkz_b200_ctx *ctx, const Geometry &G, int *K, int *macro_tiles, long long *unknowns) {
   cudaStream_t s = ctx->stream;
+  unsigned flags = 0;
+  ctx->sleeps = cudaGetDeviceFlags(&flags) == cudaSuccess &&
+                (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
   const bool macro = ctx->cfg.mic_block != 8;
   const unsigned seq = next_mail(ctx);
   launch_pool_count(G, ctx->tile_count, ctx->bsum, ctx->usum, false, ctx->mail, macro ? 0 : seq, s);
@@ -714,7 +713,7 @@ static int wait_progress(shkz_b200_ctx *ctx, int iter, Progress *p) {
     v = __atomic_load_n(&ctx->mail->progress, __ATOMIC_ACQUIRE);
     return (int)(unsigned)v >= iter || (v >> kProgressDone) != 0;
   };
-  if (poll_mail(ctx->stream, arrived)) {
+  if (poll_mail(ctx, arrived)) {
     p->iter = (int)(unsigned)v;
     p->done = (int)(v >> kProgressDone) & 0xff;
     p->nan = (v & kProgressNan) != 0;

@@ -149,3 +149,31 @@ def test_waits_sleep_under_blocking_synchronisation():
                          capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stderr[-2000:]
     assert float(out.stdout.split()[-1]) < 0.5, out.stdout
+
+
+def test_two_contexts_solve_at_once():
+    """Two threads, a context and a scene each, project at the same time: their
+    sweeps share the SMs, wait only for their own, and give what they give
+    alone."""
+    import threading
+    scenes = [_Scene((40, 33, 50), 0.6, 5, 16), _Scene((96, 80, 64), 0.5, 9, 16)]
+    config = {"Residual": 1e-5}
+    alone = [_solve(sc, **config) for sc in scenes]
+    got = [[], []]
+
+    def work(i):
+        for _ in range(6):
+            got[i].append(_solve(scenes[i], **config))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(2):
+        assert len(got[i]) == 6
+        for res, p, vel in got[i]:
+            assert (res["status"], res["iterations"], res["reresid"]) == (0, alone[i][0]["iterations"], alone[i][0]["reresid"])
+            np.testing.assert_array_equal(p, alone[i][1])
+            for a, b in zip(vel, alone[i][2]):
+                np.testing.assert_array_equal(a, b)
