@@ -328,7 +328,7 @@ def run_splat(args):
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "ms": call_ms, "algo_bytes_per_launch": algo, "traffic": traffic,
                 "note": ("not HBM-bound: the gather (about 3/5 of the call) is bound by L1 passes and FP64 conversions, "
-                         "each face summing its particles serially in the reference's order; traffic was 9.5x the "
+                         "each face summing its particles serially in the reference's order; traffic is 9.0x the "
                          "algorithmic bytes because of the hash (packed and bucket-ordered particle copies, the "
                          "gather's L2 re-reads)")}
     # end to end through the host-buffer entry point, pinned host arrays

@@ -41,8 +41,8 @@
 // Measured on a B200 against a CTA per macro tile with a barrier per diagonal
 // and whole-tile hand-offs (same values): sweep pair on a full 256 x 128 x 256
 // grid, 8.4 M cells, 246 us against 341 us, 256^3 340 against 526 us; a hop
-// between pencils takes 2.3 (z) and 2.8 us (y), of which the trip through L2 is
-// 1.2, and a step 156 ns, set by the solver's instructions (10 shared loads, 6
+// between pencils takes 2.1 (z) and 2.7 us (y), of which the trip through L2 is
+// 1.2, and a step 153 ns, set by the solver's instructions (10 shared loads, 6
 // shuffles, 32 multiply-adds). Tried: 4 x 2 blocks with plane-wise faces (3.95 us
 // a hop), tagged 64-bit face words, fences or branches in the solver's loop
 // (each 60 - 200 ns a step).
