@@ -964,28 +964,33 @@ int learned_prepare(LearnedModel *m, const Geometry &G, const int *tile_state, c
     m->gb[l][2] = (m->NZ[l] + 7) / 8;
   }
   if (resize) {
+    bool ok = true;
+    auto regrow = [&](auto *&p, size_t bytes) {
+      if (p) cudaFree(p);
+      p = nullptr;
+      ok = ok && cudaMalloc(&p, bytes) == cudaSuccess;
+      if (!ok) p = nullptr;
+    };
     for (int l = 0; l < 3; ++l) {
-      if (m->blk[l]) cudaFree(m->blk[l]);
-      if (m->blkd[l]) cudaFree(m->blkd[l]);
       const size_t nb = (size_t)m->gb[l][0] * m->gb[l][1] * m->gb[l][2];
-      if (cudaMalloc(&m->blk[l], nb) != cudaSuccess || cudaMalloc(&m->blkd[l], nb) != cudaSuccess)
-        return SHKZ_B200_ERR_NOMEM;
+      regrow(m->blk[l], nb);
+      regrow(m->blkd[l], nb);
     }
     for (int t = 0; t < T_COUNT; ++t) {
-      if (m->T[t]) cudaFree(m->T[t]);
-      if (m->Gt[t]) cudaFree(m->Gt[t]);
       const size_t n = nvox(m, kTensorLevel[t]) * kTensorC[t];
-      if (cudaMalloc(&m->T[t], n * 2) != cudaSuccess || cudaMalloc(&m->Gt[t], n * 4) != cudaSuccess)
-        return SHKZ_B200_ERR_NOMEM;
+      regrow(m->T[t], n * 2);
+      regrow(m->Gt[t], n * 4);
     }
-    if (m->Z) cudaFree(m->Z);
-    if (m->gZ) cudaFree(m->gZ);
-    if (m->gpre) cudaFree(m->gpre);
-    if (m->gx) cudaFree(m->gx);
     const size_t n0 = nvox(m, 0);
-    if (cudaMalloc(&m->Z, n0 * 4) != cudaSuccess || cudaMalloc(&m->gZ, n0 * 4) != cudaSuccess ||
-        cudaMalloc(&m->gpre, n0 * 64 * 2) != cudaSuccess || cudaMalloc(&m->gx, n0 * 64 * 2) != cudaSuccess)
+    regrow(m->Z, n0 * 4);
+    regrow(m->gZ, n0 * 4);
+    regrow(m->gpre, n0 * 64 * 2);
+    regrow(m->gx, n0 * 64 * 2);
+    if (!ok) {
+      cudaGetLastError();
+      m->NX[0] = 0;  // no size is held: the next call allocates anew
       return SHKZ_B200_ERR_NOMEM;
+    }
   }
   for (int l = 0; l < 3; ++l) {
     count_launches(1);
